@@ -25,10 +25,6 @@
 namespace nestb {
 namespace {
 
-#ifndef NEST_F64R_UNROLL
-#define NEST_F64R_UNROLL 1
-#endif
-constexpr int kUnrollD = NEST_F64R_UNROLL;  // row-loop unroll
 constexpr int LOOKD = 3;                   // stage-input rows in flight ahead of the march
 constexpr int RING_UD = 4, RING_ND = 2;    // ring slots: stage input, U^n (stage 2)
 __host__ __device__ constexpr int ring_d_per_warp(int stage) { return (RING_UD + (stage == 2 ? RING_ND : 0)) * 4 * 32; }
@@ -44,69 +40,122 @@ __device__ __forceinline__ void cpd_wait() { asm volatile("cp.async.wait_group %
 
 using W4 = Win4<double>;
 
-__device__ __forceinline__ W4 half_step(const W4& w, const W4& s, double h) {
-    return { w.a + h * s.a, w.b + h * s.b, w.c + h * s.c, w.d + h * s.d };
-}
-__device__ __forceinline__ W4 half_back(const W4& w, const W4& s) {
-    return { w.a - 0.5 * s.a, w.b - 0.5 * s.b, w.c - 0.5 * s.c, w.d - 0.5 * s.d };
-}
+// Arithmetic policies of a row: the IEEE division and square root, or the
+// branch-free ones of f64div.cuh with their range tests.  Both give the same
+// values wherever the tests pass; a row in which one fails for a lane that can
+// reach an output is computed again with the IEEE policy before anything of it
+// is stored.
+//
+// What the tests rest on.  prim() tests rho and p of every cell the row adds to
+// the window (and the two momenta as numerators); a finite u or v follows, with
+// |u| < 2^181, because 2^-128 <= p = (gamma - 1) (E - ke) < 2^128 needs
+// ke < 2^233.  A row whose window holds a cell that failed runs with the IEEE
+// policy as a whole (`hold` below).  A minmod face state w -+ s/2 lies between w
+// and half way to a neighbour, so rho and p of a face need no test of their own
+// (with the other limiters, which can reach or pass the neighbour's value, they
+// get one).  dS = SR - SL is at least about the smaller sound speed where the
+// average flux is taken, and its numerators stay under 2^880; the mass,
+// transverse and energy ones, which can be tiny, are tested (the normal one
+// holds SR p - SL p, which cannot).
+struct ArithIeee {
+    static constexpr bool checked = false;
+    struct Recip { double b; };
+    __device__ __forceinline__ Recip recip(double b) const { return { b }; }
+    __device__ __forceinline__ double quot(double a, const Recip& r) const { return a / r.b; }
+    __device__ __forceinline__ double root(double x) const { return sqrt(x); }
+    __device__ __forceinline__ double half(double w, double h, double s) const { return w + h * s; }
+    __device__ __forceinline__ void pos(double) {}
+    __device__ __forceinline__ void num(double) {}
+    __device__ __forceinline__ bool ok() const { return true; }
+};
+struct ArithFast {
+    static constexpr bool checked = true;
+    struct Recip { double b, y; };
+    F64Range r;
+    __device__ __forceinline__ Recip recip(double b) const { return { b, recip_f64(b) }; }
+    __device__ __forceinline__ double quot(double a, const Recip& q) const { return quot_f64(a, q.b, q.y); }
+    __device__ __forceinline__ double root(double x) const { return sqrt_f64(x); }
+    // h = +-1/2: h s is exact (slopes in range are multiples of 2^-1000), so the
+    // fused form rounds the same sum
+    __device__ __forceinline__ double half(double w, double h, double s) const { return fma(h, s, w); }
+    __device__ __forceinline__ void pos(double x) { r.pos(x); }
+    __device__ __forceinline__ void num(double a) { r.num(a); }
+    __device__ __forceinline__ bool ok() const { return r.ok(); }
+};
 
-// Division policies of a row: the IEEE division, or the checked fast
-// division of f64div.cuh, which returns the same value whenever it leaves
-// `ok` set (a row with any cleared flag in the warp is recomputed with the
-// IEEE policy before anything of it is stored).
-struct DivIeee {
-    __device__ __forceinline__ double div(double x, double y) { return x / y; }
-};
-struct DivChecked {
-    bool ok = true;
-    __device__ __forceinline__ double div(double x, double y) { return div_rn_checked(x, y, ok); }
-};
+// Face states w + s/2 and w - s/2.
+template <class A>
+__device__ __forceinline__ W4 face_up(const A& m, const W4& w, const W4& s) {
+    return { m.half(w.a, 0.5, s.a), m.half(w.b, 0.5, s.b), m.half(w.c, 0.5, s.c), m.half(w.d, 0.5, s.d) };
+}
+template <class A>
+__device__ __forceinline__ W4 face_dn(const A& m, const W4& w, const W4& s) {
+    return { m.half(w.a, -0.5, s.a), m.half(w.b, -0.5, s.b), m.half(w.c, -0.5, s.c), m.half(w.d, -0.5, s.d) };
+}
 
 // cons2prim, hlle4 and cell_speeds_p of euler2d_kernels.cuh for the FP64
 // plain form (the same expressions in the same order, so the same values),
-// with their divisions taken from a policy.
-template <class D>
-__device__ __forceinline__ W4 prim_d(D& d, const W4& c, double gm1) {
-    const double u = d.div(c.b, c.a), v = d.div(c.c, c.a);
-    const double p = gm1 * (c.d - ke2(c.a, u, v));
-    return { c.a, u, v, smax(p, 0.0) };
+// with their divisions and square roots taken from a policy.
+template <class A>
+__device__ __forceinline__ W4 prim_d(A& m, const W4& c, double gm1) {
+    const auto ir = m.recip(c.a);
+    const double u = m.quot(c.b, ir), v = m.quot(c.c, ir);
+    const double p = smax(gm1 * (c.d - ke2(c.a, u, v)), 0.0);
+    m.pos(c.a); m.pos(p); m.num(c.b); m.num(c.c);
+    return { c.a, u, v, p };
 }
 
-template <class D>
-__device__ __forceinline__ void hlle4_d(D& d, double gamma, double gm1, double rL, double nL, double tL, double pL,
-                                        double rR, double nR, double tR, double pR, double& f0, double& f1,
-                                        double& f2, double& f3) {
-    const double cL = sqrt(d.div(gamma * pL, rL));
-    const double cR = sqrt(d.div(gamma * pR, rR));
-    const double EL = d.div(pL, gm1) + ke2(rL, nL, tL);
-    const double ER = d.div(pR, gm1) + ke2(rR, nR, tR);
+// ig: reciprocal of gamma - 1; FACE: test the face states.
+template <bool FACE, class A>
+__device__ __forceinline__ void hlle4_d(A& m, double gamma, const typename A::Recip& ig, double rL, double nL,
+                                        double tL, double pL, double rR, double nR, double tR, double pR, double& f0,
+                                        double& f1, double& f2, double& f3) {
+    const double cL = m.root(m.quot(gamma * pL, m.recip(rL)));
+    const double cR = m.root(m.quot(gamma * pR, m.recip(rR)));
+    const double EL = m.quot(pL, ig) + ke2(rL, nL, tL);
+    const double ER = m.quot(pR, ig) + ke2(rR, nR, tR);
     const double SL = smin(nL - cL, nR - cR);
     const double SR = smax(nL + cL, nR + cR);
     const double mL = rL * nL, mR = rR * nR;
     const double FL0 = mL, FL1 = mL * nL + pL, FL2 = mL * tL, FL3 = (EL + pL) * nL;
     const double FR0 = mR, FR1 = mR * nR + pR, FR2 = mR * tR, FR3 = (ER + pR) * nR;
-    if (SL >= 0.0) {
+    if (FACE) { m.pos(rL); m.pos(pL); m.pos(rR); m.pos(pR); }
+    if (A::checked) {
+        // the average flux in every lane, then the regime's selection
+        const double SLR = SL * SR, dS = SR - SL;
+        const auto id = m.recip(dS);
+        const double a0 = SR * FL0 - SL * FR0 + SLR * (rR - rL), a1 = SR * FL1 - SL * FR1 + SLR * (mR - mL);
+        const double a2 = SR * FL2 - SL * FR2 + SLR * (rR * tR - rL * tL), a3 = SR * FL3 - SL * FR3 + SLR * (ER - EL);
+        m.num(a0); m.num(a2); m.num(a3);
+        const bool l = SL >= 0.0, r = SR <= 0.0;
+        f0 = l ? FL0 : r ? FR0 : m.quot(a0, id);
+        f1 = l ? FL1 : r ? FR1 : m.quot(a1, id);
+        f2 = l ? FL2 : r ? FR2 : m.quot(a2, id);
+        f3 = l ? FL3 : r ? FR3 : m.quot(a3, id);
+    } else if (SL >= 0.0) {
         f0 = FL0; f1 = FL1; f2 = FL2; f3 = FL3;
     } else if (SR <= 0.0) {
         f0 = FR0; f1 = FR1; f2 = FR2; f3 = FR3;
     } else {
-        const double SLR = SL * SR, dS = SR - SL;
-        f0 = d.div(SR * FL0 - SL * FR0 + SLR * (rR - rL), dS);
-        f1 = d.div(SR * FL1 - SL * FR1 + SLR * (mR - mL), dS);
-        f2 = d.div(SR * FL2 - SL * FR2 + SLR * (rR * tR - rL * tL), dS);
-        f3 = d.div(SR * FL3 - SL * FR3 + SLR * (ER - EL), dS);
+        const double SLR = SL * SR;
+        const auto id = m.recip(SR - SL);
+        f0 = m.quot(SR * FL0 - SL * FR0 + SLR * (rR - rL), id);
+        f1 = m.quot(SR * FL1 - SL * FR1 + SLR * (mR - mL), id);
+        f2 = m.quot(SR * FL2 - SL * FR2 + SLR * (rR * tR - rL * tL), id);
+        f3 = m.quot(SR * FL3 - SL * FR3 + SLR * (ER - EL), id);
     }
 }
 
-template <class D>
-__device__ __forceinline__ double speeds_d(D& d, double U0, double U1, double U2, double U3, double gamma,
+template <class A>
+__device__ __forceinline__ double speeds_d(A& m, double U0, double U1, double U2, double U3, double gamma,
                                            double gm1, double& sx, double& sy) {
     const double rho = smax(U0, 1e-10);
-    const double u = d.div(U1, rho), v = d.div(U2, rho);
+    const auto ir = m.recip(rho);
+    const double u = m.quot(U1, ir), v = m.quot(U2, ir);
     const double ke = 0.5 * rho * (u * u + v * v);
     const double p = smax(gm1 * (U3 - ke), 1e-10);
-    const double c = sqrt(d.div(gamma * p, rho));
+    const double c = m.root(m.quot(gamma * p, ir));
+    m.pos(rho); m.pos(p); m.num(U1); m.num(U2);
     sx = fabs(u) + c;
     sy = fabs(v) + c;
     return gm1 * (U3 - ke2(rho, u, v));
@@ -188,6 +237,16 @@ __device__ __forceinline__ void f64r_body(const StageArgs<double>& a, int strip,
         return { __ldg(Ui + o), __ldg(Ui + vs + o), __ldg(Ui + 2 * vs + o), __ldg(Ui + 3 * vs + o) };
     };
 
+    // gamma and gamma - 1 inside the range tests' assumptions; else every row
+    // takes the IEEE policy.  `hold`: rows still to run with it because the
+    // window holds a cell that failed a test (a cell enters as row i+2 and
+    // leaves with the upper face state of row i, three rows later).
+    const int hold_all = gamma < 1024.0 && gm1 > 0x1p-20 ? 0 : 1 << 30;
+    int hold = hold_all;
+    constexpr bool FACE = LIM != LIM_MINMOD;
+    const typename ArithFast::Recip igf{ gm1, recip_f64(gm1) };
+    const typename ArithIeee::Recip igi{ gm1 };
+
     // prologue: rows i0-2 .. i0+1, the x-flux of face i0-1/2 and the upper
     // x-face state of row i0
     W4 Wq, Wq1, Pq, Fm;
@@ -199,28 +258,30 @@ __device__ __forceinline__ void f64r_body(const StageArgs<double>& a, int strip,
         cpd_commit();
         cpd_wait<0>();
         __syncwarp();
-        // with the checked divisions, again with IEEE ones if a lane up to the
-        // last ghost column failed one (as in the row loop below)
-        auto pro = [&](auto& d) {
-            const W4 Wa = prim_d(d, c0, gm1), Wb = prim_d(d, c1, gm1);
-            Wq = prim_d(d, ring_row(i0), gm1);
-            Wq1 = prim_d(d, ring_row(i0 + 1), gm1);
+        auto pro = [&](auto& m, auto& mp, const auto& ig) {
+            const W4 Wa = prim_d(mp, c0, gm1), Wb = prim_d(mp, c1, gm1);
+            Wq = prim_d(mp, ring_row(i0), gm1);
+            Wq1 = prim_d(mp, ring_row(i0 + 1), gm1);
             const W4 Sb = limit4(Wa, Wb, Wq, lim), Sq = limit4(Wb, Wq, Wq1, lim);
-            const W4 L = half_step(Wb, Sb, 0.5), R = half_back(Wq, Sq);
-            hlle4_d(d, gamma, gm1, L.a, L.b, L.c, L.d, R.a, R.b, R.c, R.d, Fm.a, Fm.b, Fm.c, Fm.d);
-            Pq = half_step(Wq, Sq, 0.5);
+            const W4 L = face_up(m, Wb, Sb), R = face_dn(m, Wq, Sq);
+            hlle4_d<FACE>(m, gamma, ig, L.a, L.b, L.c, L.d, R.a, R.b, R.c, R.d, Fm.a, Fm.b, Fm.c, Fm.d);
+            Pq = face_up(m, Wq, Sq);
         };
-        DivChecked dpro;
-        pro(dpro);
-        if (__any_sync(0xffffffffu, !dpro.ok && j <= ny + 1)) {
-            DivIeee di;
-            pro(di);
+        // columns up to the last ghost column can reach an output; lanes past
+        // it read the row padding
+        ArithFast m, mp;
+        pro(m, mp, igf);
+        const bool badp = __any_sync(0xffffffffu, !mp.ok() && j <= ny + 1);
+        if (badp) hold = max(hold, 3);
+        if (badp || hold || __any_sync(0xffffffffu, !m.ok() && j <= ny + 1)) {
+            ArithIeee mi;
+            pro(mi, mi, igi);
         }
     }
 
     double smx = 0.0, smy = 0.0;
     double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
-#pragma unroll kUnrollD
+#pragma unroll 1
     for (int k = 0; k < rows; ++k) {
         const int i = i0 + k;
         // refill the slots of row i-1 once every lane has read them; then
@@ -237,20 +298,22 @@ __device__ __forceinline__ void f64r_body(const StageArgs<double>& a, int strip,
         // transverse u; the left face from the left neighbour), the update of
         // every lane's cell of row i and, in stage 2, its wave speeds.
         struct RowOut {
-            W4 W2, S1, Fc, s;
+            W4 W2, P1, Fc, s;  // P1: upper x-face state of row i+1
             double sx, sy, pc;
         };
-        auto row = [&](auto& dp, auto& dv) {
+        auto row = [&](auto& mp, auto& mf, const auto& ig) {
             RowOut o;
-            o.W2 = prim_d(dp, ring_row(i + 2), gm1);
-            o.S1 = limit4(Wq, Wq1, o.W2, lim);
-            const W4 M1 = half_back(Wq1, o.S1);
-            hlle4_d(dv, gamma, gm1, Pq.a, Pq.b, Pq.c, Pq.d, M1.a, M1.b, M1.c, M1.d, o.Fc.a, o.Fc.b, o.Fc.c, o.Fc.d);
+            o.W2 = prim_d(mp, ring_row(i + 2), gm1);
+            const W4 S1 = limit4(Wq, Wq1, o.W2, lim);
+            const W4 M1 = face_dn(mf, Wq1, S1);
+            o.P1 = face_up(mf, Wq1, S1);
+            hlle4_d<FACE>(mf, gamma, ig, Pq.a, Pq.b, Pq.c, Pq.d, M1.a, M1.b, M1.c, M1.d, o.Fc.a, o.Fc.b, o.Fc.c,
+                          o.Fc.d);
             const W4 sy = limit4(shfl_up4(Wq), Wq, shfl_dn4(Wq), lim);
-            const W4 Rq = shfl_dn4(half_back(Wq, sy));
-            const W4 Ly = half_step(Wq, sy, 0.5);
+            const W4 Rq = shfl_dn4(face_dn(mf, Wq, sy));
+            const W4 Ly = face_up(mf, Wq, sy);
             W4 Gy;
-            hlle4_d(dv, gamma, gm1, Ly.a, Ly.c, Ly.b, Ly.d, Rq.a, Rq.c, Rq.b, Rq.d, Gy.a, Gy.c, Gy.b, Gy.d);
+            hlle4_d<FACE>(mf, gamma, ig, Ly.a, Ly.c, Ly.b, Ly.d, Rq.a, Rq.c, Rq.b, Rq.d, Gy.a, Gy.c, Gy.b, Gy.d);
             const W4 Gl = shfl_up4(Gy);
             const W4 C0 = ring_row(i);
             o.s.a = C0.a - (dtdx * (o.Fc.a - Fm.a) + dtdy * (Gy.a - Gl.a));
@@ -263,24 +326,27 @@ __device__ __forceinline__ void f64r_body(const StageArgs<double>& a, int strip,
                 o.s.b = 0.5 * (N0.b + o.s.b);
                 o.s.c = 0.5 * (N0.c + o.s.c);
                 o.s.d = 0.5 * (N0.d + o.s.d);
-                o.pc = speeds_d(dv, o.s.a, o.s.b, o.s.c, o.s.d, gamma, gm1, o.sx, o.sy);
+                o.pc = speeds_d(mf, o.s.a, o.s.b, o.s.c, o.s.d, gamma, gm1, o.sx, o.sy);
             }
             return o;
         };
-        // The checked divisions first; if one of them that can reach an
-        // output could not be shown to be correctly rounded, the whole row
-        // again with IEEE divisions.  Either way the stored values are those
-        // of the IEEE arithmetic.  What reaches an output: the primitives of
-        // every lane up to the last ghost column (y-slopes of the lanes two
-        // away), and the fluxes and wave speeds of lanes 1..29 inside the
-        // domain (lane j-1's y-face is lane j's left face); lanes past the
-        // ghost columns read the row padding.
-        DivChecked dp, dc;
-        RowOut o = row(dp, dc);
-        const bool need = (!dp.ok && j <= ny + 1) || (!dc.ok && lane >= 1 && lane < 30 && j < ny);
-        if (__any_sync(0xffffffffu, need)) {
-            DivIeee di;
-            o = row(di, di);
+        // The branch-free arithmetic first; if a range test of something that
+        // can reach an output failed, the whole row again with the IEEE
+        // operations.  Either way the stored values are those of the IEEE
+        // arithmetic.  What reaches an output: the primitives of every lane
+        // up to the last ghost column (y-slopes of the lanes two away), and
+        // the fluxes and wave speeds of lanes 1..29 inside the domain (lane
+        // j-1's y-face is lane j's left face); lanes past the ghost columns
+        // read the row padding.
+        ArithFast mp, mf;
+        RowOut o = row(mp, mf, igf);
+        const bool badp = __any_sync(0xffffffffu, !mp.ok() && j <= ny + 1);
+        const bool badf = __any_sync(0xffffffffu, !mf.ok() && lane >= 1 && lane < 30 && j < ny);
+        if (badp) hold = max(hold, 4);
+        if (badf || hold > 0) {
+            ArithIeee mi;
+            o = row(mi, mi, igi);
+            if (hold > 0) --hold;
         }
 
         if (out_col) {
@@ -307,7 +373,7 @@ __device__ __forceinline__ void f64r_body(const StageArgs<double>& a, int strip,
             }
         }
         Fm = o.Fc;
-        Pq = half_step(Wq1, o.S1, 0.5);
+        Pq = o.P1;
         Wq = Wq1;
         Wq1 = o.W2;
     }
@@ -334,18 +400,23 @@ __device__ __forceinline__ void f64r_body(const StageArgs<double>& a, int strip,
     }
 }
 
-// Row-loop unroll and register budget (0: ptxas's choice).
+// Register budget: 168 a thread, 12 warps per SM.  The kernels are bound by the
+// FP64 pipe (about 360 / 410 FP64 instructions a row, two issue cycles each,
+// put a 4096^2 step at 0.81 ms) and by the latency of its division and square
+// root chains, and with no branch in them the compiler interleaves the x- and
+// y-face chains of a row: more registers a warp pay off against fewer warps.
+// 4096^2 diagonal Riemann problem, ms per step over 64 steps (24-row tiles):
+// budget 128 (16 warps, spills) 1.313, 144 (14) 1.328, ptxas's own choice (158,
+// 12) 1.297, 168 (12) 1.261, 192 (10) 1.421, unrolled by 2 1.429.  With the
+// quotients tested one by one by an exact residual and the IEEE square root the
+// step took 2.090 ms, 1000 steps of the 2048^2 periodic Kelvin-Helmholtz state
+// 576 -> 349 ms.  Tile rows now: 16 1.286, 24 1.261, 32 1.265, 48 1.283.
 #ifndef NEST_F64R_REGS
-#define NEST_F64R_REGS 0
-#endif
-#if NEST_F64R_REGS > 0
-#define NEST_F64R_ATTR __maxnreg__(NEST_F64R_REGS)
-#else
-#define NEST_F64R_ATTR __launch_bounds__(256)
+#define NEST_F64R_REGS 168
 #endif
 
 template <int STAGE, bool TOT, int LIM>
-__global__ void NEST_F64R_ATTR k2d_f64r(StageArgs<double> a) {
+__global__ void __maxnreg__(NEST_F64R_REGS) k2d_f64r(StageArgs<double> a) {
     f64r_body<STAGE, TOT, LIM>(a, blockIdx.x * blockDim.y + threadIdx.y, blockIdx.y);
 }
 
@@ -377,25 +448,47 @@ cudaError_t launch_2d_step_f64r(double* U, double* U1, const Geo2D& g, const Loo
 }
 
 namespace {
+// The policies' quotient, its sign set for a divisor of either sign, and
+// whether the kernels would keep it.
 __global__ void k_div_selftest(const double* a, const double* b, double* q, int* ok, int n) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) {
-        bool k = true;
-        q[t] = div_rn_checked(a[t], b[t], k);
-        ok[t] = k ? 1 : 0;
+        const double d = fabs(b[t]), v = copysign(1.0, b[t]) * a[t];
+        q[t] = quot_f64(v, d, recip_f64(d));
+        ok[t] = quot_in_range(v, d, q[t]) ? 1 : 0;
+    }
+}
+__global__ void k_sqrt_selftest(const double* a, double* r, int* ok, int n) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) {
+        r[t] = sqrt_f64(a[t]);
+        ok[t] = a[t] >= 0x1p-257 && a[t] < 0x1p268 ? 1 : 0;
     }
 }
 }  // namespace
 
 }  // namespace nestb
 
-extern "C" nest_status nest_selftest_div_f64(const double* d_a, const double* d_b, double* d_q, int* d_ok, int n) {
-    if (!d_a || !d_b || !d_q || !d_ok || n < 0) return nestb::record_error(NEST_ERR_INVALID, "null array or n < 0");
+namespace {
+template <class Launch>
+nest_status selftest(const void* d_a, const void* d_q, const void* d_ok, int n, const char* what, Launch launch) {
+    if (!d_a || !d_q || !d_ok || n < 0) return nestb::record_error(NEST_ERR_INVALID, "null array or n < 0");
     if (n == 0) return NEST_OK;
-    nestb::k_div_selftest<<<(n + 255) / 256, 256>>>(d_a, d_b, d_q, d_ok, n);
+    launch((n + 255) / 256);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (e != cudaSuccess)
-        return nestb::record_error(NEST_ERR_CUDA, std::string("division self-test: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) return nestb::record_error(NEST_ERR_CUDA, std::string(what) + cudaGetErrorString(e));
     return NEST_OK;
+}
+}  // namespace
+
+extern "C" nest_status nest_selftest_div_f64(const double* d_a, const double* d_b, double* d_q, int* d_ok, int n) {
+    if (!d_b) return nestb::record_error(NEST_ERR_INVALID, "null array or n < 0");
+    return selftest(d_a, d_q, d_ok, n, "division self-test: ",
+                    [&](int blocks) { nestb::k_div_selftest<<<blocks, 256>>>(d_a, d_b, d_q, d_ok, n); });
+}
+
+extern "C" nest_status nest_selftest_sqrt_f64(const double* d_x, double* d_r, int* d_ok, int n) {
+    return selftest(d_x, d_r, d_ok, n, "square root self-test: ",
+                    [&](int blocks) { nestb::k_sqrt_selftest<<<blocks, 256>>>(d_x, d_r, d_ok, n); });
 }

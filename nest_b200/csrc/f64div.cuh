@@ -1,75 +1,114 @@
-// Correctly rounded FP64 division without a slow-path branch in the common
-// case, for the FP64 plain form's row marches (sm_100a; compiled with
-// -fmad=false, every fused multiply-add below is an explicit fma()).
+// Correctly rounded FP64 division and square root without slow-path branches,
+// for the FP64 plain form (sm_100a; every fused multiply-add below is an
+// explicit fma(), so the units' -fmad=false does not matter here).
 //
-// Method (textbook, not a restatement of any library routine):
-//   * y ~ 1/b from the hardware approximation (PTX rcp.approx.ftz.f64),
-//     refined by two Newton-Raphson steps y <- y + y (1 - b y), each of which
-//     roughly doubles the number of correct bits;
-//   * q0 = a y, then one residual correction q = q0 + (a - b q0) y, with the
-//     residual formed exactly by a fused multiply-add (P. Markstein,
-//     "Computation of elementary functions on the IBM RISC System/6000
-//     processor", IBM J. Res. Dev. 34(1), 1990);
-//   * a rounding test on the exact residual r = a - b q: q is the correctly
-//     rounded quotient RN(a/b) if |a/b - q| < ulp(q)/2, i.e. |r| < |b| ulp(q)/2
-//     (a quotient of two doubles is never exactly halfway between two
-//     doubles, so no tie arises), provided r is exact, which holds when q is
-//     within an ulp of a/b and nothing under- or overflows (J.-M. Muller et
-//     al., Handbook of Floating-Point Arithmetic, 2nd ed., 2018, ch. 4).  A q
-//     further than an ulp from a/b gives |r| >= |b| ulp(q) and fails the
-//     test, so an accepted q is always RN(a/b).
-// The test is only trusted inside a safe range: |a| and |q| in
-// [2^-959, 2^961).  There ulp(q)/2 >= 2^-1012 and the threshold
-// |b| ulp(q)/2 ~ |a| 2^-53 are normal, nothing overflows, and a - b q is a
-// multiple of ulp(b) ulp(q) >= 2^-1074 smaller than 2^53 of them, so the
-// fused multiply-add forms it exactly.  Where |q| is a power of two the
-// spacing below it is half the spacing above, and the test takes the
-// narrower interval on both sides.  That refuses nothing correct: a quotient
-// of two doubles is a power of two p or at least half the spacing above p
-// away from it, so a correct power-of-two quotient is exact (r = 0), and the
-// full-width test would be as sound there.
-// r = 0 is an exact quotient; with a = 0 and b finite and nonzero that is
-// the zero of sign(a) xor sign(b), the sign every quotient is given.
-// Everything else, and any q the test does not accept, clears `ok`; the
-// caller then recomputes with the IEEE division.  (Scaling numerators under
-// 2^-959 by a power of two to keep them on the fast path measured slower than
-// recomputing the few rows that meet them.)
+// The IEEE division and square root that nvcc emits for `a / b` and `sqrt(x)`
+// carry a rarely taken slow path each, and a stage has 20 divisions and five
+// square roots a cell: their branches, not the FP64 arithmetic, held the
+// kernels back.  The forms here have no branch and no rounding test.  They
+// return the IEEE result whenever the operands lie in a safe range; a kernel
+// accumulates the range tests of everything that reaches an output in an
+// F64Range and, where one fails, repeats the work with the IEEE operations
+// before anything is stored.
+//
+// Division a / b (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990; J.-M. Muller
+// et al., Handbook of Floating-Point Arithmetic, 2nd ed., 2018, ch. 4):
+//   * y = recip_f64(b): from the hardware approximation y0 (measured over every
+//     high word: |1 - b y0| < 2^-19.9) three Newton-Raphson steps
+//     y <- y + y (1 - b y).  The second leaves 1/b to 2^-79 and its rounding;
+//     the last one's residual is exact (y is within 0.6 ulp), so y is the
+//     rounding of (1/b)(1 - eta) with 0 <= eta < 2^-105.  One y serves every
+//     quotient by b.
+//   * q0 = a y, r = b q0 - a, q = q0 - r y (quot_f64).  With eps the relative
+//     error of y, q is the rounding of a/b + (a/b - q0) eps.  A quotient of
+//     two doubles stays at least ulp(q) 2^-53 / m_b away from every midpoint
+//     of two doubles (m_b in [1, 2) the significand of b), and |eps| <= m_b
+//     2^-54 + 2^-105.  Next to a midpoint |a/b - q0| is half an ulp, or one and
+//     a half if q0 is not a faithful rounding.  Half an ulp: the
+//     perturbation is smaller than the distance, because m_b <= 2 - 2^-52.
+//     One and a half: q0 = RN(a y) can only be that far off where a's
+//     significand exceeds 2 - 5 2^-52 and b's is larger still, and all
+//     those quotients lie next to a double, not next to a midpoint.  So q =
+//     RN(a / b).
+//   * r = b q0 - a rather than a - b q0 keeps the sign of a zero quotient:
+//     with b > 0, a = -0 gives r = +0 and q = q0 - 0 = -0.
+// Square root (Markstein, as above): h ~ 1 / (2 sqrt(x)) from the hardware
+// approximation (measured: |1 - x y0^2| < 2^-19.0) by two Newton-Raphson steps
+// h <- h + h (1/2 - 2 x h^2), with relative error |eta| < 1.6 2^-53 in the end,
+// and g ~ s = sqrt(x) from the first of them (2^-39), then twice
+// g <- g + (x - g^2) h.  The first leaves g within half an ulp (and a few
+// 2^-26 of one) of s; the second has an exact residual and rounds
+// s - d^2 / (2 s) + d eta (d = s - g).  With s in [1, 2), a midpoint m below s has
+// s - m >= 7 ulp^2 / (8 s) (in units of ulp^2 / 4, m^2 is 1 modulo 8 and x a
+// multiple of 8), and one above s has m - s >= ulp^2 / (8 s), with equality only
+// for x = 1 + ulp and x = 4 - 2 ulp, the next case being 9 times as far: what is
+// added to s stays inside these but for the few arguments that come closest,
+// and tests/test_gpu_div.py runs those.
 #pragma once
 
 #include <cuda_runtime.h>
 
 namespace nestb {
 
-__device__ __forceinline__ unsigned f64_biased_exp(double x) { return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu; }
-
-// Whether a biased exponent lies in [64, 1983] (|x| in [2^-959, 2^961)).
-__device__ __forceinline__ bool f64_exp_safe(unsigned ex) { return ex - 64u < 1920u; }
-
-__device__ __forceinline__ double div_rn_checked(double a, double b, bool& ok) {
+__device__ __forceinline__ double recip_f64(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
     y = fma(y, fma(-b, y, 1.0), y);
     y = fma(y, fma(-b, y, 1.0), y);
-    const double q0 = a * y;
-    const double qm = fma(fma(-b, q0, a), y, q0);
-    const int ha = __double2hiint(a), hb = __double2hiint(b);
-    // the IEEE quotient's sign is sign(a) xor sign(b); setting it also gives
-    // a zero quotient its sign
-    const double q = __hiloint2double((__double2hiint(qm) & 0x7fffffff) | ((ha ^ hb) & (int)0x80000000u),
-                                      __double2loint(qm));
-    const double r = fma(-b, q, a);
-    const int hq = __double2hiint(q);
-    const unsigned exq = ((unsigned)hq >> 20) & 0x7ffu;
-    // ulp(q)/2 = 2^(e(q) - 53): q's exponent field lowered by 53, mantissa 0
-    const double hu = __hiloint2double((int)((unsigned)hq & 0x7ff00000u) - (53 << 20), 0);
-    // |q| a power of two: the spacing below it is half, so the narrower
-    // interval is used on both sides there
-    const bool pow2 = (((unsigned)hq & 0xfffffu) | (unsigned)__double2loint(q)) == 0u;
-    const double thr = fabs(b) * (pow2 ? 0.5 * hu : hu);
-    const bool aok = f64_exp_safe(f64_biased_exp(a));
-    // r = 0: an exact quotient (a = 0 included, b finite and nonzero: else r is NaN)
-    ok = ok && ((aok && f64_exp_safe(exq) && fabs(r) < thr) || (r == 0.0 && (aok || a == 0.0)));
-    return q;
+    return fma(y, fma(-b, y, 1.0), y);
 }
+
+// RN(a / b) for y = recip_f64(b), in range.
+__device__ __forceinline__ double quot_f64(double a, double b, double y) {
+    const double q = a * y;
+    return fma(-fma(b, q, -a), y, q);
+}
+
+// RN(sqrt(x)), in range.
+__device__ __forceinline__ double sqrt_f64(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double x2 = x + x;
+    double h = 0.5 * y;
+    h = fma(h, fma(-(x2 * h), h, 0.5), h);
+    double g = x2 * h;
+    h = fma(h, fma(-g, h, 0.5), h);
+    g = fma(fma(-g, g, x), h, g);
+    return fma(fma(-g, g, x), h, g);
+}
+
+// Whether q = quot_f64(a, b, recip_f64(b)), b > 0, lies where the argument above
+// holds on its own: b in [2^-960, 2^961), and a = 0 or |a| and |q| in
+// [2^-959, 2^961).  (The kernels use the cheaper F64Range, which is narrower.)
+__device__ __forceinline__ bool f64_exp_safe(double x, unsigned lo) {
+    return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - lo < 1984u - lo;
+}
+__device__ __forceinline__ bool quot_in_range(double a, double b, double q) {
+    return f64_exp_safe(b, 63) && (a == 0.0 || (f64_exp_safe(a, 64) && f64_exp_safe(q, 64)));
+}
+
+// Range tests, accumulated over a group of operations and read once.
+//   pos(x): x in [2^-128, 2^128).  Adding a constant to the high word moves
+//     that range of exponents to the top 16th of the exponent field and, for
+//     a positive x, sets the sign bit: the AND over all x keeps the top four
+//     bits set only if every x passes (two integer operations each).
+//   num(a): a = 0 or |a| >= 2^-800.  Twice the high word, less one where the
+//     low word is 0, is 0xffffffff for a zero, below 2 for a subnormal, and
+//     orders by exponent otherwise; the minimum is kept.
+// With b in [2^-129, 2^192) and |a| < 2^880 a quotient whose numerator passes
+// num() is 0 or normal, nothing overflows, and b q - a is a multiple of
+// 2^-1074, so the residual above is exact.
+struct F64Range {
+    unsigned all = 0xffffffffu, low = 0xffffffffu;
+    __device__ __forceinline__ void pos(double x) {
+        all &= (unsigned)__double2hiint(x) + ((897u << 20) ^ 0x80000000u);
+    }
+    __device__ __forceinline__ void num(double a) {
+        const unsigned k = 2u * (unsigned)__double2hiint(a) + (__double2loint(a) != 0 ? 1u : 0u) - 1u;
+        low = min(low, k);
+    }
+    __device__ __forceinline__ bool ok() const { return all >= 0xf0000000u && low >= (223u << 21); }
+};
 
 }  // namespace nestb

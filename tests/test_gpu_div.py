@@ -116,3 +116,83 @@ def test_special_values(gpu):
     assert ok[(a == 0.1) & (b == 0.4)].all() and ok[(a == 3.0) & (b == 3.0)].all()  # exact quotients 0.25 and 1
     # nothing non-finite, zero-divisor or subnormal is accepted
     assert not ok[~np.isfinite(a) | ~np.isfinite(b) | (b == 0)].any()
+
+
+def run_sqrt(lib, x):
+    import torch
+    dx = torch.from_numpy(np.ascontiguousarray(x, dtype=np.float64)).cuda()
+    dr = torch.empty_like(dx)
+    dok = torch.zeros(dx.numel(), dtype=torch.int32, device="cuda")
+    st = lib.nest_selftest_sqrt_f64(C.c_void_p(dx.data_ptr()), C.c_void_p(dr.data_ptr()), C.c_void_p(dok.data_ptr()),
+                                    dx.numel())
+    return st, dr.cpu().numpy(), dok.cpu().numpy().astype(bool)
+
+
+def nearest_to_midpoints(odd, bits):
+    """Every m = 2 k + 1 in [2^53, 2^54) with m^2 = -odd (mod 2^bits), odd = 7
+    (mod 8): then m^2 + odd is a double's significand times a power of two, and
+    its root lies odd quarter ulps^2 over twice itself from the midpoint m / 2
+    (square roots modulo 2^j, lifted one bit at a time)."""
+    roots = {1}
+    for j in range(3, bits):
+        # each root modulo 2^j (up to sign and 2^(j-1)) gives one modulo 2^(j+1)
+        roots = {r if (r * r + odd) % (1 << (j + 1)) == 0 else r + (1 << (j - 1)) for r in roots}
+        assert all((r * r + odd) % (1 << (j + 1)) == 0 for r in roots)
+    out = set()
+    for r in roots:
+        for q in (r, -r, r + (1 << (bits - 1)), -r + (1 << (bits - 1))):
+            q %= 1 << bits
+            out |= {m for m in (q, q + (1 << bits)) if 1 << 53 <= m < 1 << 54}
+    return sorted(out)
+
+
+def test_sqrt_hard_cases(gpu):
+    """The doubles whose square roots come nearest to a midpoint of two doubles,
+    on both sides (x = (m^2 + c) / 4 in units of ulp^2, |c| up to 511), at
+    every scale of the range: each root is the IEEE one."""
+    from nest_b200 import _capi as A
+    xs = []
+    for c in range(-513, 512):
+        if c % 8 != 7:  # m^2 = 1 and x = 0 (mod 8): c = 7 (mod 8), both signs
+            continue
+        for mod in (54, 55):  # x in [1, 2) and x in [2, 4)
+            for m in nearest_to_midpoints(c, mod):
+                x = m * m + c
+                e = x.bit_length() - 53
+                if x % (1 << e) == 0 and x.bit_length() in (107, 108):
+                    xs.append((x >> e) * 2.0 ** (e - 106))
+    xs = np.unique(np.array(xs))
+    assert 1.0 + 2.0 ** -52 in xs and 4.0 - 2.0 ** -51 in xs and len(xs) > 100
+    x = np.concatenate([xs * 4.0 ** k for k in (0, 1, -1, 7, -40, 60, -128, 128)])
+    st, r, ok = run_sqrt(A.lib, x)
+    assert st == A.NEST_OK and ok.all()
+    bad = bits(r) != bits(np.sqrt(x))
+    assert not bad.any(), x[bad][:5]
+
+
+def test_sqrt_wide_range(gpu):
+    from nest_b200 import _capi as A
+    rng = np.random.default_rng(19)
+    n = 4_000_000
+    x = rng.uniform(1.0, 4.0, n) * 4.0 ** rng.integers(-128, 133, n).astype(np.float64)
+    x[: n // 4] = np.nextafter(4.0, 0, dtype=np.float64) - np.spacing(2.0) * rng.integers(0, 1 << 20, n // 4)
+    x[n // 4: n // 2] = 1.0 + np.spacing(1.0) * rng.integers(0, 1 << 20, n // 4)
+    s = rng.uniform(1.0, 2.0, n // 4)
+    x[n // 2: 3 * n // 4] = s * s  # roots next to doubles
+    st, r, ok = run_sqrt(A.lib, x)
+    assert st == A.NEST_OK and ok.all()
+    bad = bits(r) != bits(np.sqrt(x))
+    assert not bad.any(), x[bad][:5]
+
+
+def test_division_divisors_near_two(gpu):
+    """Divisors and numerators with significands next to 2 (where the rounded
+    reciprocal's relative error is largest), all pairs of the last 512."""
+    from nest_b200 import _capi as A
+    k = np.arange(1, 513) * 2.0 ** -52
+    a, b = np.meshgrid(2.0 - k, 2.0 - k, indexing="ij")
+    a, b = a.ravel(), b.ravel()
+    assert check(A.lib, a, b).all()
+    assert check(A.lib, -a * 2.0 ** -700, b * 2.0 ** 37).all()
+    rng = np.random.default_rng(23)
+    assert check(A.lib, rng.uniform(1.0, 2.0, b.size), b).all()
