@@ -689,7 +689,7 @@ def bench_sod1d(reps: int = 20):
     return {"n": n, "bc": "outflow", "cfl": 0.4, "t_final": t, "steps": steps, "ms": m,
             "value": n * steps * 2 / (m * 1e-3), "unit": UNIT, "l1_rho_vs_exact": l1_rho_1d(rho, t),
             "launches": 1, "dtype": "f64",
-            "kernel": "k1d_cluster (one thread-block cluster of 16 CTAs runs the whole loop in shared memory)"}
+            "kernel": "k1d_loop (one thread-block cluster of 16 CTAs runs the whole loop in shared memory)"}
 
 
 def ke_v(U, nx, ny):

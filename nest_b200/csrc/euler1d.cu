@@ -6,10 +6,11 @@
 // and matches it bit for bit.
 //
 // Two execution shapes:
-//   * resident: one CTA holds the whole domain in shared memory and runs the
-//     complete time loop (dt, ghost fill, both stages, Heun average) with no
-//     kernel boundary and no host round-trip per step.  Used while
-//     12 * (n + 4) doubles fit in shared memory.
+//   * resident (k1d_loop): one CTA, or a thread-block cluster of 16 (8), holds
+//     the whole domain on chip and runs the complete time loop (dt, ghost fill,
+//     both stages, Heun average) with no kernel boundary and no host round-trip
+//     per step, up to 4080 cells.  Where no cluster can be placed, one CTA with
+//     several cells per thread (k1d_resident) takes up to about 2300.
 //   * tiled (euler1d_tiled.cuh): a whole step per launch over 224-cell tiles
 //     (the stage-1 halo recomputed per CTA), or the two stage kernels; stage
 //     2 fuses the Heun average, the ghost fill of the new state and the
@@ -21,7 +22,7 @@
 #include <map>
 #include <mutex>
 
-#include "common.cuh"
+#include "euler1d_arith.cuh"
 #include "kernels.h"
 
 namespace nestb {
@@ -50,7 +51,8 @@ __device__ __forceinline__ void ghost_copies_1d(double* A, int nt, int n, int h,
     }
 }
 
-// Resident single-CTA solver: the whole extended domain lives in shared
+// Resident single-CTA solver for devices that cannot place a cluster (more
+// cells than k1d_loop's one CTA takes): the whole extended domain lives in shared
 // memory (U, U1, primitives W, face fluxes F) and the CTA runs the complete
 // time loop.  A step is four phases separated by four barriers:
 //   faces of stage 1 (PLM + HLLE from W)        | update U1, its primitives and ghost copies |
@@ -215,159 +217,106 @@ k1d_resident(double* __restrict__ Ug, int n, int h, double dx, double gamma, int
     }
 }
 
-// Cluster form of the resident solver: a thread-block cluster of NC CTAs
-// (one per SM) splits the cells into NC contiguous chunks and every CTA runs
-// the complete time loop on its chunk in its own shared memory.  A CTA holds
-// its chunk's U and U1, the primitives W of its cells plus two halo cells on
-// each side, and its face fluxes.  Right after computing the primitives of
-// its first two and last two cells it stores them into the halo slots of the
-// neighbouring CTAs (distributed shared memory); W is double-buffered by
-// stage, so one cluster barrier per stage orders those stores against the
-// neighbours' reads.  The wave-speed maximum for dt is reduced over the
-// cluster by reading every CTA's warp maxima after the stage-2 barrier, so
-// all CTAs derive the same dt.  The per-face and per-cell arithmetic is the
-// single-CTA kernel's (nest's OpenMP loop), so the result is the same bit for
-// bit; spreading the FP64 division / square-root work over NC SMs is the gain.
-template <int LIM>
-__global__ void __launch_bounds__(256)
-k1d_cluster(double* __restrict__ Ug, int n, int h, int m, double dx, double gamma, int bc, LoopParams lp,
-            StepCtrl* ctrl, int p) {
+// Max over a warp of a non-negative double's bit pattern: two 32-bit
+// reductions (the high words, then the low words of the lanes that hold the
+// maximum) in place of five shuffle rounds.
+__device__ __forceinline__ double warp_max_speed(double s) {
+    const unsigned hi = (unsigned)__double2hiint(s), lo = (unsigned)__double2loint(s);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    return __hiloint2double((int)mh, (int)ml);
+}
+
+// Largest chunk of the resident loop: cells per CTA (9 warps of 31 cells).
+constexpr int LOOP_WARPS = 9, LOOP_CELLS = 31 * LOOP_WARPS;
+
+// The resident time loop: the NC CTAs of a thread-block cluster (one per SM), or
+// one CTA, split the cells into contiguous chunks of m and run the complete
+// loop.  One thread owns one cell: its U and U1 stay in registers, and only the
+// primitives go through shared memory, with two halo cells on each side.  Lane
+// k of a warp computes the face to the right of cell first + k - 1, and takes the
+// left face of its own cell (k >= 1) from the lane below, so a warp computes 32
+// faces for 31 cells and a stage needs no barrier between its fluxes and its
+// update.  The threads of a CTA's first two and last two cells also store
+// their primitives into the halo slots of the neighbouring CTAs (distributed
+// shared memory); the primitives are double-buffered by stage, so one barrier
+// per stage orders those stores against the reads.  Each warp sends its
+// wave-speed maximum to every CTA before the stage-2 barrier, so after it dt
+// comes from local shared memory, while the stage-1 fluxes (which do not need
+// dt) are computed.
+// What bounds it is one thread's chain of dependent FP64 operations: a step is
+// two face chains and two cell chains, and in a cluster two barriers of about
+// 0.45 us.  Sod tube, us per step (with IEEE divisions and square roots, state in
+// shared memory and a barrier between fluxes and update): 100 cells 1.50 (5.87),
+// 200 cells 1.92 (6.47), both one CTA; 1024 cells on 16 CTAs 2.51 (4.67), 4080
+// cells 3.49 (5.68).
+// LIM: the slope limiter fixed at compile time (LIM_MINMOD, nest's default) or
+// -1 to read it from the loop parameters.
+template <bool CLUSTER, int LIM>
+__global__ void __launch_bounds__(32 * LOOP_WARPS)
+k1d_loop(double* __restrict__ Ug, int n, int h, int m, double dx, double gamma, int bc, LoopParams lp,
+         StepCtrl* ctrl, int p) {
     namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
     extern __shared__ double sm[];
-    const int NC = (int)cl.num_blocks();
-    const int r = (int)cl.block_rank();
-    const int tid = threadIdx.x, T = blockDim.x, nw = (T + 31) >> 5;
+    const int NC = CLUSTER ? (int)cg::this_cluster().num_blocks() : 1;
+    const int r = CLUSTER ? (int)cg::this_cluster().block_rank() : 0;
+    auto sync = [&]() {
+        if (CLUSTER) cg::this_cluster().sync();
+        else __syncthreads();
+    };
+    auto peer = [&](double* a, int rank) { return CLUSTER ? cg::this_cluster().map_shared_rank(a, rank) : a; };
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int nt = n + 2 * h;
     const int c_lo = r * m, mloc = min(n, c_lo + m) - c_lo;  // this CTA's cells [c_lo, c_lo + mloc)
     const int mw = m + 4;                                     // W row: 2 halo slots each side
-    double* U = sm;                  // [3][m]
-    double* U1 = U + 3 * m;          // [3][m]
-    double* W = U1 + 3 * m;          // [2][3][mw]: buffer b, variable k, local cell l at 2 + l
-    double* F = W + 6 * mw;          // [3][m + 1]
-    double* red = F + 3 * (m + 1);   // [32] warp maxima
-    const double gm1 = gamma - 1.0;
+    double* const W = sm;             // [2][3][mw]: buffer b, variable k, local cell l at 2 + l
+    double* const red = W + 6 * mw;   // [NC * nw] wave-speed maxima of every warp
+    const Gas<double> gas(gamma);
     const int left = (r + NC - 1) % NC, right = (r + 1) % NC;
     const int mloc_left = min(n, left * m + m) - left * m;
-    auto Wb = [&](int b) { return W + b * 3 * mw; };
-    // W buffer b of CTA `rank`, variable k, local slot s (halo slots 0, 1 and mloc + 2, mloc + 3)
-    auto peerW = [&](int rank, int b, int k, int slot) {
-        return cl.map_shared_rank(W, rank) + b * 3 * mw + k * mw + slot;
-    };
-    // primitives of local cell l into buffer b, plus the halo copies it feeds
-    auto prims_of = [&](int l, double rr, double mm, double ee, int b) {
-        const double u = mm / rr;
-        const double pr = eos_pressure(gm1, rr, mm, ee);
-        const double v[3] = { rr, u, pr };
-        double* w = Wb(b);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) w[k * mw + 2 + l] = v[k];
-        const int c = c_lo + l;
-        if (bc == BC_PERIODIC) {
-            // first two cells -> right halo of the left neighbour; last two -> left halo of the right neighbour
-            if (l < 2)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) *peerW(left, b, k, mloc_left + 2 + l) = v[k];
-            if (l >= mloc - 2)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) *peerW(right, b, k, l - (mloc - 2)) = v[k];
-        } else {
-            if (l < 2 && r > 0)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) *peerW(left, b, k, mloc_left + 2 + l) = v[k];
-            if (l >= mloc - 2 && r < NC - 1)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) *peerW(right, b, k, l - (mloc - 2)) = v[k];
-            if (c == 0)  // zero-gradient ghosts of the domain's first cell
-#pragma unroll
-                for (int k = 0; k < 3; ++k) { w[k * mw + 0] = v[k]; w[k * mw + 1] = v[k]; }
-            if (c == n - 1)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) { w[k * mw + mloc + 2] = v[k]; w[k * mw + mloc + 3] = v[k]; }
-        }
-    };
-    auto speeds = [&](int b) {
-        double ms = 0.0;
-        for (int l = tid; l < mloc; l += T) {
-            const double* w = Wb(b);
-            const double rr = w[2 + l], u = w[mw + 2 + l], pr = w[2 * mw + 2 + l];
-            const double cs = sqrt(gamma * pr / rr);
-            ms = smax(ms, fabs(u) + cs);
-        }
-        ms = warp_max(ms);
-        if ((tid & 31) == 0) red[tid >> 5] = ms;
-    };
-    // max over every CTA's warp maxima: each lane reads its share of the
-    // NC * nw values (remote loads in parallel), then a warp max; every warp
-    // computes the same value, so all threads hold the same dt
-    auto cluster_max = [&]() {
-        double ms = 0.0;
-        const int lane = tid & 31, total = NC * nw;
-        for (int q = lane; q < total; q += 32) ms = smax(ms, cl.map_shared_rank(red, q / nw)[q % nw]);
-        return warp_max(ms);
+
+    const int l = 31 * warp + lane - 1;       // this lane's face is to the right of local cell l
+    const bool own = lane >= 1 && l < mloc;   // and it owns cell l
+    const int c = c_lo + l;
+    const int ls = min(l, mloc - 1);          // lanes past the chunk repeat its last face
+
+    // stores the primitives of the own cell into buffer b and the halo slots it feeds
+    auto put = [&](int b, double v0, double v1, double v2) {
+        auto to = [&](double* base, int slot) {
+            double* w = base + b * 3 * mw + slot;
+            w[0] = v0; w[mw] = v1; w[2 * mw] = v2;
+        };
+        to(W, 2 + l);
+        const bool per = bc == BC_PERIODIC;
+        if (l < 2 && (per || r > 0)) to(peer(W, left), mloc_left + 2 + l);
+        if (l >= mloc - 2 && (per || r < NC - 1)) to(peer(W, right), l - (mloc - 2));
+        if (!per && c == 0) { to(W, 0); to(W, 1); }
+        if (!per && c == n - 1) { to(W, mloc + 2); to(W, mloc + 3); }
     };
     auto faces = [&](int b) {
-        const double* Wc = Wb(b);
-        for (int f = tid; f <= mloc; f += T) {
-            // face between local cells f-1 and f: W slots a = f + 1, b = f + 2
-            const int a = f + 1, bb = f + 2;
-            double sa[3], sb[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const double* w = Wc + k * mw;
-                sa[k] = limit(w[a] - w[a - 1], w[bb] - w[a], LIM >= 0 ? LIM : lp.lim);
-                sb[k] = limit(w[bb] - w[a], w[bb + 1] - w[bb], LIM >= 0 ? LIM : lp.lim);
-            }
-            const double rL = Wc[a] + 0.5 * sa[0], uL = Wc[mw + a] + 0.5 * sa[1], pL = Wc[2 * mw + a] + 0.5 * sa[2];
-            const double rR = Wc[bb] - 0.5 * sb[0], uR = Wc[mw + bb] - 0.5 * sb[1], pR = Wc[2 * mw + bb] - 0.5 * sb[2];
-            double f0, f1, f2;
-            hlle1d(gamma, gm1, rL, uL, pL, rR, uR, pR, f0, f1, f2);
-            F[f] = f0; F[(m + 1) + f] = f1; F[2 * (m + 1) + f] = f2;
-        }
+        const double* w = W + b * 3 * mw + ls + 1;
+        return plm_flux(gas, LIM >= 0 ? LIM : lp.lim, [&](int k, int s) { return w[k * mw + s]; }, 0, 1, 2, 3);
     };
-    // stage update of this CTA's cells; in stage 2 (heun) also the max |u|+c
-    // of the new state (same formulas as `speeds`) into red and the
-    // positivity check of step `step_done`: a failing cell makes the maximum
-    // infinite, which ends the loop on every CTA of the cluster
-    auto update = [&](const double* Uin, double* Uout, bool heun, double dtdx, int bnext, int step_done) {
-        double ms = 0.0;
-        for (int l = tid; l < mloc; l += T) {
-            double v[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                v[k] = Uin[k * m + l] - dtdx * (F[k * (m + 1) + l + 1] - F[k * (m + 1) + l]);
-                if (heun) v[k] = 0.5 * (Uout[k * m + l] + v[k]);
-                Uout[k * m + l] = v[k];
-            }
-            prims_of(l, v[0], v[1], v[2], bnext);
-            if (heun) {
-                const double* w = Wb(bnext);
-                const double rr = w[2 + l], u = w[mw + 2 + l], pr = w[2 * mw + 2 + l];
-                const double cs = sqrt(gamma * pr / rr);
-                ms = smax(ms, fabs(u) + cs);
-                if (!(rr > 0.0) || !(pr > 0.0)) {
-                    flag_cell(ctrl, step_done, rr, pr, c_lo + l, 0);
-                    ms = __longlong_as_double(0x7ff0000000000000ll);
-                }
-            }
-        }
-        if (heun) {
-            ms = warp_max(ms);
-            if ((tid & 31) == 0) red[tid >> 5] = ms;
-        }
+    auto send_max = [&](double s) {
+        s = warp_max_speed(s);
+        if (lane < NC) peer(red, lane)[r * nw + warp] = s;
+    };
+    auto read_max = [&]() {
+        double s = 0.0;
+        for (int q = lane; q < NC * nw; q += 32) s = smax(s, red[q]);
+        return warp_max_speed(s);
     };
 
-    // prologue: this CTA's cells, their primitives (buffer 0) and the first dt
-    for (int i = tid; i < 3 * m; i += T) {
-        const int k = i / m, l = i - k * m;
-        U[i] = l < mloc ? Ug[k * nt + h + c_lo + l] : 0.0;
-        U1[i] = 0.0;
+    // prologue: the own cell, its primitives (buffer 0) and the first wave speeds
+    double u0 = 1.0, u1 = 0.0, u2 = 1.0;
+    if (own) { u0 = Ug[h + c]; u1 = Ug[nt + h + c]; u2 = Ug[2 * nt + h + c]; }
+    if (CLUSTER) sync();  // every CTA of the cluster runs before its memory is written
+    {
+        const Cell1<double> w = cell1d<true>(gas, u0, u1, u2);
+        if (own) put(0, u0, w.u, w.p);
+        send_max(own ? smax(0.0, fabs(w.u) + w.cs) : 0.0);
     }
-    __syncthreads();
-    for (int l = tid; l < mloc; l += T) prims_of(l, U[l], U[m + l], U[2 * m + l], 0);
-    cl.sync();
-    speeds(0);
-    cl.sync();
+    sync();
 
     double time = ctrl->time[p];
     int step = ctrl->step[p];
@@ -378,51 +327,72 @@ k1d_cluster(double* __restrict__ Ug, int n, int h, int m, double dx, double gamm
         if (lp.t_final > 0.0 && !(time < lp.t_final)) break;
         if (lp.max_steps > 0 && step >= lp.max_steps) break;
         if (lp.dts_in && step >= lp.dts_cap) break;
-        // the stage-1 fluxes do not depend on dt: compute them while the
-        // cluster-wide maximum (remote loads) and dt are in flight
-        faces(0);
-        const double ms = cluster_max();
+        const double ms = read_max();
+        const F3<double> f = faces(0);
         double dt;
         if (lp.fixed_dt > 0.0) {
             dt = lp.fixed_dt;
         } else if (lp.dts_in) {
             dt = lp.dts_in[step];
         } else {
-            dt = lp.cfl * dx / ms;
+            dt = div_rn(lp.cfl * dx, ms);
             if (lp.t_final > 0.0) dt = smin(dt, lp.t_final - time);
         }
-        if (!(ms == ms) || ms > 1.79e308) { if (r == 0 && tid == 0) atomicOr(&ctrl->err, ERRW_NONFINITE); break; }
-        if (r == 0 && tid == 0 && lp.dts_out && step < lp.dts_cap) lp.dts_out[step] = dt;
-        const double dtdx = dt / dx;
-        __syncthreads();                // stage 1 fluxes (from W0 = prims(U)) complete
-        update(U, U1, false, dtdx, 1, 0);  // U1, W1 = prims(U1) and the neighbours' halos
-        cl.sync();
-        faces(1);                       // stage 2 fluxes
-        __syncthreads();
-        update(U1, U, true, dtdx, 0, step + 1);  // U = (U + U1 - dt L(U1)) / 2, W0 = prims(U), max |u|+c
-        cl.sync();
+        if (!(ms == ms) || ms > 1.79e308) { if (r == 0 && threadIdx.x == 0) atomicOr(&ctrl->err, ERRW_NONFINITE); break; }
+        if (r == 0 && threadIdx.x == 0 && lp.dts_out && step < lp.dts_cap) lp.dts_out[step] = dt;
+        const double dtdx = div_rn(dt, dx);
+        // stage 1: U1 = U - dtdx (F_right - F_left)
+        const double v0 = u0 - dtdx * (f.a - __shfl_up_sync(0xffffffffu, f.a, 1));
+        const double v1 = u1 - dtdx * (f.b - __shfl_up_sync(0xffffffffu, f.b, 1));
+        const double v2 = u2 - dtdx * (f.c - __shfl_up_sync(0xffffffffu, f.c, 1));
+        {
+            const Cell1<double> w = cell1d<false>(gas, v0, v1, v2);
+            if (own) put(1, v0, w.u, w.p);
+        }
+        sync();
+        // stage 2: U = (U + U1 - dtdx (F_right - F_left)) / 2, its wave speed
+        // and positivity (a failing cell makes the maximum infinite, which
+        // ends the loop on every CTA)
+        const F3<double> e = faces(1);
+        u0 = 0.5 * (u0 + (v0 - dtdx * (e.a - __shfl_up_sync(0xffffffffu, e.a, 1))));
+        u1 = 0.5 * (u1 + (v1 - dtdx * (e.b - __shfl_up_sync(0xffffffffu, e.b, 1))));
+        u2 = 0.5 * (u2 + (v2 - dtdx * (e.c - __shfl_up_sync(0xffffffffu, e.c, 1))));
+        {
+            const Cell1<double> w = cell1d<true>(gas, u0, u1, u2);
+            double s = 0.0;
+            if (own) {
+                put(0, u0, w.u, w.p);
+                s = smax(0.0, fabs(w.u) + w.cs);
+                if (!(u0 > 0.0) || !(w.p > 0.0)) {
+                    flag_cell(ctrl, step + 1, u0, w.p, c, 0);
+                    s = __longlong_as_double(0x7ff0000000000000ll);
+                }
+            }
+            send_max(s);
+        }
+        sync();
         time += dt;
         ++step;
     }
     // state and the domain's ghost cells back to global memory
-    for (int i = tid; i < 3 * mloc; i += T) {
-        const int k = i / mloc, l = i - k * mloc;
-        const double v = U[k * m + l];
-        const int c = c_lo + l;
-        Ug[k * nt + h + c] = v;
-        if (bc == BC_PERIODIC) {
-            if (c >= n - h) Ug[k * nt + c + h - n] = v;
-            if (c < h) Ug[k * nt + h + n + c] = v;
-        } else {
-            if (c == 0) for (int e = 0; e < h; ++e) Ug[k * nt + e] = v;
-            if (c == n - 1) for (int e = h + n; e < nt; ++e) Ug[k * nt + e] = v;
+    if (own) {
+        const double v[3] = { u0, u1, u2 };
+        for (int k = 0; k < 3; ++k) {
+            Ug[k * nt + h + c] = v[k];
+            if (bc == BC_PERIODIC) {
+                if (c >= n - h) Ug[k * nt + c + h - n] = v[k];
+                if (c < h) Ug[k * nt + h + n + c] = v[k];
+            } else {
+                if (c == 0) for (int g = 0; g < h; ++g) Ug[k * nt + g] = v[k];
+                if (c == n - 1) for (int g = h + n; g < nt; ++g) Ug[k * nt + g] = v[k];
+            }
         }
     }
-    if (r == 0 && tid == 0) {
+    if (r == 0 && threadIdx.x == 0) {
         ctrl->time[p] = time; ctrl->step[p] = step;
         ctrl->time[p ^ 1] = time; ctrl->step[p ^ 1] = step;
     }
-    cl.sync();  // no CTA leaves while a neighbour may still read its shared memory
+    if (CLUSTER) sync();  // no CTA leaves while a neighbour's stores to it may be in flight
 }
 
 size_t resident_smem_bytes(int n, int h) {
@@ -430,48 +400,67 @@ size_t resident_smem_bytes(int n, int h) {
     return sizeof(double) * (size_t)(9 * nt + 3 * (n + 1) + 33);
 }
 
-// Cluster launch of the resident solver with NC CTAs; returns
-// cudaErrorNotSupported (nothing launched) when the chunk sizes or the
+// Launch of the resident loop with a cluster of NC CTAs (1: a plain launch).
+struct LoopShape {
+    int m, threads;
+    size_t smem;
+};
+// Chunk and block size for n cells on NC CTAs; false where they do not fit
+// (every CTA of a cluster needs two cells for the halos).
+static bool loop_shape(int n, int NC, LoopShape& s) {
+    s.m = (n + NC - 1) / NC;
+    if (s.m > LOOP_CELLS || (NC > 1 && (s.m < 2 || n - (NC - 1) * s.m < 2))) return false;
+    s.threads = (s.m + 30) / 31 * 32;
+    s.smem = sizeof(double) * (size_t)(6 * (s.m + 4) + NC * (s.threads / 32));
+    return true;
+}
+
+template <class K>
+static cudaError_t cluster_config(K kern, int NC, const LoopShape& s, cudaLaunchConfig_t& cfg,
+                                  cudaLaunchAttribute* at, int& clusters) {
+    cudaError_t e;
+    clusters = 0;
+    if (NC > 8 && (e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
+        return e;
+    cfg = {};
+    cfg.gridDim = dim3(NC, 1, 1);
+    cfg.blockDim = dim3(s.threads, 1, 1);
+    cfg.dynamicSmemBytes = s.smem;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = NC;
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if ((e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg)) != cudaSuccess) {
+        cudaGetLastError();
+        clusters = 0;
+    }
+    return cudaSuccess;
+}
+
+// Returns cudaErrorNotSupported (nothing launched) when the chunk sizes or the
 // device's cluster occupancy do not allow that cluster size.
 static cudaError_t launch_1d_cluster(double* U, int n, int h, double dx, double gamma, int bc, const LoopParams& lp,
                                      StepCtrl* ctrl, int p, cudaStream_t st, int NC) {
-    const int m = (n + NC - 1) / NC;
-    if (m < 2 || n - (NC - 1) * m < 2) return cudaErrorNotSupported;  // every CTA needs two cells for the halos
-    const int threads = (m + 1 + 31) / 32 * 32;
-    if (threads > 256) return cudaErrorNotSupported;
-    const size_t smem = sizeof(double) * (size_t)(3 * m + 3 * m + 6 * (m + 4) + 3 * (m + 1) + 32);
-    auto kern = lp.lim == LIM_MINMOD ? k1d_cluster<LIM_MINMOD> : k1d_cluster<-1>;
-    cudaError_t e;
-    if (NC > 8 && (e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
-        return e;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
-        return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(NC, 1, 1);
-    cfg.blockDim = dim3(threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = NC;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if ((e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg)) != cudaSuccess) {
-        cudaGetLastError();
-        return cudaErrorNotSupported;
-    }
+    LoopShape s;
+    if (!loop_shape(n, NC, s)) return cudaErrorNotSupported;
+    auto kern = lp.lim == LIM_MINMOD ? k1d_loop<true, LIM_MINMOD> : k1d_loop<true, -1>;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    int clusters;
+    cudaError_t e = cluster_config(kern, NC, s, cfg, &at, clusters);
+    if (e != cudaSuccess) return e;
     if (clusters < 1) return cudaErrorNotSupported;
-    return cudaLaunchKernelEx(&cfg, kern, U, n, h, m, dx, gamma, bc, lp, ctrl, p);
+    cfg.stream = st;
+    return cudaLaunchKernelEx(&cfg, kern, U, n, h, s.m, dx, gamma, bc, lp, ctrl, p);
 }
 
 // Whether launch_1d_cluster can place a cluster of 16 or 8 CTAs for n cells
 // on the current device (the chunk-size rules and the cluster occupancy query
 // of launch_1d_cluster, with nothing launched); remembered per device and n.
 bool cluster_1d_available(int n, int h) {
-    if (n < 256) return false;
+    if (n < 256 || n > 4080) return false;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     static std::mutex mu;
@@ -481,34 +470,14 @@ bool cluster_1d_available(int n, int h) {
     if (it != known.end()) return it->second;
     bool ok = false;
     for (int NC : {16, 8}) {
-        const int m = (n + NC - 1) / NC;
-        if (m < 2 || n - (NC - 1) * m < 2) continue;
-        const int threads = (m + 1 + 31) / 32 * 32;
-        if (threads > 256) continue;
-        const size_t smem = sizeof(double) * (size_t)(3 * m + 3 * m + 6 * (m + 4) + 3 * (m + 1) + 32);
+        LoopShape s;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        int clusters = 0;
+        if (!loop_shape(n, NC, s)) continue;
         // both limiter instances use the same threads and shared memory; the
         // minmod one stands for both
-        if (NC > 8 && cudaFuncSetAttribute(k1d_cluster<LIM_MINMOD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-            cudaGetLastError();
-            continue;
-        }
-        if (cudaFuncSetAttribute(k1d_cluster<LIM_MINMOD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            cudaGetLastError();
-            continue;
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(NC, 1, 1);
-        cfg.blockDim = dim3(threads, 1, 1);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = NC;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, k1d_cluster<LIM_MINMOD>, &cfg) != cudaSuccess) {
+        if (cluster_config(k1d_loop<true, LIM_MINMOD>, NC, s, cfg, &at, clusters) != cudaSuccess) {
             cudaGetLastError();
             continue;
         }
@@ -520,12 +489,21 @@ bool cluster_1d_available(int n, int h) {
 
 cudaError_t launch_1d_resident(double* U, int n, int h, double dx, double gamma, int bc,
                                const LoopParams& lp, StepCtrl* ctrl, int p, cudaStream_t st) {
-    // 256 cells or more: a cluster of 16 (else 8) CTAs, one per SM
-    if (n >= 256) {
-        for (int NC : {16, 8}) {
-            cudaError_t e = launch_1d_cluster(U, n, h, dx, gamma, bc, lp, ctrl, p, st, NC);
-            if (e != cudaErrorNotSupported) return e;
-        }
+    const bool mm = lp.lim == LIM_MINMOD;
+    // up to 279 cells one CTA, whose barrier is cheap (256 cells: 2.39 us a step
+    // on one CTA, 2.43 on a cluster; 434: 2.96 on one CTA of 14 warps, 2.39 on a
+    // cluster)
+    if (n <= LOOP_CELLS) {
+        LoopShape s;
+        loop_shape(n, 1, s);
+        (mm ? k1d_loop<false, LIM_MINMOD> : k1d_loop<false, -1>)<<<1, s.threads, s.smem, st>>>(U, n, h, s.m, dx, gamma,
+                                                                                         bc, lp, ctrl, p);
+        return cudaGetLastError();
+    }
+    // a cluster of 16 (else 8) CTAs, one per SM
+    for (int NC : {16, 8}) {
+        cudaError_t e = launch_1d_cluster(U, n, h, dx, gamma, bc, lp, ctrl, p, st, NC);
+        if (e != cudaErrorNotSupported) return e;
     }
     size_t smem = resident_smem_bytes(n, h);
     // K faces per thread: at least two (independent FP64 chains per thread),
@@ -540,7 +518,6 @@ cudaError_t launch_1d_resident(double* U, int n, int h, double dx, double gamma,
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess) kern<<<1, threads, smem, st>>>(U, n, h, dx, gamma, bc, lp, ctrl, p);
     };
-    const bool mm = lp.lim == LIM_MINMOD;
     if (K == 2 && threads <= 640) mm ? go(k1d_resident<2, 640, LIM_MINMOD>) : go(k1d_resident<2, 640, -1>);
     else if (K == 2) mm ? go(k1d_resident<2, 1024, LIM_MINMOD>) : go(k1d_resident<2, 1024, -1>);
     else mm ? go(k1d_resident<3, 1024, LIM_MINMOD>) : go(k1d_resident<3, 1024, -1>);

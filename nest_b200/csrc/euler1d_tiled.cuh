@@ -13,7 +13,7 @@
 // recomputing the stage-1 halo per CTA.
 #pragma once
 
-#include "common.cuh"
+#include "euler1d_arith.cuh"
 #include "kernels.h"
 
 namespace nestb {
@@ -26,16 +26,6 @@ constexpr int T1 = 224;
 // phase loops twice, in whole warps (the stage-2 reduction shuffles over
 // full warps)
 constexpr int NT1 = T1 + 32;
-
-// Max |u|+c of one cell (benchmark_euler1d.cpp:170-178); p receives the
-// cell's pressure (eos_t::pressure, clamped at 0) for the positivity check.
-template <typename T>
-__device__ __forceinline__ T cell_speed_1d(T rho, T mom, T erg, T gamma, T gm1, T& p) {
-    T u = mom / rho;
-    p = eos_pressure(gm1, rho, mom, erg);
-    T c = sqrt(gamma * p / rho);
-    return fabs(u) + c;
-}
 
 // Writes the ghost copies that the value of interior cell c (0-based) feeds.
 template <typename T>
@@ -61,8 +51,7 @@ k1d_stage(const T* __restrict__ Uin, const T* Un, T* Uout,
     pdl_wait();
     pdl_trigger();
     int nt = n + 2 * h;
-    const T gamma = (T)gamma_d;
-    const T gm1 = (T)(gamma_d - 1.0);
+    const Gas<T> gas(gamma_d);
     double dt;
     if (STAGE == 1) {
         bool done = step_is_done(ctrl, p, lp);
@@ -85,24 +74,16 @@ k1d_stage(const T* __restrict__ Uin, const T* Un, T* Uout,
     for (int t = threadIdx.x; t < T1 + 4; t += NT1) {
         int e = min(h + c0 - 2 + t, nt - 1);
         T rho = Uin[e], mom = Uin[nt + e], erg = Uin[2 * nt + e];
+        const Cell1<T> w = cell1d<false>(gas, rho, mom, erg);
         W[0][t] = rho;
-        W[1][t] = mom / rho;
-        W[2][t] = eos_pressure(gm1, rho, mom, erg);
+        W[1][t] = w.u;
+        W[2][t] = w.p;
     }
     __syncthreads();
     int nf = min(T1, n - c0) + 1;  // faces of this tile
     for (int f = threadIdx.x; f < nf; f += NT1) {
-        int a = f + 1, b = f + 2;  // tile-local W indices around the face
-        T sa[3], sb[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            sa[k] = limit(W[k][a] - W[k][a - 1], W[k][b] - W[k][a], LIM >= 0 ? LIM : lp.lim);
-            sb[k] = limit(W[k][b] - W[k][a], W[k][b + 1] - W[k][b], LIM >= 0 ? LIM : lp.lim);
-        }
-        T f0, f1, f2;
-        hlle1d(gamma, gm1, W[0][a] + T(0.5) * sa[0], W[1][a] + T(0.5) * sa[1], W[2][a] + T(0.5) * sa[2],
-               W[0][b] - T(0.5) * sb[0], W[1][b] - T(0.5) * sb[1], W[2][b] - T(0.5) * sb[2], f0, f1, f2);
-        F[0][f] = f0; F[1][f] = f1; F[2][f] = f2;
+        const F3<T> q = plm_flux(gas, LIM >= 0 ? LIM : lp.lim, [&](int k, int t) { return W[k][t]; }, f, f + 1, f + 2, f + 3);
+        F[0][f] = q.a; F[1][f] = q.b; F[2][f] = q.c;
     }
     __syncthreads();
     int c = c0 + threadIdx.x;
@@ -121,9 +102,9 @@ k1d_stage(const T* __restrict__ Uin, const T* Un, T* Uout,
             push_ghosts_1d(Uout, nt, k, c, n, h, bc, v[k]);
         }
         if (STAGE == 2) {
-            T pr;
-            ms = (double)cell_speed_1d(v[0], v[1], v[2], gamma, gm1, pr);
-            if (!(v[0] > T(0)) || !(pr > T(0))) flag_cell(ctrl, ctrl->step[p] + 1, (double)v[0], (double)pr, c, 0);
+            const Cell1<T> w = cell1d<true>(gas, v[0], v[1], v[2]);
+            ms = (double)(fabs(w.u) + w.cs);
+            if (!(v[0] > T(0)) || !(w.p > T(0))) flag_cell(ctrl, ctrl->step[p] + 1, (double)v[0], (double)w.p, c, 0);
         }
     }
     if (STAGE == 2) {
@@ -182,8 +163,7 @@ k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out,
     pdl_wait();
     pdl_trigger();
     const int nt = n + 2 * h;
-    const T gamma = (T)gamma_d;
-    const T gm1 = (T)(gamma_d - 1.0);
+    const Gas<T> gas(gamma_d);
     const int c0 = blockIdx.x * T1;
     if (step_is_done(ctrl, p, lp)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) publish_step(ctrl, p, lp, true, 0.0, false);
@@ -217,25 +197,17 @@ k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out,
         const int e = h + source_cell_1d(c0 - 4 + t, n, bc);
         const T rho = Un[e], mom = Un[nt + e], erg = Un[2 * nt + e];
         Q[0][t] = rho; Q[1][t] = mom; Q[2][t] = erg;
+        const Cell1<T> w = cell1d<false>(gas, rho, mom, erg);
         W[0][t] = rho;
-        W[1][t] = mom / rho;
-        W[2][t] = eos_pressure(gm1, rho, mom, erg);
+        W[1][t] = w.u;
+        W[2][t] = w.p;
     }
     __syncthreads();
     // face f between the cells of W slots f+1 and f+2
     auto faces = [&](int nf) {
         for (int f = threadIdx.x; f < nf; f += NT1) {
-            const int a = f + 1, b = f + 2;
-            T sa[3], sb[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                sa[k] = limit(W[k][a] - W[k][a - 1], W[k][b] - W[k][a], LIM >= 0 ? LIM : lp.lim);
-                sb[k] = limit(W[k][b] - W[k][a], W[k][b + 1] - W[k][b], LIM >= 0 ? LIM : lp.lim);
-            }
-            T f0, f1, f2;
-            hlle1d(gamma, gm1, W[0][a] + T(0.5) * sa[0], W[1][a] + T(0.5) * sa[1], W[2][a] + T(0.5) * sa[2],
-                   W[0][b] - T(0.5) * sb[0], W[1][b] - T(0.5) * sb[1], W[2][b] - T(0.5) * sb[2], f0, f1, f2);
-            F[0][f] = f0; F[1][f] = f1; F[2][f] = f2;
+            const F3<T> q = plm_flux(gas, LIM >= 0 ? LIM : lp.lim, [&](int k, int t) { return W[k][t]; }, f, f + 1, f + 2, f + 3);
+            F[0][f] = q.a; F[1][f] = q.b; F[2][f] = q.c;
         }
     };
     faces(T1 + 5);  // stage 1: faces between cells c0-3+f and c0-2+f
@@ -251,9 +223,10 @@ k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out,
             v[k] = Q[k][us + 2] - dtdx * (F[k][us + 1] - F[k][us]);
             V[k][u] = v[k];
         }
+        const Cell1<T> w = cell1d<false>(gas, v[0], v[1], v[2]);
         W[0][u] = v[0];
-        W[1][u] = v[1] / v[0];
-        W[2][u] = eos_pressure(gm1, v[0], v[1], v[2]);
+        W[1][u] = w.u;
+        W[2][u] = w.p;
     }
     __syncthreads();
     faces(T1 + 1);  // stage 2: faces between cells c0-1+f and c0+f
@@ -277,9 +250,9 @@ k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out,
                 push_ghosts_1d(U1out, nt, k, c, n, h, bc, V[k][t + 2]);
             }
         }
-        T pr;
-        ms = (double)cell_speed_1d(v[0], v[1], v[2], gamma, gm1, pr);
-        if (!(v[0] > T(0)) || !(pr > T(0))) flag_cell(ctrl, ctrl->step[p] + 1, (double)v[0], (double)pr, c, 0);
+        const Cell1<T> w = cell1d<true>(gas, v[0], v[1], v[2]);
+        ms = (double)(fabs(w.u) + w.cs);
+        if (!(v[0] > T(0)) || !(w.p > T(0))) flag_cell(ctrl, ctrl->step[p] + 1, (double)v[0], (double)w.p, c, 0);
     }
     ms = warp_max(ms);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -312,8 +285,7 @@ k1d_prepare(T* U, int n, int h, double gamma_d, int bc, StepCtrl* ctrl, int p) {
     pdl_wait();
     pdl_trigger();
     int nt = n + 2 * h;
-    const T gamma = (T)gamma_d;
-    const T gm1 = (T)(gamma_d - 1.0);
+    const Gas<T> gas(gamma_d);
     int c = blockIdx.x * T1 + threadIdx.x;
     double ms = 0.0;
     if (c < n) {
@@ -322,8 +294,8 @@ k1d_prepare(T* U, int n, int h, double gamma_d, int bc, StepCtrl* ctrl, int p) {
         push_ghosts_1d(U, nt, 0, c, n, h, bc, v0);
         push_ghosts_1d(U, nt, 1, c, n, h, bc, v1);
         push_ghosts_1d(U, nt, 2, c, n, h, bc, v2);
-        T pr;
-        ms = (double)cell_speed_1d(v0, v1, v2, gamma, gm1, pr);
+        const Cell1<T> w = cell1d<true>(gas, v0, v1, v2);
+        ms = (double)(fabs(w.u) + w.cs);
     }
     ms = warp_max(ms);
     int w = threadIdx.x >> 5, l = threadIdx.x & 31;

@@ -40,11 +40,9 @@ __device__ __forceinline__ void cpd_wait() { asm volatile("cp.async.wait_group %
 
 using W4 = Win4<double>;
 
-// Arithmetic policies of a row: the IEEE division and square root, or the
-// branch-free ones of f64div.cuh with their range tests.  Both give the same
-// values wherever the tests pass; a row in which one fails for a lane that can
-// reach an output is computed again with the IEEE policy before anything of it
-// is stored.
+// A row runs with ArithFast (f64div.cuh); one in which a range test fails for a
+// lane that can reach an output is computed again with ArithIeee before anything
+// of it is stored.
 //
 // What the tests rest on.  prim() tests rho and p of every cell the row adds to
 // the window (and the two momenta as numerators); a finite u or v follows, with
@@ -57,32 +55,6 @@ using W4 = Win4<double>;
 // average flux is taken, and its numerators stay under 2^880; the mass,
 // transverse and energy ones, which can be tiny, are tested (the normal one
 // holds SR p - SL p, which cannot).
-struct ArithIeee {
-    static constexpr bool checked = false;
-    struct Recip { double b; };
-    __device__ __forceinline__ Recip recip(double b) const { return { b }; }
-    __device__ __forceinline__ double quot(double a, const Recip& r) const { return a / r.b; }
-    __device__ __forceinline__ double root(double x) const { return sqrt(x); }
-    __device__ __forceinline__ double half(double w, double h, double s) const { return w + h * s; }
-    __device__ __forceinline__ void pos(double) {}
-    __device__ __forceinline__ void num(double) {}
-    __device__ __forceinline__ bool ok() const { return true; }
-};
-struct ArithFast {
-    static constexpr bool checked = true;
-    struct Recip { double b, y; };
-    F64Range r;
-    __device__ __forceinline__ Recip recip(double b) const { return { b, recip_f64(b) }; }
-    __device__ __forceinline__ double quot(double a, const Recip& q) const { return quot_f64(a, q.b, q.y); }
-    __device__ __forceinline__ double root(double x) const { return sqrt_f64(x); }
-    // h = +-1/2: h s is exact (slopes in range are multiples of 2^-1000), so the
-    // fused form rounds the same sum
-    __device__ __forceinline__ double half(double w, double h, double s) const { return fma(h, s, w); }
-    __device__ __forceinline__ void pos(double x) { r.pos(x); }
-    __device__ __forceinline__ void num(double a) { r.num(a); }
-    __device__ __forceinline__ bool ok() const { return r.ok(); }
-};
-
 // Face states w + s/2 and w - s/2.
 template <class A>
 __device__ __forceinline__ W4 face_up(const A& m, const W4& w, const W4& s) {

@@ -78,6 +78,28 @@ __device__ __forceinline__ double sqrt_f64(double x) {
     return fma(fma(-g, g, x), h, g);
 }
 
+// RN(sqrt(q)) with q = RN(a / b), in range, and the reciprocal of b: the same
+// steps as recip_f64, quot_f64 and sqrt_f64, with the square root's first
+// approximation taken from a quotient of 2^-39 relative error, so that it runs
+// beside the exact quotient instead of after it (the second Newton-Raphson step
+// of h and everything after it use the exact q).
+__device__ __forceinline__ double sqrt_quot_f64(double a, double b, double& y) {
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = fma(y, fma(-b, y, 1.0), y);
+    const double t = a * y, t2 = t + t;
+    double h;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(h) : "d"(t));
+    h *= 0.5;
+    h = fma(h, fma(-(t2 * h), h, 0.5), h);
+    y = fma(y, fma(-b, y, 1.0), y);
+    y = fma(y, fma(-b, y, 1.0), y);
+    const double q = quot_f64(a, b, y);
+    double g = (q + q) * h;
+    h = fma(h, fma(-g, h, 0.5), h);
+    g = fma(fma(-g, g, q), h, g);
+    return fma(fma(-g, g, q), h, g);
+}
+
 // Whether q = quot_f64(a, b, recip_f64(b)), b > 0, lies where the argument above
 // holds on its own: b in [2^-960, 2^961), and a = 0 or |a| and |q| in
 // [2^-959, 2^961).  (The kernels use the cheaper F64Range, which is narrower.)
@@ -110,5 +132,53 @@ struct F64Range {
     }
     __device__ __forceinline__ bool ok() const { return all >= 0xf0000000u && low >= (223u << 21); }
 };
+
+// Arithmetic policies: the IEEE division and square root, or the branch-free
+// ones with their range tests.  Both give the same values wherever ok() holds
+// in the end.
+struct ArithIeee {
+    static constexpr bool checked = false;
+    struct Recip { double b; };
+    __device__ __forceinline__ Recip recip(double b) const { return { b }; }
+    __device__ __forceinline__ double quot(double a, const Recip& r) const { return a / r.b; }
+    __device__ __forceinline__ double root(double x) const { return sqrt(x); }
+    // sqrt(a / b); makes b's Recip
+    __device__ __forceinline__ double root_quot(double a, double b, Recip& r) const {
+        r.b = b;
+        return sqrt(a / b);
+    }
+    __device__ __forceinline__ double half(double w, double h, double s) const { return w + h * s; }
+    __device__ __forceinline__ void pos(double) {}
+    __device__ __forceinline__ void num(double) {}
+    __device__ __forceinline__ bool ok() const { return true; }
+};
+struct ArithFast {
+    static constexpr bool checked = true;
+    struct Recip { double b, y; };
+    F64Range r;
+    __device__ __forceinline__ Recip recip(double b) const { return { b, recip_f64(b) }; }
+    __device__ __forceinline__ double quot(double a, const Recip& q) const { return quot_f64(a, q.b, q.y); }
+    __device__ __forceinline__ double root(double x) const { return sqrt_f64(x); }
+    // (one multiplication more than root(quot()), for a shorter chain)
+    __device__ __forceinline__ double root_quot(double a, double b, Recip& r) const {
+        r.b = b;
+        return sqrt_quot_f64(a, b, r.y);
+    }
+    // h = +-1/2: h s is exact (slopes in range are multiples of 2^-1000), so the
+    // fused form rounds the same sum
+    __device__ __forceinline__ double half(double w, double h, double s) const { return fma(h, s, w); }
+    __device__ __forceinline__ void pos(double x) { r.pos(x); }
+    __device__ __forceinline__ void num(double a) { r.num(a); }
+    __device__ __forceinline__ bool ok() const { return r.ok(); }
+};
+
+// RN(a / b) for one quotient by a divisor that changes.
+__device__ __forceinline__ double div_rn(double a, double b) {
+    F64Range r;
+    r.pos(b);
+    r.pos(a);
+    const double q = quot_f64(a, b, recip_f64(b));
+    return r.ok() ? q : a / b;
+}
 
 }  // namespace nestb
