@@ -466,11 +466,13 @@ cudaError_t launch_2d_adjoint_stage_f32x2(const float* U, const float* Lout, con
     }
     const int strips = (g.ny + ASTRIP - 1) / ASTRIP;
     const int cx = (strips + AWARPS - 1) / AWARPS;
-    // enough row segments for one wave of resident warps, at least 16 rows each
+    // enough row segments for one wave of resident warps, at least 2 rows each
+    // (a march costs its rows and about four more; us of backward per step, at
+    // least 16 -> 2 rows a segment: 64^2 43.9 -> 22.5, 512^2 52.3 -> 40.1)
     const long long slots = (long long)sms * per_sm * AWARPS;
     int segs = (int)std::max<long long>(1, slots / ((long long)cx * AWARPS));
     int seg_rows = (g.nx + segs - 1) / segs;
-    if (seg_rows < 16) seg_rows = 16;
+    if (seg_rows < 2) seg_rows = 2;
     segs = (g.nx + seg_rows - 1) / seg_rows;
     AdjX2Args a{ U, Lout, Extra, Lin, g, dtp, (float)alpha, (float)beta, seg_rows };
     k2d_adjoint_x2<<<dim3(cx, segs), 32 * AWARPS, smem, st>>>(a);

@@ -359,9 +359,11 @@ cudaError_t launch_2d_adjoint_stage_f64rm(const double* U, const double* Lout, c
     const int strips = (g.ny + DSTRIP - 1) / DSTRIP;
     const int cx = (strips + DWARPS - 1) / DWARPS;
     const long long slots = (long long)sms * per_sm * DWARPS;
+    // one wave of resident warps, at least 2 rows a segment (us of backward per
+    // step, at least 16 -> 2 rows: 64^2 85.0 -> 31.7, 512^2 115.8 -> 79.3)
     int segs = (int)std::max<long long>(1, slots / ((long long)cx * DWARPS));
     int seg_rows = (g.nx + segs - 1) / segs;
-    if (seg_rows < 16) seg_rows = 16;
+    if (seg_rows < 2) seg_rows = 2;
     segs = (g.nx + seg_rows - 1) / seg_rows;
     AdjD64Args a{ U, Lout, Extra, Lin, g, dtp, alpha, beta, seg_rows };
     k2d_adjoint_rm64<<<dim3(cx, segs), 32 * DWARPS, smem, st>>>(a);

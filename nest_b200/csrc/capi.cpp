@@ -259,6 +259,40 @@ nest_status copy_state(nest_solver* s, void* dst, const void* src, int layout, b
 
 }  // namespace
 
+namespace {
+
+// Output columns of a warp's strip: 60 for the packed FP32 kernel, else 28.
+int strip_width(int precision, int flags) {
+    return precision == NEST_F32 && !(flags & (NEST_FLAG_FP32_SCALAR | NEST_FLAG_LIMITER_MC | NEST_FLAG_LIMITER_NONE))
+               ? 60 : STRIP;
+}
+
+// Default rows per 2D tile for `work` = rows x strips of all domains of a
+// launch.  A warp marches down its tile at about 1.6 us (FP32) / 1.3 us (FP64)
+// a row however few warps run with it, up to about four per scheduler, so a
+// small domain wants tiles as short as it takes to give every scheduler some:
+// one wave of 148 x 16 resident warps in FP32, a little over two of 148 x 12 in
+// FP64, whose kernels reach the FP64 pipe's rate with fewer.  Shorter tiles
+// than that only repeat their prologue (about two rows).  Larger domains run
+// many waves anyway and amortise the prologue with tall tiles.
+// Measured, us per step with 16 (FP32) / 24 (FP64) rows -> the rule's, in
+// parentheses the best of a sweep over 1..32 rows: FP32 64^2 59.8 -> 9.7 (9.7),
+// 256 x 192 59.2 -> 10.9, 512^2 59.1 -> 18.0 (18.0), 517 x 1003 61.3 -> 29.5 (28.7),
+// 1024^2 64.9 -> 45.9 (45.9), 1500^2 82.2 -> 75.5 (74.9), 2048^2 136.0 -> 125.1
+// (124.7), 4096^2 369.1 at 16, 368.9 at 12, 393.0 at 8; FP64 64^2 89.0 -> 18.5,
+// 512^2 90.7 -> 48.8 (48.8), 517 x 1003 103.2 -> 67.4 (65.1), 1024^2 122.5 -> 108.2
+// (108.2), 2048^2 349.6 at 24, 346.3 at 20, 381.3 at 32.  FP32 batches: 12 problems
+// of 64..256 a side 65 -> 32 (32), 48 of them 81 -> 60 (59), 64 of 48..320 108 -> 95
+// (95), 128 of 64..512 318 (32 rows; 12 rows 328).
+int default_rows(int precision, long long work, int tall64, int tall32) {
+    if (precision == NEST_F64) return (int)std::min<long long>(tall64, (work + 3999) / 4000);
+    const long long one_wave = (work + 2367) / 2368;
+    if (one_wave <= 12) return (int)one_wave;
+    return work < 100000 ? 8 : tall32;
+}
+
+}  // namespace
+
 // ===========================================================================
 // Solver API
 // ===========================================================================
@@ -296,14 +330,9 @@ nest_status nest_solver_create(const nest_solver_desc* d, nest_solver** out) {
     s->d = *d;
     s->h = d->halo;
     s->esize = d->precision == NEST_F64 ? 8 : 4;
-    // default 2D launch shape: the autotuner's choice at 4096^2, one warp per
-    // block, 16-row tiles in FP32 and 24-row tiles in FP64 (64 steps of the
-    // 4096^2 Riemann problem 1.261 ms per step against 1.286 with 16 rows and
-    // 1.265 with 32).  At 2048^2
-    // the earlier default of 64-row tiles and 4 warps per block left half the
-    // warp slots empty: a 4000-step FP32 KH forward took 891 ms against 540 ms.
     if (d->dim == 2) {
-        s->tx = d->precision == NEST_F64 ? 24 : 16;
+        const int sw = strip_width(d->precision, d->flags);
+        s->tx = default_rows(d->precision, (long long)((d->ny + sw - 1) / sw) * d->nx, 24, 16);
         s->warps = 1;
     }
     if (d->dim == 1) {
@@ -338,8 +367,10 @@ nest_status nest_solver_create(const nest_solver_desc* d, nest_solver** out) {
     if ((e = cudaMemsetAsync(s->ctrl, 0, sizeof(StepCtrl), s->st)) != cudaSuccess) return cleanup(cuda_fail(e, "memset"));
     if (d->dim == 2 && (d->flags & NEST_FLAG_TOTALS)) {
         long long nstrips = (d->ny + STRIP - 1) / STRIP;
-        // sized for the smallest tile height the tiling hook accepts (8 rows)
-        s->nrec = nstrips * ((d->nx + 7) / 8);
+        // sized for the default tile height and the smallest one the tiling
+        // hook accepts (8 rows)
+        const int rows = std::min(8, s->tx);
+        s->nrec = nstrips * ((d->nx + rows - 1) / rows);
         if ((e = cudaMalloc(&s->partials, sizeof(double) * 4 * s->nrec)) != cudaSuccess)
             return cleanup(cuda_fail(e, "cudaMalloc(partials)"));
         if ((e = cudaMemsetAsync(s->partials, 0, sizeof(double) * 4 * s->nrec, s->st)) != cudaSuccess)
@@ -787,7 +818,7 @@ struct nest_batch {
     bool prepared = false;
     int tx = 32, warps = 2, blocks = 0;
     std::map<GraphKey, cudaGraphExec_t> graphs;
-    int strip_w() const { return d.precision == NEST_F64 ? STRIP : 60; }
+    int strip_w() const { return strip_width(d.precision, 0); }
 };
 
 namespace {
@@ -928,6 +959,9 @@ nest_status nest_batch_create(const nest_batch_desc* d, nest_batch** out) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int per_sm = d->precision == NEST_F64 ? batch_max_blocks_f64(b->warps) : batch_max_blocks_f32x2(b->warps);
     b->blocks = sms * (per_sm > 0 ? per_sm : 1);
+    long long work = 0;
+    for (const BatchProblem& q : b->probs) work += (long long)((q.g.ny + b->strip_w() - 1) / b->strip_w()) * q.g.nx;
+    b->tx = default_rows(d->precision, work, 32, 32);
     nest_status r = batch_build_items(b);
     if (r != NEST_OK) return cleanup(r);
     *out = b;
