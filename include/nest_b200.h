@@ -193,8 +193,8 @@ nest_status nest_slab_step(nest_solver* s, nest_slab_comm* c, int lo, int hi, in
                            double t_final);
 
 /* ------------------------------------------------------------------------ */
-/* Batched independent 2D problems (uneven sizes).  One persistent launch   */
-/* per stage walks a device work list of (problem, column strip, row tile); */
+/* Batched independent 2D problems (uneven sizes).  One launch per stage     */
+/* covers a device work list of (problem, column strip, row tile);          */
 /* each problem keeps its own dt, time and FP64 totals; runs of steps are   */
 /* captured into CUDA graphs.  No counterpart in nest (its patches are      */
 /* advanced by serial host loops, examples/sod2d/sod2d.cpp:318-366).        */
@@ -228,12 +228,13 @@ nest_status nest_batch_step_profiled(nest_batch* b, int nsteps, double cfl, floa
 nest_status nest_batch_times(nest_batch* b, double* times, int* steps);
 /* Per-problem FP64 totals [count][4] after the last step (needs NEST_FLAG_TOTALS). */
 nest_status nest_batch_totals(nest_batch* b, double* out);
-/* Launch shape: rows per work item, warps per block, blocks per SM (0 = occupancy limit). */
+/* Launch shape: rows per work item, warps per block, blocks per SM of a persistent
+ * grid that walks the list (0: a warp per item). */
 nest_status nest_batch_set_tiling(nest_batch* b, int rows_per_tile, int warps_per_block, int blocks_per_sm);
 /* Zero every problem's time, step count and error word (states are kept;
  * ghost rings and wave speeds are rebuilt before the next step). */
 nest_status nest_batch_reset(nest_batch* b);
-/* Total interior cells, work items and persistent blocks. */
+/* Total interior cells, work items and blocks of a stage launch. */
 nest_status nest_batch_info(nest_batch* b, long long* cells, int* items, int* blocks);
 
 /* ------------------------------------------------------------------------ */

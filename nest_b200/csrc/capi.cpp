@@ -283,7 +283,8 @@ int strip_width(int precision, int flags) {
 // 512^2 90.7 -> 48.8 (48.8), 517 x 1003 103.2 -> 67.4 (65.1), 1024^2 122.5 -> 108.2
 // (108.2), 2048^2 349.6 at 24, 346.3 at 20, 381.3 at 32.  FP32 batches: 12 problems
 // of 64..256 a side 65 -> 32 (32), 48 of them 81 -> 60 (59), 64 of 48..320 108 -> 95
-// (95), 128 of 64..512 318 (32 rows; 12 rows 328).
+// (95), 128 of 64..512 318 (32 rows; 12 rows 328); FP64 batches: 64 of 48..320 312 at
+// 16 rows, 307 at 12, 346 at 4, 128 of 64..512 1057 at 16, 1061 at 32.
 int default_rows(int precision, long long work, int tall64, int tall32) {
     if (precision == NEST_F64) return (int)std::min<long long>(tall64, (work + 3999) / 4000);
     const long long one_wave = (work + 2367) / 2368;
@@ -817,6 +818,7 @@ struct nest_batch {
     int parity = 0;
     bool prepared = false;
     int tx = 32, warps = 2, blocks = 0;
+    int persistent_blocks = 0;            // 0: a warp per item
     std::map<GraphKey, cudaGraphExec_t> graphs;
     int strip_w() const { return strip_width(d.precision, 0); }
 };
@@ -850,6 +852,13 @@ nest_status batch_build_items(nest_batch* b) {
     }
     for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
     b->graphs.clear();
+    // A warp per item by default: the hardware hands out the blocks as others
+    // end, where a persistent grid's fixed stride leaves warps idle when the
+    // items do not divide evenly.  Us per step, persistent -> this: FP64, 128
+    // problems of 64..512 a side 1123 -> 1057, 64 of 48..320 333 -> 307; FP32, 256 of
+    // 64..1024 2043 -> 1972, 48 of 64..256 60.3 -> 60.0.
+    const int all = ((int)b->items.size() + b->warps - 1) / b->warps;
+    b->blocks = b->persistent_blocks > 0 ? b->persistent_blocks : all;
     return NEST_OK;
 }
 
@@ -954,14 +963,9 @@ nest_status nest_batch_create(const nest_batch_desc* d, nest_batch** out) {
         return cleanup(cuda_fail(e, "cudaMallocHost"));
     if ((e = cudaMalloc(&b->totals_dev, sizeof(double) * 4 * b->count)) != cudaSuccess)
         return cleanup(cuda_fail(e, "cudaMalloc(totals)"));
-    int sms = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int per_sm = d->precision == NEST_F64 ? batch_max_blocks_f64(b->warps) : batch_max_blocks_f32x2(b->warps);
-    b->blocks = sms * (per_sm > 0 ? per_sm : 1);
     long long work = 0;
     for (const BatchProblem& q : b->probs) work += (long long)((q.g.ny + b->strip_w() - 1) / b->strip_w()) * q.g.nx;
-    b->tx = default_rows(d->precision, work, 32, 32);
+    b->tx = default_rows(d->precision, work, 16, 32);
     nest_status r = batch_build_items(b);
     if (r != NEST_OK) return cleanup(r);
     *out = b;
@@ -1034,7 +1038,7 @@ nest_status nest_batch_set_tiling(nest_batch* b, int rows_per_tile, int warps_pe
     int per_sm = b->d.precision == NEST_F64 ? batch_max_blocks_f64(b->warps) : batch_max_blocks_f32x2(b->warps);
     if (per_sm < 1) per_sm = 1;
     if (blocks_per_sm > 0 && blocks_per_sm < per_sm) per_sm = blocks_per_sm;
-    b->blocks = sms * per_sm;
+    b->persistent_blocks = blocks_per_sm > 0 ? sms * per_sm : 0;
     return batch_build_items(b);
 }
 

@@ -69,38 +69,6 @@ cudaError_t launch_2d_step_f64(double* U, double* U1, const Geo2D& g, const Loop
     return cudaGetLastError();
 }
 
-template <int STAGE>
-__device__ __noinline__ void f64_body_call(const StageArgs<double>& a, int strip, int tile_row) {
-    stage2d_body<double, STAGE, false>(a, strip, tile_row);
-}
-
-// Persistent batched FP64 stage (bit-exact per problem).
-template <int STAGE>
-__global__ void __launch_bounds__(256) kbatch_f64(BatchArgs<double> b) {
-    const int nw = gridDim.x * blockDim.y;
-    for (int it = blockIdx.x * blockDim.y + threadIdx.y; it < b.nitems; it += nw) {
-        const int4 w = b.items[it];
-        const BatchProblem& P = b.probs[w.x];
-        StageArgs<double> a{STAGE == 1 ? b.U + P.off : b.U1 + P.off, STAGE == 2 ? b.U + P.off : nullptr,
-                            STAGE == 1 ? b.U1 + P.off : b.U + P.off, P.g, b.lp, b.ctrls + w.x,
-                            (STAGE == 2 && b.partials) ? b.partials + 4ll * P.item0 : nullptr, b.p, b.tx};
-        f64_body_call<STAGE>(a, w.y, w.z);
-    }
-}
-
-cudaError_t launch_batch_f64(const BatchArgs<double>& b, int which, int blocks, int warps, cudaStream_t st) {
-    dim3 blk(32, warps);
-    if (which & 1) kbatch_f64<1><<<blocks, blk, 0, st>>>(b);
-    if (which & 2) kbatch_f64<2><<<blocks, blk, 0, st>>>(b);
-    return cudaGetLastError();
-}
-
-int batch_max_blocks_f64(int warps) {
-    int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kbatch_f64<2>, 32 * warps, 0);
-    return nb;
-}
-
 // Per-problem deterministic sums of the per-item totals: block p sums items
 // [first[p], first[p+1]) in a fixed order.
 __global__ void __launch_bounds__(256) k_sum_batch(const double* part, const int* first, double* out) {

@@ -136,8 +136,8 @@ __device__ __forceinline__ double speeds_d(A& m, double U0, double U1, double U2
 // LIM: the slope limiter fixed at compile time (LIM_MINMOD, nest's default),
 // or -1 to read it from the loop parameters; a fixed limiter leaves no
 // limiter branch in the row loop.
-template <int STAGE, bool TOT, int LIM>
-__device__ __forceinline__ void f64r_body(const StageArgs<double>& a, int strip, int tile_row) {
+template <int STAGE, bool TOT, int LIM, class Args>
+__device__ __forceinline__ void f64r_body(const Args& a, int strip, int tile_row) {
     const Geo2D& g = a.g;
     const int lane = threadIdx.x & 31;
     const double gamma = g.gamma;
@@ -392,6 +392,39 @@ __global__ void __maxnreg__(NEST_F64R_REGS) k2d_f64r(StageArgs<double> a) {
     f64r_body<STAGE, TOT, LIM>(a, blockIdx.x * blockDim.y + threadIdx.y, blockIdx.y);
 }
 
+// Arguments of one batched work item: the arrays of its problem, whose geometry
+// stays in global memory (the body copies the fields its row loop needs).
+struct F64View {
+    const double* Uin;
+    const double* Un;
+    double* Uout;
+    const Geo2D& g;
+    const LoopParams& lp;
+    StepCtrl* ctrl;
+    double* partials;
+    int p;
+    int tx;
+};
+
+// Persistent batched stage (bit for bit the single-domain solver's result per
+// problem): every warp walks the work list (problem, strip, tile row) with the
+// grid's warp count as stride (one item each by default).
+// Us per step with TOTALS, against the register-window march with IEEE
+// divisions in 32-row items: 4 problems of 64..128 a side 24 (216), 48 of 64..256
+// 190 (258), 64 of 48..320 312 (508).
+template <int STAGE, bool TOT>
+__global__ void __maxnreg__(NEST_F64R_REGS) kbatch_f64(BatchArgs<double> b) {
+    const int nw = gridDim.x * blockDim.y;
+    for (int it = blockIdx.x * blockDim.y + threadIdx.y; it < b.nitems; it += nw) {
+        const int4 w = b.items[it];
+        const BatchProblem& P = b.probs[w.x];
+        const F64View v{STAGE == 1 ? b.U + P.off : b.U1 + P.off, STAGE == 2 ? b.U + P.off : nullptr,
+                        STAGE == 1 ? b.U1 + P.off : b.U + P.off, P.g, b.lp, b.ctrls + w.x,
+                        TOT ? b.partials + 4ll * P.item0 : nullptr, b.p, b.tx};
+        f64r_body<STAGE, TOT, LIM_MINMOD>(v, w.y, w.z);
+    }
+}
+
 template <int LIM>
 void launch_f64r_lim(const StageArgs<double>& a1, const StageArgs<double>& a2, dim3 gr, dim3 b, size_t sm1,
                      size_t sm2, int which, bool tot, cudaStream_t st) {
@@ -417,6 +450,25 @@ cudaError_t launch_2d_step_f64r(double* U, double* U1, const Geo2D& g, const Loo
     if (lp.lim == LIM_MINMOD) launch_f64r_lim<LIM_MINMOD>(a1, a2, gr, b, sm1, sm2, which, partials != nullptr, st);
     else launch_f64r_lim<-1>(a1, a2, gr, b, sm1, sm2, which, partials != nullptr, st);
     return cudaGetLastError();
+}
+
+cudaError_t launch_batch_f64(const BatchArgs<double>& b, int which, int blocks, int warps, cudaStream_t st) {
+    const dim3 blk(32, warps);
+    const size_t sm1 = f64r_ring_bytes(1, warps), sm2 = f64r_ring_bytes(2, warps);
+    if (which & 1) kbatch_f64<1, false><<<blocks, blk, sm1, st>>>(b);
+    if (which & 2) {
+        if (b.partials) kbatch_f64<2, true><<<blocks, blk, sm2, st>>>(b);
+        else kbatch_f64<2, false><<<blocks, blk, sm2, st>>>(b);
+    }
+    return cudaGetLastError();
+}
+
+// Resident blocks per SM of the batched stages (6 KB of rings a warp: no
+// opt-in shared memory up to the 8 warps a block may have).
+int batch_max_blocks_f64(int warps) {
+    int nb = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kbatch_f64<2, true>, 32 * warps, f64r_ring_bytes(2, warps));
+    return nb;
 }
 
 namespace {
