@@ -14,8 +14,12 @@
 // forward computes them: this unit is compiled with -fmad=false, the
 // primitives divide (u = m / rho), ke2 keeps its operation order and the sound
 // speed is sqrt(gamma p / rho).  Terms that only enter derivatives use
-// explicit fma().
+// explicit fma().  Division and square root are the branch-free ones of
+// f64div.cuh; the x or y part of a row in which a range test fails (rho, p and
+// the momenta of the new row's cells, rho and p of the face states, the speed
+// difference) is computed again with the IEEE ones before it is added anywhere.
 #include "euler2d_kernels.cuh"
+#include "f64div.cuh"
 #include "kernels.h"
 
 #include <algorithm>
@@ -24,10 +28,12 @@
 namespace nestb {
 namespace {
 
-// Launch shape and register budget, measured on the 2048^2 FP64 KH adjoint
-// (300 steps, backward ms): 2 warps per CTA at 168 registers (12 warps per
-// SM, no spills) 570; unbounded (176 registers, 10 warps per SM) 611 with 1,
-// 2 or 4 warps per CTA; 152 / 128 registers (spills) 591 / 592.
+// Launch shape and register budget, measured on the FP64 KH adjoint (24 steps, us
+// of backward per step, its forward recomputation included, 1024^2 / 2048^2): 2
+// warps per CTA at 168 registers (12 warps per SM, 28 bytes spilled) 211 / 717; 176
+// (10 warps) 213 / 752; 184 and unbounded (196) 216 / 763.  With the IEEE division
+// and square root 221 (1024^2), and at 64^2, where the chain's latency counts,
+// 31.7 against 27.5.
 #ifndef NEST_ADJ64_WARPS
 #define NEST_ADJ64_WARPS 2
 #define NEST_ADJ64_REGS 168
@@ -50,14 +56,17 @@ __device__ __forceinline__ void cpd_wait1() { asm volatile("cp.async.wait_group 
 // Primitives of one cell exactly as the forward FP64 stage (cons2prim, no
 // contraction); `act` = 1 where the pressure clamp p = max(p_raw, 0) is not
 // active (p_raw >= 0).
-__device__ __forceinline__ D4 prim64(const D4& U, double gm1, int& act) {
+template <class A>
+__device__ __forceinline__ D4 prim64(A& m, const D4& U, double gm1, int& act) {
     D4 w;
+    const auto ir = m.recip(U.a);
     w.a = U.a;
-    w.b = U.b / U.a;
-    w.c = U.c / U.a;
+    w.b = m.quot(U.b, ir);
+    w.c = m.quot(U.c, ir);
     const double praw = gm1 * (U.d - ke2(w.a, w.b, w.c));
     act = praw < 0.0 ? 0 : 1;
     w.d = smax(praw, 0.0);
+    m.pos(w.a); m.pos(w.d); m.num(U.b); m.num(U.c);
     return w;
 }
 
@@ -73,24 +82,23 @@ __device__ __forceinline__ double mmb(double d1, double d2, int& br) {
 // Reverse of hlle4 for one face in the relative-flux form of the FP32 row
 // march (adjoint2d_f32x2.cu, hlle2_adj): states (r, n, t, p) per side, flux
 // adjoint (f0..f3) in the order (mass, normal, transverse, energy); the
-// face-state adjoints are added to Lb and Rb.  The regime and the active
+// face-state adjoints go to Lb and Rb.  The regime and the active
 // arguments come from the forward's own sound speeds and Davis speeds.
-__device__ __forceinline__ void hlle_adj64(double gamma, double igm1, const D4& L, const D4& R, double f0,
+template <class A>
+__device__ __forceinline__ void hlle_adj64(A& m, double gamma, double igm1, const D4& L, const D4& R, double f0,
                                            double f1, double f2, double f3, D4& Lb, D4& Rb) {
     const double rL = L.a, nL = L.b, tL = L.c, pL = L.d;
     const double rR = R.a, nR = R.b, tR = R.c, pR = R.d;
-    const double cL = sqrt(gamma * pL / rL), cR = sqrt(gamma * pR / rR);
+    const double cL = m.root(m.quot(gamma * pL, m.recip(rL))), cR = m.root(m.quot(gamma * pR, m.recip(rR)));
+    m.pos(rL); m.pos(pL); m.pos(rR); m.pos(pR);
     // nsl = -min(S_L, 0), sr = max(S_R, 0) (cL - nL is exactly -(nL - cL))
     const double aL = cL - nL, aR = cR - nR, bL = nL + cL, bR = nR + cR;
     const double nsl = fmax(fmax(aL, aR), 0.0), sr = fmax(fmax(bL, bR), 0.0);
     const double den = sr + nsl;
-    double wL = 1.0, wR = 0.0, i2 = 0.0;  // S_L = S_R = 0: the forward takes F_L
-    if (den > 0.0) {
-        const double inv = 1.0 / den;
-        wL = sr * inv;
-        wR = nsl * inv;
-        i2 = inv * inv;
-    }
+    m.pos(den);
+    const double inv = m.inverse(den);
+    // S_L = S_R = 0: the forward takes F_L
+    const double wL = den > 0.0 ? sr * inv : 1.0, wR = den > 0.0 ? nsl * inv : 0.0, i2 = den > 0.0 ? inv * inv : 0.0;
     const double kL = 0.5 * fma(tL, tL, nL * nL), kR = 0.5 * fma(tR, tR, nR * nR);
     const double EL = fma(pL, igm1, rL * kL), ER = fma(pR, igm1, rR * kR);
     const double gL = wL * (nL + nsl), gR = wR * (nR - sr);
@@ -113,15 +121,11 @@ __device__ __forceinline__ void hlle_adj64(double gamma, double igm1, const D4& 
         double nb = fma(w, fma(r, X, f3 * (E + p)), fma(gs * r, Y, nb0));
         double tb = gs * r * fma(f3, t, f2);
         double pb = fma(w, Y, gs * f3 * igm1);
-        if (c > 0.0) {  // dc/dp = gamma / (2 r c), dc/dr = -c^2 / (2 r c)
-            const double h = 0.5 / (r * c);
-            pb = fma(cb * gamma, h, pb);
-            rb = fma(-cb * (c * c), h, rb);
-        }
-        out.a += rb;
-        out.b += nb;
-        out.c += tb;
-        out.d += pb;
+        // dc/dp = gamma / (2 r c), dc/dr = -c^2 / (2 r c); none at c = 0
+        const double h = c > 0.0 ? 0.5 * m.inverse(r * c) : 0.0;
+        pb = fma(cb * gamma, h, pb);
+        rb = fma(-cb * (c * c), h, rb);
+        out = { rb, nb, tb, pb };
     };
     side(wL, gL, rL, nL, tL, pL, EL, kL, XL, YL, cL, slL + srL, srL - slL, Lb);
     side(wR, gR, rR, nR, tR, pR, ER, kR, XR, YR, cR, slR + srR, srR - slR, Rb);
@@ -198,9 +202,18 @@ __global__ void NEST_ADJ64_ATTR k2d_adjoint_rm64(AdjD64Args A) {
     D4 Wm, W0, W1, P0;
     {
         int k0, k1, k2;
-        Wm = prim64(ld(A.U, r0 - 3), gm1, k0);
-        W0 = prim64(ld(A.U, r0 - 2), gm1, k1);
-        W1 = prim64(ld(A.U, r0 - 1), gm1, k2);
+        const D4 u0 = ld(A.U, r0 - 3), u1 = ld(A.U, r0 - 2), u2 = ld(A.U, r0 - 1);
+        auto prims = [&](auto& m) {
+            Wm = prim64(m, u0, gm1, k0);
+            W0 = prim64(m, u1, gm1, k1);
+            W1 = prim64(m, u2, gm1, k2);
+        };
+        ArithFast m;
+        prims(m);
+        if (__any_sync(0xffffffffu, !m.ok())) {
+            ArithIeee mi;
+            prims(mi);
+        }
         actb = ((unsigned)k0 << 2) | ((unsigned)k1 << 1) | (unsigned)k2;
         int b0, b1, b2, b3;
         D4 s{ mmb(W0.a - Wm.a, W1.a - W0.a, b0), mmb(W0.b - Wm.b, W1.b - W0.b, b1),
@@ -225,24 +238,41 @@ __global__ void NEST_ADJ64_ATTR k2d_adjoint_rm64(AdjD64Args A) {
         cpd_commit();
         cpd_wait1();
 
-        // row a+2, x-slope of row a+1
-        int k2;
-        const D4 W2 = prim64(rd(ringU + ((a + 2) & (DRU - 1)) * 128), gm1, k2);
-        actb = (actb << 1) | (unsigned)k2;
-        int c0, c1, c2, c3;
-        const D4 s1{ mmb(W1.a - W0.a, W2.a - W1.a, c0), mmb(W1.b - W0.b, W2.b - W1.b, c1),
-                     mmb(W1.c - W0.c, W2.c - W1.c, c2), mmb(W1.d - W0.d, W2.d - W1.d, c3) };
-        const int brn = c0 | (c1 << 2) | (c2 << 4) | (c3 << 6);
-
-        // x-face a+1/2: left P0, right W1 - s1/2 (normal u, transverse v)
         const D4 L0 = rd(ringL + (a & (DRL - 1)) * 128);
         const D4 L1 = rd(ringL + ((a + 1) & (DRL - 1)) * 128);
+        const D4 U2 = rd(ringU + ((a + 2) & (DRU - 1)) * 128);
+
+        // The x part: row a+2, the x-slope of row a+1 and the reverse of x-face
+        // a+1/2 (left P0, right W1 - s1/2; normal u, transverse v).
+        struct XPart {
+            D4 W2, s1, wl, wr;
+            int act, br;
+        };
+        auto xpart = [&](auto& m) {
+            XPart o;
+            o.W2 = prim64(m, U2, gm1, o.act);
+            int c0, c1, c2, c3;
+            o.s1 = { mmb(W1.a - W0.a, o.W2.a - W1.a, c0), mmb(W1.b - W0.b, o.W2.b - W1.b, c1),
+                     mmb(W1.c - W0.c, o.W2.c - W1.c, c2), mmb(W1.d - W0.d, o.W2.d - W1.d, c3) };
+            o.br = c0 | (c1 << 2) | (c2 << 4) | (c3 << 6);
+            const D4 M1{ W1.a - 0.5 * o.s1.a, W1.b - 0.5 * o.s1.b, W1.c - 0.5 * o.s1.c, W1.d - 0.5 * o.s1.d };
+            hlle_adj64(m, gamma, igm1, P0, M1, lx * (L1.a - L0.a), lx * (L1.b - L0.b), lx * (L1.c - L0.c),
+                       lx * (L1.d - L0.d), o.wl, o.wr);
+            return o;
+        };
+        ArithFast mx;
+        XPart x = xpart(mx);
+        if (__any_sync(0xffffffffu, !mx.ok())) {
+            ArithIeee mi;
+            x = xpart(mi);
+        }
+        const D4 W2 = x.W2, s1 = x.s1;
+        const int brn = x.br;
+        actb = (actb << 1) | (unsigned)x.act;
+
         D4 B1{ 0, 0, 0, 0 };
         {
-            const D4 M1{ W1.a - 0.5 * s1.a, W1.b - 0.5 * s1.b, W1.c - 0.5 * s1.c, W1.d - 0.5 * s1.d };
-            D4 wl{ 0, 0, 0, 0 }, wr{ 0, 0, 0, 0 };
-            hlle_adj64(gamma, igm1, P0, M1, lx * (L1.a - L0.a), lx * (L1.b - L0.b), lx * (L1.c - L0.c),
-                       lx * (L1.d - L0.d), wl, wr);
+            const D4 wl = x.wl, wr = x.wr;
             // slope adjoint of row a is complete: wl/2 + Sp, scattered by its code
             auto scat = [&](double wl_, double wr_, double sp, int br, double& bm, double& b0, double& b1) {
                 const double s = fma(0.5, wl_, sp);
@@ -258,28 +288,43 @@ __global__ void NEST_ADJ64_ATTR k2d_adjoint_rm64(AdjD64Args A) {
             Sp = { -0.5 * wr.a, -0.5 * wr.b, -0.5 * wr.c, -0.5 * wr.d };
         }
 
-        // y-direction part of row a
+        // y-direction part of row a: face (c | c+1), normal v, transverse u; flux
+        // order (mass, mv, mu, E)
         if (a >= r0 && a < r0 + rows) {
-            D4 P, R;
-            int y0, y1, y2, y3;
-            auto yvar = [&](double w, int& br, double& p, double& rr) {
-                const double lw = __shfl_up_sync(0xffffffffu, w, 1);
-                const double rw = __shfl_down_sync(0xffffffffu, w, 1);
-                const double s = mmb(w - lw, rw - w, br);
-                p = w + 0.5 * s;
-                rr = __shfl_down_sync(0xffffffffu, w - 0.5 * s, 1);
+            struct YPart {
+                D4 wl, wr;
+                int br;
             };
-            yvar(W0.a, y0, P.a, R.a);
-            yvar(W0.b, y1, P.b, R.b);
-            yvar(W0.c, y2, P.c, R.c);
-            yvar(W0.d, y3, P.d, R.d);
-            const D4 Lr{ __shfl_down_sync(0xffffffffu, L0.a, 1), __shfl_down_sync(0xffffffffu, L0.b, 1),
-                         __shfl_down_sync(0xffffffffu, L0.c, 1), __shfl_down_sync(0xffffffffu, L0.d, 1) };
-            // face (c | c+1): normal v, transverse u; flux order (mass, mv, mu, E)
-            const D4 PL{ P.a, P.c, P.b, P.d }, RR{ R.a, R.c, R.b, R.d };
-            D4 wl{ 0, 0, 0, 0 }, wr{ 0, 0, 0, 0 };
-            hlle_adj64(gamma, igm1, PL, RR, ly * (Lr.a - L0.a), ly * (Lr.c - L0.c), ly * (Lr.b - L0.b),
-                       ly * (Lr.d - L0.d), wl, wr);
+            auto ypart = [&](auto& m) {
+                YPart o;
+                D4 P, R;
+                int y0, y1, y2, y3;
+                auto yvar = [&](double w, int& br, double& p, double& rr) {
+                    const double lw = __shfl_up_sync(0xffffffffu, w, 1);
+                    const double rw = __shfl_down_sync(0xffffffffu, w, 1);
+                    const double s = mmb(w - lw, rw - w, br);
+                    p = w + 0.5 * s;
+                    rr = __shfl_down_sync(0xffffffffu, w - 0.5 * s, 1);
+                };
+                yvar(W0.a, y0, P.a, R.a);
+                yvar(W0.b, y1, P.b, R.b);
+                yvar(W0.c, y2, P.c, R.c);
+                yvar(W0.d, y3, P.d, R.d);
+                o.br = y0 | (y1 << 2) | (y2 << 4) | (y3 << 6);
+                const D4 Lr{ __shfl_down_sync(0xffffffffu, L0.a, 1), __shfl_down_sync(0xffffffffu, L0.b, 1),
+                             __shfl_down_sync(0xffffffffu, L0.c, 1), __shfl_down_sync(0xffffffffu, L0.d, 1) };
+                const D4 PL{ P.a, P.c, P.b, P.d }, RR{ R.a, R.c, R.b, R.d };
+                hlle_adj64(m, gamma, igm1, PL, RR, ly * (Lr.a - L0.a), ly * (Lr.c - L0.c), ly * (Lr.b - L0.b),
+                           ly * (Lr.d - L0.d), o.wl, o.wr);
+                return o;
+            };
+            ArithFast my;
+            YPart y = ypart(my);
+            if (__any_sync(0xffffffffu, !my.ok())) {
+                ArithIeee mi;
+                y = ypart(mi);
+            }
+            const D4 wl = y.wl, wr = y.wr;
             auto ycell = [&](double l, double r, int br, double& b) {
                 const double q = __shfl_up_sync(0xffffffffu, r, 1);  // right-state adjoint of the face on the left
                 const double sb = 0.5 * (l - q);
@@ -288,16 +333,18 @@ __global__ void NEST_ADJ64_ATTR k2d_adjoint_rm64(AdjD64Args A) {
                 const double t2p = __shfl_up_sync(0xffffffffu, t2, 1);
                 b += (l + q) + ((t1 - t2) + (t2p - t1n));
             };
-            ycell(wl.a, wr.a, y0, B0.a);
-            ycell(wl.c, wr.c, y1, B0.b);
-            ycell(wl.b, wr.b, y2, B0.c);
-            ycell(wl.d, wr.d, y3, B0.d);
+            ycell(wl.a, wr.a, y.br & 3, B0.a);
+            ycell(wl.c, wr.c, (y.br >> 2) & 3, B0.b);
+            ycell(wl.b, wr.b, (y.br >> 4) & 3, B0.c);
+            ycell(wl.d, wr.d, (y.br >> 6) & 3, B0.d);
         }
 
         // row a-1 is complete
         if (a - 1 >= r0 && out) {
             const D4 Lm = rd(ringL + ((a - 1) & (DRL - 1)) * 128);
-            const double ir = 1.0 / Wm.a, u = Wm.b, v = Wm.c;
+            F64Range rr;
+            rr.pos(Wm.a);
+            const double ir = rr.ok() ? recip_f64(Wm.a) : 1.0 / Wm.a, u = Wm.b, v = Wm.c;
             const double g3 = ((actb >> 3) & 1u) ? gm1 * Bm.d : 0.0;
             const double q2 = 0.5 * fma(v, v, u * u);
             D4 o{ fma(g3, q2, Bm.a - fma(Bm.c, v, Bm.b * u) * ir), fma(-g3, u, Bm.b * ir), fma(-g3, v, Bm.c * ir),
