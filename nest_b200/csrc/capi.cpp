@@ -85,8 +85,9 @@ LoopParams base_params(const nest_solver* s) {
 
 // Ghost fill + wave-speed maxima of the current state into slot `parity`.
 nest_status nestb::rt::prepare(nest_solver* s) {
-    // both slots: the one-launch 1D step adds into maxs[1 - parity][1]
-    CK(cudaMemsetAsync(&s->ctrl->maxs[0][0], 0, sizeof s->ctrl->maxs, s->st));
+    // both slots, and the 1D choice of words that follows them
+    static_assert(offsetof(StepCtrl, sel) == offsetof(StepCtrl, maxs) + sizeof(StepCtrl::maxs), "one memset for both");
+    CK(cudaMemsetAsync(&s->ctrl->maxs[0][0], 0, sizeof s->ctrl->maxs + sizeof s->ctrl->sel, s->st));
     cudaError_t e;
     if (s->d.dim == 1 && s->d.precision == NEST_F32) {
         e = launch_1d_prepare_f32((float*)s->U, s->d.nx, s->h, s->d.gamma, s->d.bc_x, s->ctrl, s->parity, s->st);
@@ -672,7 +673,8 @@ nest_status nest_solver_stage(nest_solver* s, int which, double cfl, double t_fi
 nest_status nest_solver_speed_slot(nest_solver* s, void** dev) {
     nest_status r = check(s);
     if (r != NEST_OK) return r;
-    if (!s->prepared && (r = prepare(s)) != NEST_OK) return r;
+    // in 1D the word alternates from step to step: put it back to the first
+    if ((!s->prepared || s->d.dim == 1) && (r = prepare(s)) != NEST_OK) return r;
     if (dev) *dev = &s->ctrl->maxs[s->parity][0];
     return NEST_OK;
 }

@@ -63,6 +63,9 @@ struct StepCtrl {
     double time[2];                 // simulated time at the start of the step
     double dt[2];                   // dt chosen by stage 1 of the step
     unsigned long long maxs[2][2];  // [p][axis] max wave speed of U at the start of step p (bits of a non-negative double)
+    // 1D: sel[p] = w + 2 t for the step in slot p: its maximum is in maxs[p][w], and
+    // a one-launch step adds the next one to maxs[1-p][t], which is 0 (publish_step_1d)
+    int sel[2];
     int step[2];                    // completed steps at the start of the step
     int active[2];                  // stage 1 sets it: 1 = the step runs, 0 = finished
     unsigned repairs;               // FP32 form: number of repaired cells
@@ -72,11 +75,6 @@ struct StepCtrl {
     int bad_i, bad_j;               // its interior index (1D: bad_j = 0)
     int pad_;
     double bad_rho, bad_p;          // and its density and pressure
-    // one-launch 1D steps: blocks of the running step that have added their
-    // wave speed to maxs[q][1] (the last one moves the maximum to maxs[q][0],
-    // clears maxs[q][1] and resets this count)
-    unsigned blocks_done;
-    unsigned pad2_;
 };
 
 // Time-loop parameters shared by all launches of a solver.
@@ -163,10 +161,7 @@ __device__ __forceinline__ double prescribed_dt(const StepCtrl* c, int p, const 
 }
 
 // Block 0 / thread 0 of stage 1: publish dt and prepare the next slot.
-// clear_next = false in a one-launch 1D step, whose other blocks may already
-// be adding to slot q (its last block writes maxs[q][0]).
-__device__ __forceinline__ void publish_step(StepCtrl* c, int p, const LoopParams& lp, bool done, double dt,
-                                             bool clear_next = true) {
+__device__ __forceinline__ void publish_step(StepCtrl* c, int p, const LoopParams& lp, bool done, double dt) {
     int q = p ^ 1;
     if (done) {
         c->active[p] = 0;
@@ -181,12 +176,57 @@ __device__ __forceinline__ void publish_step(StepCtrl* c, int p, const LoopParam
     c->dt[p] = dt;
     c->time[q] = c->time[p] + dt;
     c->step[q] = c->step[p] + 1;
-    if (clear_next) {
-        c->maxs[q][0] = 0ull;
-        c->maxs[q][1] = 0ull;
-    }
+    c->maxs[q][0] = 0ull;
+    c->maxs[q][1] = 0ull;
     int s = c->step[p];
     if (lp.dts_out && s < lp.dts_cap) lp.dts_out[s] = dt;
+}
+
+// The same for 1D.  The blocks of a one-launch step add the next maximum while
+// others may still be reading this one's slot or starting, so no word that the
+// step reads or adds to may be cleared in it: the maximum alternates between the
+// two words of a slot.  A step that reads maxs[p][w] and adds to maxs[q][t] clears
+// maxs[p][1-w], which the step after it (slot q, reading word t) adds to.
+// After the two stage launches the maximum is in maxs[q][0] (stage 2 adds it).
+__device__ __forceinline__ void publish_step_1d(StepCtrl* c, int p, const LoopParams& lp, bool done, double dt,
+                                                bool one_launch) {
+    const int q = p ^ 1, w = c->sel[p] & 1, t = c->sel[p] >> 1;
+    c->maxs[p][1 - w] = 0ull;
+    if (done) {
+        c->active[p] = 0;
+        c->time[q] = c->time[p];
+        c->step[q] = c->step[p];
+        c->maxs[q][w] = c->maxs[p][w];
+        c->maxs[q][1 - w] = 0ull;
+        c->sel[q] = w + 2 * (1 - w);
+        c->active[q] = 0;
+        return;
+    }
+    c->active[p] = 1;
+    c->dt[p] = dt;
+    c->time[q] = c->time[p] + dt;
+    c->step[q] = c->step[p] + 1;
+    if (one_launch) {
+        c->sel[q] = t + 2 * (1 - w);
+    } else {
+        c->maxs[q][0] = 0ull;
+        c->maxs[q][1] = 0ull;
+        c->sel[q] = 2 * (1 - w);
+    }
+    const int s = c->step[p];
+    if (lp.dts_out && s < lp.dts_cap) lp.dts_out[s] = dt;
+}
+
+__device__ __forceinline__ double speed_1d(const StepCtrl* c, int p) { return bits_speed(c->maxs[p][c->sel[p] & 1]); }
+
+// Max over a warp of a non-negative double's bit pattern: two 32-bit
+// reductions (the high words, then the low words of the lanes that hold the
+// maximum) in place of five shuffle rounds.
+__device__ __forceinline__ double warp_max_speed(double s) {
+    const unsigned hi = (unsigned)__double2hiint(s), lo = (unsigned)__double2loint(s);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    return __hiloint2double((int)mh, (int)ml);
 }
 
 // ---------------------------------------------------------------------------

@@ -11,8 +11,8 @@
 //     both stages, Heun average) with no kernel boundary and no host round-trip
 //     per step, up to 4080 cells.  Where no cluster can be placed, one CTA with
 //     several cells per thread (k1d_resident) takes up to about 2300.
-//   * tiled (euler1d_tiled.cuh): a whole step per launch over 224-cell tiles
-//     (the stage-1 halo recomputed per CTA), or the two stage kernels; stage
+//   * tiled (euler1d_tiled.cuh): a whole step per launch, a warp per 24 cells
+//     (the stage-1 halo recomputed per warp), or the two stage kernels; stage
 //     2 fuses the Heun average, the ghost fill of the new state and the
 //     max-wave-speed reduction; dt is derived on the device from that
 //     maximum, so steps need no host synchronisation (they are captured in
@@ -215,16 +215,6 @@ k1d_resident(double* __restrict__ Ug, int n, int h, double dx, double gamma, int
         ctrl->time[p] = time; ctrl->step[p] = step;
         ctrl->time[p ^ 1] = time; ctrl->step[p ^ 1] = step;
     }
-}
-
-// Max over a warp of a non-negative double's bit pattern: two 32-bit
-// reductions (the high words, then the low words of the lanes that hold the
-// maximum) in place of five shuffle rounds.
-__device__ __forceinline__ double warp_max_speed(double s) {
-    const unsigned hi = (unsigned)__double2hiint(s), lo = (unsigned)__double2loint(s);
-    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-    return __hiloint2double((int)mh, (int)ml);
 }
 
 // Largest chunk of the resident loop: cells per CTA (9 warps of 31 cells).

@@ -9,8 +9,8 @@
 // copies it feeds; stage 2 fuses the Heun average and the block's max
 // |u|+c (one atomic per block).  dt is derived on the device from that
 // maximum by the next stage 1, so a step is two launches and no host
-// synchronisation.  k1d_step runs a whole step in one launch (out of place),
-// recomputing the stage-1 halo per CTA.
+// synchronisation.  k1d_step runs a whole step in one launch (out of place), a
+// warp per 24 cells with nothing in shared memory.
 #pragma once
 
 #include "euler1d_arith.cuh"
@@ -55,14 +55,14 @@ k1d_stage(const T* __restrict__ Uin, const T* Un, T* Uout,
     double dt;
     if (STAGE == 1) {
         bool done = step_is_done(ctrl, p, lp);
-        double ms = bits_speed(ctrl->maxs[p][0]);
+        double ms = speed_1d(ctrl, p);
         double pd = done ? -1.0 : prescribed_dt(ctrl, p, lp);
         if (pd > 0.0) dt = pd;
         else {
             dt = lp.cfl * dx / ms;
             if (lp.t_final > 0.0) dt = smin(dt, lp.t_final - ctrl->time[p]);
         }
-        if (blockIdx.x == 0 && threadIdx.x == 0) publish_step(ctrl, p, lp, done, dt);
+        if (blockIdx.x == 0 && threadIdx.x == 0) publish_step_1d(ctrl, p, lp, done, dt, false);
         if (done) return;
     } else {
         if (!ctrl->active[p]) return;
@@ -134,145 +134,125 @@ __device__ __forceinline__ int source_cell_1d(int c, int n, int bc) {
     return min(max(c, 0), n - 1);
 }
 
+constexpr int STEP_CELLS = 24;  // output cells per warp of k1d_step
+constexpr int STEP_WARPS = 4;   // warps per CTA
+
+// Stage fluxes of a warp whose lane k holds the primitives w of cell k: lane k
+// returns the face between cells k and k+1 (k = 1 .. 29 where all 32 cells are
+// valid), in the expressions of plm_flux.
+template <typename T>
+__device__ __forceinline__ F3<T> warp_flux(const Gas<T>& g, int lim, const T (&w)[3]) {
+    T P[3], M[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const T d = __shfl_down_sync(0xffffffffu, w[k], 1) - w[k];
+        const T s = limit(__shfl_up_sync(0xffffffffu, d, 1), d, lim);
+        P[k] = w[k] + T(0.5) * s;
+        M[k] = __shfl_down_sync(0xffffffffu, w[k] - T(0.5) * s, 1);
+    }
+    return face_flux(g, P[0], P[1], P[2], M[0], M[1], M[2]);
+}
+
 // One whole RK2 (Heun) step in one launch, out of place (Un -> Unext; the
-// caller alternates two buffers).  A CTA owns T1 cells and keeps everything
-// of its step in shared memory:
-//   U^n and its primitives over the cells c0-4 .. c0+T1+3,
-//   the stage-1 faces and U1 over c0-2 .. c0+T1+1 (the 2-cell halo of U1 is
-//   recomputed here instead of being exchanged through global memory),
-//   the primitives of U1, the stage-2 faces and the Heun update of the T1
-//   cells, the new state's ghost copies, positivity check and max |u|+c.
-// Every value is computed by the same expression, on the same operands, as in
-// the two stage kernels (and nest's loop): U1 of a ghost cell is U1 of the
-// cell it copies, which the periodic wrap of the primitives gives directly
-// and the zero-gradient case takes from that cell's faces.  The wave-speed
-// maximum is reduced into maxs[q][1]; the last block to finish moves it to
-// maxs[q][0] (block 0 cannot clear a slot at its start that other blocks may
-// already be adding to).  U1out (optional) receives U1 of the step with its
-// ghosts.  A finished step (time, step count or error) copies Un to Unext so
-// that the state ends in the buffer the caller expects.
+// caller alternates two buffers).  A warp owns 24 cells and works alone: lane k
+// holds cell c0 - 4 + k (its U^n, primitives, U1 and its primitives in registers),
+// faces and neighbours' slopes come by shuffles.  The four lanes at each side are
+// the halo of the two stages, recomputed by the neighbouring warps instead of
+// being exchanged.  Every value is computed by the same expression, on the
+// same operands, as in the two stage kernels (and nest's loop): U1 of a ghost
+// cell is U1 of the cell it copies, which the periodic wrap of the primitives
+// gives directly and the zero-gradient case takes from that cell's lane.  The
+// block's maximum goes to the next step's slot in one fire-and-forget atomic
+// (publish_step_1d clears the words).  U1out (optional) receives U1 of the step
+// with its ghosts.  A finished step (time, step count or error) copies Un to
+// Unext so that the state ends in the buffer the caller expects.
+// Bound: one chain of two stages and the launch.  us per step (FP64 5003 / 65536 /
+// 200003 cells, FP32 50021): 4.10 / 6.03 / 12.5, 2.95, against 6.03 / 7.32 / 14.3, 5.52 with 224-cell
+// CTAs that staged each phase through shared memory and moved the maximum with
+// a counter of finished blocks.
 template <typename T, int LIM>
-__global__ void __launch_bounds__(NT1)
+__global__ void __launch_bounds__(32 * STEP_WARPS)
 k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out, int n, int h, double dx,
          double gamma_d, int bc, LoopParams lp, StepCtrl* ctrl, int p) {
-    __shared__ T Q[3][T1 + 8];  // U^n, cells c0-4 ..
-    __shared__ T W[3][T1 + 8];  // primitives of U^n (cells c0-4 ..), then of U1 (cells c0-2 ..)
-    __shared__ T F[3][T1 + 5];  // faces of the stage
-    __shared__ T V[3][T1 + 4];  // U1, cells c0-2 ..
-    __shared__ double red[NT1 / 32];
+    __shared__ double red[STEP_WARPS];
+    const Gas<T> gas(gamma_d);
+    const int nt = n + 2 * h;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c0 = (blockIdx.x * STEP_WARPS + warp) * STEP_CELLS, c = c0 - 4 + lane;
+    const bool own = lane >= 4 && lane < 4 + STEP_CELLS && c < n;
+    const int e = h + source_cell_1d(c, n, bc);
+    const int lim = LIM >= 0 ? LIM : lp.lim;
+    const double rdx = lp.cfl * dx;
+    auto store = [&](T* U, const T (&v)[3]) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            U[k * nt + h + c] = v[k];
+            push_ghosts_1d(U, nt, k, c, n, h, bc, v[k]);
+        }
+    };
     pdl_wait();
     pdl_trigger();
-    const int nt = n + 2 * h;
-    const Gas<T> gas(gamma_d);
-    const int c0 = blockIdx.x * T1;
+    const T u[3] = { Un[e], Un[nt + e], Un[2 * nt + e] };
     if (step_is_done(ctrl, p, lp)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) publish_step(ctrl, p, lp, true, 0.0, false);
-        for (int t = threadIdx.x; t < T1; t += NT1) {
-            const int c = c0 + t;
-            if (c < n)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const T v = Un[k * nt + h + c];
-                    Unext[k * nt + h + c] = v;
-                    push_ghosts_1d(Unext, nt, k, c, n, h, bc, v);
-                }
-        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) publish_step_1d(ctrl, p, lp, true, 0.0, true);
+        if (own) store(Unext, u);
         return;
     }
+    T w[3];
+    {
+        const Cell1<T> q = cell1d<false>(gas, u[0], u[1], u[2]);
+        w[0] = u[0]; w[1] = q.u; w[2] = q.p;
+    }
+    const F3<T> f = warp_flux(gas, lim, w);  // needs no dt
+    const int sel = ctrl->sel[p];
     double dt;
     {
         const double pd = prescribed_dt(ctrl, p, lp);
         if (pd > 0.0) {
             dt = pd;
         } else {
-            dt = lp.cfl * dx / bits_speed(ctrl->maxs[p][0]);
+            dt = div_rn(rdx, bits_speed(ctrl->maxs[p][sel & 1]));
             if (lp.t_final > 0.0) dt = smin(dt, lp.t_final - ctrl->time[p]);
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) publish_step(ctrl, p, lp, false, dt, false);
-    const T dtdx = (T)(dt / dx);
+    if (blockIdx.x == 0 && threadIdx.x == 0) publish_step_1d(ctrl, p, lp, false, dt, true);
+    const T dtdx = (T)div_rn(dt, dx);
 
-    // U^n and its primitives, cells c0-4+t (read from the interior cell each copies)
-    for (int t = threadIdx.x; t < T1 + 8; t += NT1) {
-        const int e = h + source_cell_1d(c0 - 4 + t, n, bc);
-        const T rho = Un[e], mom = Un[nt + e], erg = Un[2 * nt + e];
-        Q[0][t] = rho; Q[1][t] = mom; Q[2][t] = erg;
-        const Cell1<T> w = cell1d<false>(gas, rho, mom, erg);
-        W[0][t] = rho;
-        W[1][t] = w.u;
-        W[2][t] = w.p;
-    }
-    __syncthreads();
-    // face f between the cells of W slots f+1 and f+2
-    auto faces = [&](int nf) {
-        for (int f = threadIdx.x; f < nf; f += NT1) {
-            const F3<T> q = plm_flux(gas, LIM >= 0 ? LIM : lp.lim, [&](int k, int t) { return W[k][t]; }, f, f + 1, f + 2, f + 3);
-            F[0][f] = q.a; F[1][f] = q.b; F[2][f] = q.c;
-        }
-    };
-    faces(T1 + 5);  // stage 1: faces between cells c0-3+f and c0-2+f
-    __syncthreads();
-    // U1 of cells c0-2+u (faces u, u+1; U^n slot u+2) and its primitives into W slot u
-    for (int u = threadIdx.x; u < T1 + 4; u += NT1) {
-        // zero-gradient ghost: the value of the end cell it copies, which lies
-        // in this window whenever the window reaches past the domain
-        const int us = bc == BC_PERIODIC ? u : source_cell_1d(c0 - 2 + u, n, bc) - c0 + 2;
-        T v[3];
+    T v[3] = { u[0] - dtdx * (f.a - __shfl_up_sync(0xffffffffu, f.a, 1)),
+               u[1] - dtdx * (f.b - __shfl_up_sync(0xffffffffu, f.b, 1)),
+               u[2] - dtdx * (f.c - __shfl_up_sync(0xffffffffu, f.c, 1)) };
+    if (bc != BC_PERIODIC && (c0 < 4 || c0 + STEP_CELLS + 4 > n)) {
+        // zero-gradient ghosts: U1 of the end cell they copy, a lane of this warp
+        // whenever the warp reaches past the domain
+        const int src = min(max(c, 0), n - 1) - (c0 - 4);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            v[k] = Q[k][us + 2] - dtdx * (F[k][us + 1] - F[k][us]);
-            V[k][u] = v[k];
-        }
-        const Cell1<T> w = cell1d<false>(gas, v[0], v[1], v[2]);
-        W[0][u] = v[0];
-        W[1][u] = w.u;
-        W[2][u] = w.p;
+        for (int k = 0; k < 3; ++k) v[k] = __shfl_sync(0xffffffffu, v[k], src & 31);
     }
-    __syncthreads();
-    faces(T1 + 1);  // stage 2: faces between cells c0-1+f and c0+f
-    __syncthreads();
-    const int t = threadIdx.x, c = c0 + t;
+    {
+        const Cell1<T> q = cell1d<false>(gas, v[0], v[1], v[2]);
+        w[0] = v[0]; w[1] = q.u; w[2] = q.p;
+    }
+    const F3<T> g = warp_flux(gas, lim, w);
+    const T x[3] = { T(0.5) * (u[0] + (v[0] - dtdx * (g.a - __shfl_up_sync(0xffffffffu, g.a, 1)))),
+                     T(0.5) * (u[1] + (v[1] - dtdx * (g.b - __shfl_up_sync(0xffffffffu, g.b, 1)))),
+                     T(0.5) * (u[2] + (v[2] - dtdx * (g.c - __shfl_up_sync(0xffffffffu, g.c, 1)))) };
+    const Cell1<T> q = cell1d<true>(gas, x[0], x[1], x[2]);
     double ms = 0.0;
-    if (t < T1 && c < n) {
-        const int e = h + c;
-        T v[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const T s = V[k][t + 2] - dtdx * (F[k][t + 1] - F[k][t]);
-            v[k] = T(0.5) * (Q[k][t + 4] + s);
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            Unext[k * nt + e] = v[k];
-            push_ghosts_1d(Unext, nt, k, c, n, h, bc, v[k]);
-            if (U1out) {
-                U1out[k * nt + e] = V[k][t + 2];
-                push_ghosts_1d(U1out, nt, k, c, n, h, bc, V[k][t + 2]);
-            }
-        }
-        const Cell1<T> w = cell1d<true>(gas, v[0], v[1], v[2]);
-        ms = (double)(fabs(w.u) + w.cs);
-        if (!(v[0] > T(0)) || !(w.p > T(0))) flag_cell(ctrl, ctrl->step[p] + 1, (double)v[0], (double)w.p, c, 0);
+    if (own) {
+        store(Unext, x);
+        if (U1out) store(U1out, v);
+        ms = (double)(fabs(q.u) + q.cs);
+        if (!(x[0] > T(0)) || !(q.p > T(0))) flag_cell(ctrl, ctrl->step[p] + 1, (double)x[0], (double)q.p, c, 0);
     }
-    ms = warp_max(ms);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) red[w] = ms;
+    ms = warp_max_speed(ms);
+    if (lane == 0) red[warp] = ms;
     __syncthreads();
-    if (w == 0) {
-        double x = (l < NT1 / 32) ? red[l] : 0.0;
-        x = warp_max(x);
-        if (l == 0) {
-            const int q = p ^ 1;
-            if (!(x == x) || x > 1.79e308) atomicOr(&ctrl->err, ERRW_NONFINITE);
-            atomic_max_speed(&ctrl->maxs[q][1], x);
-            __threadfence();
-            if (atomicAdd(&ctrl->blocks_done, 1u) == gridDim.x - 1) {
-                // every block has added its maximum
-                __threadfence();
-                ctrl->maxs[q][0] = atomicExch(&ctrl->maxs[q][1], 0ull);
-                ctrl->blocks_done = 0u;
-            }
-        }
+    if (threadIdx.x == 0) {
+        // as bit patterns, which order like the speeds (a NaN above them all)
+        unsigned long long m = speed_bits(red[0]);
+        for (int i = 1; i < STEP_WARPS; ++i) m = max(m, speed_bits(red[i]));
+        if (!(bits_speed(m) <= 1.79e308)) atomicOr(&ctrl->err, ERRW_NONFINITE);
+        atomicMax(&ctrl->maxs[p ^ 1][sel >> 1], m);
     }
 }
 
@@ -332,9 +312,9 @@ cudaError_t launch_1d_step_t(T* U, T* U1, int n, int h, double dx, double gamma,
 template <typename T>
 cudaError_t launch_1d_fused_t(const T* Un, T* Unext, T* U1out, int n, int h, double dx, double gamma, int bc,
                               const LoopParams& lp, StepCtrl* ctrl, int p, cudaStream_t st) {
-    int blocks = (n + T1 - 1) / T1;
-    return launch_pdl(lp.lim == LIM_MINMOD ? k1d_step<T, LIM_MINMOD> : k1d_step<T, -1>, dim3(blocks), dim3(NT1), 0, st,
-                      Un, Unext, U1out, n, h, dx, gamma, bc, lp, ctrl, p);
+    const int cells = STEP_CELLS * STEP_WARPS, blocks = (n + cells - 1) / cells;
+    return launch_pdl(lp.lim == LIM_MINMOD ? k1d_step<T, LIM_MINMOD> : k1d_step<T, -1>, dim3(blocks),
+                      dim3(32 * STEP_WARPS), 0, st, Un, Unext, U1out, n, h, dx, gamma, bc, lp, ctrl, p);
 }
 
 }  // namespace
