@@ -11,7 +11,7 @@
 //     both stages, Heun average) with no kernel boundary and no host round-trip
 //     per step, up to 4080 cells.  Where no cluster can be placed, one CTA with
 //     several cells per thread (k1d_resident) takes up to about 2300.
-//   * tiled (euler1d_tiled.cuh): a whole step per launch, a warp per 24 cells
+//   * tiled (euler1d_tiled.cuh): a whole step per launch, a warp per 24 or 56 cells
 //     (the stage-1 halo recomputed per warp), or the two stage kernels; stage
 //     2 fuses the Heun average, the ghost fill of the new state and the
 //     max-wave-speed reduction; dt is derived on the device from that

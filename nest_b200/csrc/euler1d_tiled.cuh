@@ -10,7 +10,7 @@
 // |u|+c (one atomic per block).  dt is derived on the device from that
 // maximum by the next stage 1, so a step is two launches and no host
 // synchronisation.  k1d_step runs a whole step in one launch (out of place), a
-// warp per 24 cells with nothing in shared memory.
+// warp per 24 or 56 cells with nothing in shared memory.
 #pragma once
 
 #include "euler1d_arith.cuh"
@@ -134,76 +134,117 @@ __device__ __forceinline__ int source_cell_1d(int c, int n, int bc) {
     return min(max(c, 0), n - 1);
 }
 
-constexpr int STEP_CELLS = 24;  // output cells per warp of k1d_step
-constexpr int STEP_WARPS = 4;   // warps per CTA
+constexpr int STEP_WARPS = 4;  // warps per CTA of k1d_step
+// output cells of a warp with CPL cells per lane: all but four at each end
+__host__ __device__ constexpr int step_cells(int cpl) { return 32 * cpl - 8; }
 
-// Stage fluxes of a warp whose lane k holds the primitives w of cell k: lane k
-// returns the face between cells k and k+1 (k = 1 .. 29 where all 32 cells are
-// valid), in the expressions of plm_flux.
-template <typename T>
-__device__ __forceinline__ F3<T> warp_flux(const Gas<T>& g, int lim, const T (&w)[3]) {
-    T P[3], M[3];
+// Stage fluxes of a warp whose lanes hold the primitives w of CPL neighbouring
+// cells each: f[i] is the face to the right of the lane's cell i, in the
+// expressions of plm_flux (valid two cells inside the valid ones).
+template <typename T, int CPL>
+__device__ __forceinline__ void warp_flux(const Gas<T>& g, int lim, const T (&w)[CPL][3], F3<T> (&f)[CPL]) {
+    T P[CPL][3], M[CPL + 1][3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const T d = __shfl_down_sync(0xffffffffu, w[k], 1) - w[k];
-        const T s = limit(__shfl_up_sync(0xffffffffu, d, 1), d, lim);
-        P[k] = w[k] + T(0.5) * s;
-        M[k] = __shfl_down_sync(0xffffffffu, w[k] - T(0.5) * s, 1);
+        T d[CPL];
+#pragma unroll
+        for (int i = 0; i < CPL; ++i)
+            d[i] = (i + 1 < CPL ? w[i + 1 < CPL ? i + 1 : 0][k] : __shfl_down_sync(0xffffffffu, w[0][k], 1)) - w[i][k];
+        const T dm = __shfl_up_sync(0xffffffffu, d[CPL - 1], 1);
+#pragma unroll
+        for (int i = 0; i < CPL; ++i) {
+            const T s = limit(i > 0 ? d[i > 0 ? i - 1 : 0] : dm, d[i], lim);
+            P[i][k] = w[i][k] + T(0.5) * s;
+            M[i][k] = w[i][k] - T(0.5) * s;
+        }
+        M[CPL][k] = __shfl_down_sync(0xffffffffu, M[0][k], 1);
     }
-    return face_flux(g, P[0], P[1], P[2], M[0], M[1], M[2]);
+#pragma unroll
+    for (int i = 0; i < CPL; ++i)
+        f[i] = face_flux(g, P[i][0], P[i][1], P[i][2], M[i + 1][0], M[i + 1][1], M[i + 1][2]);
+}
+
+// v[i] = u[i] - dtdx (right flux - left flux) of the lane's cells.
+template <typename T, int CPL>
+__device__ __forceinline__ void warp_update(const T (&u)[CPL][3], const F3<T> (&f)[CPL], T dtdx, T (&v)[CPL][3]) {
+    const F3<T> l = { __shfl_up_sync(0xffffffffu, f[CPL - 1].a, 1), __shfl_up_sync(0xffffffffu, f[CPL - 1].b, 1),
+                      __shfl_up_sync(0xffffffffu, f[CPL - 1].c, 1) };
+#pragma unroll
+    for (int i = 0; i < CPL; ++i) {
+        const F3<T> q = i > 0 ? f[i > 0 ? i - 1 : 0] : l;
+        v[i][0] = u[i][0] - dtdx * (f[i].a - q.a);
+        v[i][1] = u[i][1] - dtdx * (f[i].b - q.b);
+        v[i][2] = u[i][2] - dtdx * (f[i].c - q.c);
+    }
 }
 
 // One whole RK2 (Heun) step in one launch, out of place (Un -> Unext; the
-// caller alternates two buffers).  A warp owns 24 cells and works alone: lane k
-// holds cell c0 - 4 + k (its U^n, primitives, U1 and its primitives in registers),
-// faces and neighbours' slopes come by shuffles.  The four lanes at each side are
-// the halo of the two stages, recomputed by the neighbouring warps instead of
-// being exchanged.  Every value is computed by the same expression, on the
-// same operands, as in the two stage kernels (and nest's loop): U1 of a ghost
-// cell is U1 of the cell it copies, which the periodic wrap of the primitives
-// gives directly and the zero-gradient case takes from that cell's lane.  The
-// block's maximum goes to the next step's slot in one fire-and-forget atomic
-// (publish_step_1d clears the words).  U1out (optional) receives U1 of the step
-// with its ghosts.  A finished step (time, step count or error) copies Un to
-// Unext so that the state ends in the buffer the caller expects.
+// caller alternates two buffers).  A warp owns 24 cells (56 with two per lane)
+// and works alone: lane k holds cells c0 - 4 + CPL k .. (their U^n, primitives, U1
+// and its primitives in registers), faces and neighbours' slopes come by
+// shuffles.  The four cells at each end are the halo of the two stages,
+// recomputed by the neighbouring warps instead of being exchanged.  Every value
+// is computed by the same expression, on the same operands, as in the two stage
+// kernels (and nest's loop): U1 of a ghost cell is U1 of the cell it copies, which
+// the periodic wrap of the primitives gives directly and the zero-gradient case
+// takes from that cell's lane.  The block's maximum goes to the next step's slot
+// in one fire-and-forget atomic (publish_step_1d clears the words).  U1out
+// (optional) receives U1 of the step with its ghosts.  A finished step (time,
+// step count or error) copies Un to Unext so that the state ends in the buffer
+// the caller expects.
 // Bound: one chain of two stages and the launch.  us per step (FP64 5003 / 65536 /
-// 200003 cells, FP32 50021): 4.10 / 6.03 / 12.5, 2.95, against 6.03 / 7.32 / 14.3, 5.52 with 224-cell
-// CTAs that staged each phase through shared memory and moved the maximum with
-// a counter of finished blocks.
-template <typename T, int LIM>
+// 200003 cells, FP32 50021): 4.1 / 5.1 / 10.8, 3.0, against 6.0 / 7.3 / 14.3, 5.5 with
+// 224-cell CTAs that staged each phase through shared memory and moved the
+// maximum with a counter of finished blocks.
+template <typename T, int LIM, int CPL>
 __global__ void __launch_bounds__(32 * STEP_WARPS)
 k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out, int n, int h, double dx,
          double gamma_d, int bc, LoopParams lp, StepCtrl* ctrl, int p) {
+    constexpr int CELLS = step_cells(CPL);
     __shared__ double red[STEP_WARPS];
     const Gas<T> gas(gamma_d);
     const int nt = n + 2 * h;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int c0 = (blockIdx.x * STEP_WARPS + warp) * STEP_CELLS, c = c0 - 4 + lane;
-    const bool own = lane >= 4 && lane < 4 + STEP_CELLS && c < n;
-    const int e = h + source_cell_1d(c, n, bc);
+    const int c0 = (blockIdx.x * STEP_WARPS + warp) * CELLS, c = c0 - 4 + CPL * lane;
     const int lim = LIM >= 0 ? LIM : lp.lim;
     const double rdx = lp.cfl * dx;
-    auto store = [&](T* U, const T (&v)[3]) {
+    auto own = [&](int i) {
+        const int x = CPL * lane + i;
+        return x >= 4 && x < 4 + CELLS && c + i < n;
+    };
+    auto store = [&](T* U, const T (&v)[3], int ci) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            U[k * nt + h + c] = v[k];
-            push_ghosts_1d(U, nt, k, c, n, h, bc, v[k]);
+            U[k * nt + h + ci] = v[k];
+            push_ghosts_1d(U, nt, k, ci, n, h, bc, v[k]);
         }
     };
+    T u[CPL][3], v[CPL][3], w[CPL][3];
+    int e[CPL];
+#pragma unroll
+    for (int i = 0; i < CPL; ++i) e[i] = h + source_cell_1d(c + i, n, bc);
     pdl_wait();
     pdl_trigger();
-    const T u[3] = { Un[e], Un[nt + e], Un[2 * nt + e] };
+#pragma unroll
+    for (int i = 0; i < CPL; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) u[i][k] = Un[k * nt + e[i]];
     if (step_is_done(ctrl, p, lp)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) publish_step_1d(ctrl, p, lp, true, 0.0, true);
-        if (own) store(Unext, u);
+        for (int i = 0; i < CPL; ++i)
+            if (own(i)) store(Unext, u[i], c + i);
         return;
     }
-    T w[3];
-    {
-        const Cell1<T> q = cell1d<false>(gas, u[0], u[1], u[2]);
-        w[0] = u[0]; w[1] = q.u; w[2] = q.p;
-    }
-    const F3<T> f = warp_flux(gas, lim, w);  // needs no dt
+    auto prims = [&](const T (&a)[CPL][3]) {
+#pragma unroll
+        for (int i = 0; i < CPL; ++i) {
+            const Cell1<T> q = cell1d<false>(gas, a[i][0], a[i][1], a[i][2]);
+            w[i][0] = a[i][0]; w[i][1] = q.u; w[i][2] = q.p;
+        }
+    };
+    F3<T> f[CPL];
+    prims(u);
+    warp_flux(gas, lim, w, f);  // needs no dt
     const int sel = ctrl->sel[p];
     double dt;
     {
@@ -218,41 +259,52 @@ k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out,
     if (blockIdx.x == 0 && threadIdx.x == 0) publish_step_1d(ctrl, p, lp, false, dt, true);
     const T dtdx = (T)div_rn(dt, dx);
 
-    T v[3] = { u[0] - dtdx * (f.a - __shfl_up_sync(0xffffffffu, f.a, 1)),
-               u[1] - dtdx * (f.b - __shfl_up_sync(0xffffffffu, f.b, 1)),
-               u[2] - dtdx * (f.c - __shfl_up_sync(0xffffffffu, f.c, 1)) };
-    if (bc != BC_PERIODIC && (c0 < 4 || c0 + STEP_CELLS + 4 > n)) {
-        // zero-gradient ghosts: U1 of the end cell they copy, a lane of this warp
-        // whenever the warp reaches past the domain
-        const int src = min(max(c, 0), n - 1) - (c0 - 4);
+    warp_update(u, f, dtdx, v);
+    if (bc != BC_PERIODIC && (c0 < 4 || c0 + CELLS + 4 > n)) {
+        // zero-gradient ghosts: U1 of the end cell they copy, held by a lane of this
+        // warp whenever the warp reaches past the domain
+        T r[CPL][3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) v[k] = __shfl_sync(0xffffffffu, v[k], src & 31);
+        for (int i = 0; i < CPL; ++i) {
+            const int x = (min(max(c + i, 0), n - 1) - (c0 - 4)) & (32 * CPL - 1);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                r[i][k] = __shfl_sync(0xffffffffu, v[0][k], x / CPL);
+                if (CPL > 1) {
+                    const T hi = __shfl_sync(0xffffffffu, v[CPL - 1][k], x / CPL);
+                    if (x % CPL) r[i][k] = hi;
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < CPL; ++i)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[i][k] = r[i][k];
     }
-    {
-        const Cell1<T> q = cell1d<false>(gas, v[0], v[1], v[2]);
-        w[0] = v[0]; w[1] = q.u; w[2] = q.p;
-    }
-    const F3<T> g = warp_flux(gas, lim, w);
-    const T x[3] = { T(0.5) * (u[0] + (v[0] - dtdx * (g.a - __shfl_up_sync(0xffffffffu, g.a, 1)))),
-                     T(0.5) * (u[1] + (v[1] - dtdx * (g.b - __shfl_up_sync(0xffffffffu, g.b, 1)))),
-                     T(0.5) * (u[2] + (v[2] - dtdx * (g.c - __shfl_up_sync(0xffffffffu, g.c, 1)))) };
-    const Cell1<T> q = cell1d<true>(gas, x[0], x[1], x[2]);
+    prims(v);
+    warp_flux(gas, lim, w, f);
+    warp_update(v, f, dtdx, w);
     double ms = 0.0;
-    if (own) {
-        store(Unext, x);
-        if (U1out) store(U1out, v);
-        ms = (double)(fabs(q.u) + q.cs);
-        if (!(x[0] > T(0)) || !(q.p > T(0))) flag_cell(ctrl, ctrl->step[p] + 1, (double)x[0], (double)q.p, c, 0);
+#pragma unroll
+    for (int i = 0; i < CPL; ++i) {
+        const T x[3] = { T(0.5) * (u[i][0] + w[i][0]), T(0.5) * (u[i][1] + w[i][1]), T(0.5) * (u[i][2] + w[i][2]) };
+        const Cell1<T> q = cell1d<true>(gas, x[0], x[1], x[2]);
+        if (own(i)) {
+            store(Unext, x, c + i);
+            if (U1out) store(U1out, v[i], c + i);
+            // (a NaN is dropped here and flagged below)
+            ms = smax(ms, (double)(fabs(q.u) + q.cs));
+            if (!(x[0] > T(0)) || !(q.p > T(0))) flag_cell(ctrl, ctrl->step[p] + 1, (double)x[0], (double)q.p, c + i, 0);
+        }
     }
     ms = warp_max_speed(ms);
     if (lane == 0) red[warp] = ms;
     __syncthreads();
     if (threadIdx.x == 0) {
-        // as bit patterns, which order like the speeds (a NaN above them all)
-        unsigned long long m = speed_bits(red[0]);
-        for (int i = 1; i < STEP_WARPS; ++i) m = max(m, speed_bits(red[i]));
-        if (!(bits_speed(m) <= 1.79e308)) atomicOr(&ctrl->err, ERRW_NONFINITE);
-        atomicMax(&ctrl->maxs[p ^ 1][sel >> 1], m);
+        double m = red[0];
+        for (int i = 1; i < STEP_WARPS; ++i) m = smax(m, red[i]);
+        if (m > 1.79e308) atomicOr(&ctrl->err, ERRW_NONFINITE);
+        atomic_max_speed(&ctrl->maxs[p ^ 1][sel >> 1], m);
     }
 }
 
@@ -309,12 +361,23 @@ cudaError_t launch_1d_step_t(T* U, T* U1, int n, int h, double dx, double gamma,
     return e;
 }
 
+// Cells from which k1d_step takes two per lane: fewer halo cells and more
+// independent work per warp against a longer chain, and below half the blocks
+// fit an SM beside those of the next launch, which wait there.  us per step, one /
+// two per lane: FP64 30000 cells 4.36 / 4.87, 50021 5.91 / 5.27, 65536 6.04 / 5.13,
+// 200003 12.4 / 10.8, 400000 22.8 / 19.2; FP32 50021 3.34 / 3.73, 65536 3.46 / 3.47,
+// 100000 5.41 / 3.97, 400000 14.3 / 9.4.
+template <typename T> constexpr int STEP_TWO_CELLS = sizeof(T) == 8 ? 40000 : 80000;
+
 template <typename T>
 cudaError_t launch_1d_fused_t(const T* Un, T* Unext, T* U1out, int n, int h, double dx, double gamma, int bc,
                               const LoopParams& lp, StepCtrl* ctrl, int p, cudaStream_t st) {
-    const int cells = STEP_CELLS * STEP_WARPS, blocks = (n + cells - 1) / cells;
-    return launch_pdl(lp.lim == LIM_MINMOD ? k1d_step<T, LIM_MINMOD> : k1d_step<T, -1>, dim3(blocks),
-                      dim3(32 * STEP_WARPS), 0, st, Un, Unext, U1out, n, h, dx, gamma, bc, lp, ctrl, p);
+    const bool two = n >= STEP_TWO_CELLS<T>;
+    const int cells = step_cells(two ? 2 : 1) * STEP_WARPS, blocks = (n + cells - 1) / cells;
+    auto kern = lp.lim == LIM_MINMOD ? (two ? k1d_step<T, LIM_MINMOD, 2> : k1d_step<T, LIM_MINMOD, 1>)
+                                     : (two ? k1d_step<T, -1, 2> : k1d_step<T, -1, 1>);
+    return launch_pdl(kern, dim3(blocks), dim3(32 * STEP_WARPS), 0, st, Un, Unext, U1out, n, h, dx, gamma, bc, lp,
+                      ctrl, p);
 }
 
 }  // namespace
