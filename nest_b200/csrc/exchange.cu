@@ -72,6 +72,15 @@ struct nest_exchange {
     long long total = 0;
 };
 
+// Every copy of a 1D plan as a (destination, source) pair of element offsets.
+std::vector<std::pair<long long, long long>> nestb::exchange_pairs_1d(const nest_exchange* x) {
+    std::vector<std::pair<long long, long long>> v;
+    for (const Region& r : x->regs)
+        for (int k = 0; k < x->nvars; ++k)
+            for (int a = 0; a < r.n0; ++a) v.push_back({r.dst + k * r.dvar + a, r.src + k * r.svar + a});
+    return v;
+}
+
 extern "C" {
 
 nest_status nest_exchange_create_periodic(int dim, int nx, int ny, int npx, int npy, int nvars, int halo,

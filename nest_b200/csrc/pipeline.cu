@@ -23,13 +23,16 @@
 //              (compute_dt, sod1d.cpp:97-128 and :222-223),
 //   CHECK      nest's positivity check every `k` steps (sod1d.cpp:279-301),
 //   CLOCK      time += dt, step += 1.
-// dt, time and the step count live in a device control block, so a step
-// needs no host synchronisation and runs of steps are replayed from CUDA
-// graphs.  A CFL_DT stage that finds time >= t_final marks the step
+// A 1D pipeline of up to 16384 cells runs whole, all stages and all steps, in one
+// launch of one CTA or one thread-block cluster (k_pipe_loop); others run a
+// launch per stage.  dt, time and the step count live in a device control block,
+// so a step needs no host synchronisation and runs of per-stage steps are
+// replayed from CUDA graphs.  A CFL_DT stage that finds time >= t_final marks the step
 // inactive: the later stages of that execution do nothing.
 //
 // Compiled with -fmad=false: every formula keeps nest's operation order, so
 // results equal nest's CPU code bit for bit.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -38,11 +41,13 @@
 #include <new>
 #include <vector>
 
+#include "euler1d_arith.cuh"
 #include "solver_impl.h"
 
 using namespace nestb;
 using namespace nestb::rt;
 
+namespace nestb {
 namespace {
 
 // One patch of the storage: element offset of its block, interior extents
@@ -202,7 +207,200 @@ struct Stage {
     double param;
 };
 
+// ---------------------------------------------------------------------------
+// The whole pipeline in one launch (1D)
+// ---------------------------------------------------------------------------
+
+constexpr int LOOP_STAGES = 32, LOOP_BUFFERS = 17;
+constexpr int LOOP_THREADS = 512, LOOP_K = 2;  // threads per CTA, cells per thread
+// Up to this many cells one CTA (cheap barriers), above a cluster of 16, whose six
+// barriers a step cost about 0.45 us each: us per step, one CTA / cluster, 400 cells
+// 10.1 / 14.2, 640 14.0 / 13.9, 1024 16.9 / 14.5.
+constexpr int LOOP_ONE_CTA = 640;
+
+struct LoopArgs {
+    int nstages;
+    Stage st[LOOP_STAGES];
+    unsigned sync_before;         // bit s: stage s needs a barrier before it
+    double* buf[LOOP_BUFFERS];
+    const PatchInfo* P;
+    int npatch, ncells, h;
+    const int2* copies;           // exchange: (destination, source) element offsets
+    int ncopies;
+    double dx, gamma;
+    int lim;
+    PipeCtrl* c;
+    int steps;                    // executions of the stage list at most
+    int max_steps, step0;         // > 0: stop at a multiple of 8 executions once step - step0 reaches it
+};
+
+// Executes the stage list up to `steps` times in one CTA or one cluster: a
+// thread owns up to LOOP_K cells in every stage, so element-wise stages follow
+// one another without a barrier, and only a stage that reads other threads'
+// elements (EXCHANGE, EULER_RHS, the CFL maximum), or overwrites what others may
+// still be reading, waits for one (LoopArgs::sync_before).  Every thread keeps the
+// clock in registers; they all compute the same dt.  The formulas are those of
+// the stage kernels above, with the branch-free division and square root.
+// An execution whose CFL stage finds the run finished is the last one (its halo
+// exchanges still run; further ones would change nothing).
+// Bound: the latency of the stages' chains and their barriers.  nest's sod1d step
+// (ten stages, twelve launches), us per step against a launch per stage: 100 cells
+// 7.0 (26), 400 10.1 (30), 1024 14.5 (31), 4000 14.6 (31), 16000 26 (38).
+template <bool CLUSTER>
+__global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
+    namespace cg = cooperative_groups;
+    __shared__ double red[2][16 * (LOOP_THREADS / 32)];
+    const int NC = CLUSTER ? (int)cg::this_cluster().num_blocks() : 1;
+    const int rank = CLUSTER ? (int)cg::this_cluster().block_rank() : 0;
+    auto sync = [&]() {
+        if (CLUSTER) cg::this_cluster().sync();
+        else __syncthreads();
+    };
+    const int T = blockDim.x, nw = T >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int gt = rank * T + threadIdx.x, NT = NC * T;
+    const Gas<double> gas(a.gamma);
+    const double gm1 = a.gamma - 1.0;
+    PipeCtrl* const c = a.c;
+
+    // the thread's cells: element offset, plane stride, place in the patch
+    struct Own {
+        long long e;
+        int plane, patch, i, n0;
+    } own[LOOP_K];
+#pragma unroll
+    for (int k = 0; k < LOOP_K; ++k) {
+        own[k] = { 0, 0, -1, 0, 0 };
+        int f = gt + k * NT;
+        if (f < a.ncells) {
+            int p = 0;
+            while (f >= a.P[p].n0) f -= a.P[p++].n0;
+            own[k] = { a.P[p].off + a.h + f, a.P[p].ext0, p, f, a.P[p].n0 };
+        }
+    }
+    double time = c->time, dt = c->dt;
+    int step = c->step, active = c->active;
+    const double t_final = c->t_final;
+    int cfl_count = 0;
+    if (CLUSTER) sync();  // every CTA of the cluster runs before its memory is written
+
+    for (int n = 0; n < a.steps; ++n) {
+        // batches of 8, as a launch per stage runs them
+        if (n > 0 && (n & 7) == 0 && ((a.max_steps > 0 && step - a.step0 >= a.max_steps) || !(time < t_final))) break;
+        bool finished = false;
+        for (int s = 0; s < a.nstages; ++s) {
+            const Stage& g = a.st[s];
+            if ((a.sync_before >> s) & 1u) sync();
+            double* const src = a.buf[g.src];
+            double* const dst = a.buf[g.dst];
+            if (g.kind == NEST_STAGE_CFL_DT) {
+                double ms = 0.0;
+#pragma unroll
+                for (int k = 0; k < LOOP_K; ++k)
+                    if (own[k].patch >= 0) {
+                        const long long e = own[k].e;
+                        const int pl = own[k].plane;
+                        const Cell1<double> w = cell1d<true>(gas, src[e], src[e + pl], src[e + 2 * pl]);
+                        ms = smax(ms, fabs(w.u) + w.cs);
+                    }
+                ms = warp_max_speed(ms);
+                double* const r = red[cfl_count & 1];
+                ++cfl_count;
+                if (lane < NC)
+                    (CLUSTER ? cg::this_cluster().map_shared_rank(r, lane) : r)[rank * nw + warp] = ms;
+                sync();
+                double m = 0.0;
+                for (int q = lane; q < NC * nw; q += 32) m = smax(m, r[q]);
+                m = warp_max_speed(m);
+                const unsigned err = *reinterpret_cast<volatile unsigned*>(&c->err);
+                active = (!(t_final > 0.0) || time < t_final) && !(err & ERRW_STOP) ? 1 : 0;
+                if (active) {
+                    dt = div_rn(g.param * a.dx, m);
+                    if (t_final > 0.0) dt = smin(dt, t_final - time);
+                }
+                finished = !active;
+                continue;
+            }
+            if (g.kind == NEST_STAGE_EXCHANGE) {
+                for (int q = gt; q < a.ncopies; q += NT) {
+                    const int2 d = a.copies[q];
+                    src[d.x] = src[d.y];
+                }
+                continue;
+            }
+            if (!active) continue;
+            switch (g.kind) {
+                case NEST_STAGE_EULER_RHS: {
+                    const double dtdx = div_rn(dt, a.dx);
+#pragma unroll
+                    for (int k = 0; k < LOOP_K; ++k) {
+                        if (own[k].patch < 0) continue;
+                        const long long e = own[k].e;
+                        const int pl = own[k].plane, i = own[k].i;
+                        double U[3], W[5][3];  // cells i-2 .. i+2
+#pragma unroll
+                        for (int q = 0; q < 5; ++q) {
+                            // one-sided at the patch edges: i-2 -> i-1 on the first cell, i+2 -> i+1 on the last
+                            const long long x = e + (q == 0 && i == 0 ? -1 : q == 4 && i == own[k].n0 - 1 ? 1 : q - 2);
+                            const double r = src[x], m = src[x + pl], E = src[x + 2 * pl];
+                            const Cell1<double> w = cell1d<false>(gas, r, m, E);
+                            W[q][0] = r; W[q][1] = w.u; W[q][2] = w.p;
+                            if (q == 2) { U[0] = r; U[1] = m; U[2] = E; }
+                        }
+                        double aL[3], aR[3], bL[3], bR[3], cL[3], cR[3];
+                        plm3(W[0], W[1], W[2], a.lim, aL, aR);
+                        plm3(W[1], W[2], W[3], a.lim, bL, bR);
+                        plm3(W[2], W[3], W[4], a.lim, cL, cR);
+                        const F3<double> fl = face_flux(gas, aR[0], aR[1], aR[2], bL[0], bL[1], bL[2]);
+                        const F3<double> fr = face_flux(gas, bR[0], bR[1], bR[2], cL[0], cL[1], cL[2]);
+                        dst[e] = U[0] - dtdx * (fr.a - fl.a);
+                        dst[e + pl] = U[1] - dtdx * (fr.b - fl.b);
+                        dst[e + 2 * pl] = U[2] - dtdx * (fr.c - fl.c);
+                    }
+                    break;
+                }
+                case NEST_STAGE_COPY:
+                case NEST_STAGE_AVERAGE: {
+                    const double* const aux = a.buf[g.aux];
+#pragma unroll
+                    for (int k = 0; k < LOOP_K; ++k)
+                        if (own[k].patch >= 0)
+                            for (int v = 0; v < 3; ++v) {
+                                const long long e = own[k].e + (long long)v * own[k].plane;
+                                dst[e] = g.kind == NEST_STAGE_COPY ? src[e] : 0.5 * src[e] + 0.5 * aux[e];
+                            }
+                    break;
+                }
+                case NEST_STAGE_CHECK:
+                    if ((step + 1) % (int)g.param == 0) {
+#pragma unroll
+                        for (int k = 0; k < LOOP_K; ++k)
+                            if (own[k].patch >= 0) {
+                                double r, u, p;
+                                prim1d(src, own[k].e, own[k].plane, gm1, r, u, p);
+                                if (!(r > 0.0) || !(p > 0.0)) {
+                                    const unsigned bit = (r == r && p == p) ? ERRW_NONPOSITIVE : ERRW_NONFINITE;
+                                    if (!(atomicOr(&c->err, bit) & ERRW_STOP)) {
+                                        c->bad_step = step + 1; c->bad_cell = own[k].i; c->bad_patch = own[k].patch;
+                                        c->bad_rho = r; c->bad_p = p;
+                                    }
+                                }
+                            }
+                    }
+                    break;
+                case NEST_STAGE_CLOCK:
+                    time = time + dt;
+                    step = step + 1;
+                    break;
+            }
+        }
+        if (finished) break;
+    }
+    if (CLUSTER) sync();  // no CTA leaves while another's stores to it may be in flight
+    if (gt == 0) { c->time = time; c->dt = dt; c->step = step; c->active = active; }
+}
+
 }  // namespace
+}  // namespace nestb
 
 struct nest_pipeline {
     nest_exchange* plan = nullptr;
@@ -216,10 +414,15 @@ struct nest_pipeline {
     PipeCtrl* ctrl = nullptr;
     PipeCtrl* host_ctrl = nullptr;
     std::vector<Stage> stages;
+    int ncells = 0;
+    int2* dcopies = nullptr;          // 1D: the exchange plan's element pairs
+    int ncopies = 0;
+    int loop_ctas = 0;                // CTAs of the one-launch form (0: a launch per stage)
     cudaStream_t own = nullptr;
     std::map<std::pair<void*, cudaStream_t>, cudaGraphExec_t> graphs;
 };
 
+namespace nestb {
 namespace {
 
 constexpr int PIPE_GRAPH_STEPS = 8;
@@ -273,6 +476,114 @@ cudaError_t launch_stage(nest_pipeline* p, const Stage& s, void* state, cudaStre
     return cudaGetLastError();
 }
 
+// Barriers of the one-launch form: what has happened to each buffer since the
+// last one decides whether a stage must wait (the list repeats, so it starts from
+// what its own end leaves behind).
+unsigned loop_barriers(const std::vector<Stage>& st) {
+    struct Seen {
+        bool own_written = false;   // interiors, each element by its owner
+        bool halo_written = false;
+        bool read_across = false;   // by threads other than the owner
+    };
+    unsigned bits = 0;
+    Seen b[LOOP_BUFFERS];
+    for (int pass = 0; pass < 2; ++pass)
+        for (size_t s = 0; s < st.size(); ++s) {
+            const Stage& g = st[s];
+            bool wait = false;
+            switch (g.kind) {
+                case NEST_STAGE_EXCHANGE: wait = b[g.src].own_written || b[g.src].read_across; break;
+                case NEST_STAGE_EULER_RHS:
+                    wait = b[g.src].own_written || b[g.src].halo_written || b[g.dst].read_across;
+                    break;
+                case NEST_STAGE_COPY:
+                case NEST_STAGE_AVERAGE: wait = b[g.dst].read_across; break;
+                default: break;
+            }
+            if (wait) {
+                bits |= 1u << s;
+                for (Seen& x : b) x = Seen{};
+            }
+            switch (g.kind) {
+                case NEST_STAGE_EXCHANGE: b[g.src].read_across = b[g.src].halo_written = true; break;
+                case NEST_STAGE_EULER_RHS: b[g.src].read_across = b[g.dst].own_written = true; break;
+                case NEST_STAGE_COPY:
+                case NEST_STAGE_AVERAGE: b[g.dst].own_written = true; break;
+                case NEST_STAGE_CFL_DT:  // waits inside, after its own reads
+                    for (Seen& x : b) x = Seen{};
+                    break;
+                default: break;
+            }
+        }
+    return bits;
+}
+
+bool use_loop(const nest_pipeline* p) { return p->loop_ctas > 0 && p->stages.size() <= LOOP_STAGES; }
+
+cudaError_t launch_loop(nest_pipeline* p, void* state, int steps, int max_steps, int step0, cudaStream_t st) {
+    LoopArgs a{};
+    a.nstages = (int)p->stages.size();
+    for (int s = 0; s < a.nstages; ++s) a.st[s] = p->stages[s];
+    a.sync_before = loop_barriers(p->stages);
+    for (int b = 0; b <= p->nwork; ++b) a.buf[b] = buffer(p, state, b);
+    a.P = p->dpatches;
+    a.npatch = p->npatch; a.ncells = p->ncells; a.h = p->halo;
+    a.copies = p->dcopies; a.ncopies = p->ncopies;
+    a.dx = p->dx; a.gamma = p->gamma; a.lim = p->lim;
+    a.c = p->ctrl;
+    a.steps = steps; a.max_steps = max_steps; a.step0 = step0;
+    const int NC = p->loop_ctas;
+    const int per = (p->ncells + NC - 1) / NC;  // cells per CTA
+    const int threads = std::min(LOOP_THREADS, (per + 31) / 32 * 32);
+    if (NC == 1) {
+        k_pipe_loop<false><<<1, threads, 0, st>>>(a);
+        return cudaGetLastError();
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(NC, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = NC;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_pipe_loop<true>, a);
+}
+
+// CTAs of the one-launch form for a 1D pipeline: one for the smallest, else a
+// cluster of 16 (or the 8 every device places), 0 where the cells do not fit.
+int loop_ctas_for(int ncells) {
+    if (ncells <= LOOP_ONE_CTA) return 1;
+    for (int NC : {16, 8}) {
+        if (ncells > NC * LOOP_THREADS * LOOP_K) continue;
+        if (NC > 8 &&
+            cudaFuncSetAttribute(k_pipe_loop<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(NC, 1, 1);
+        cfg.blockDim = dim3(LOOP_THREADS, 1, 1);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = NC;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, k_pipe_loop<true>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        if (clusters >= 1) return NC;
+    }
+    return 0;
+}
+
 cudaError_t launch_all(nest_pipeline* p, void* state, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     for (const Stage& s : p->stages)
@@ -301,6 +612,7 @@ nest_status pcheck(const nest_pipeline* p) {
 }
 
 }  // namespace
+}  // namespace nestb
 
 extern "C" {
 
@@ -333,8 +645,18 @@ nest_status nest_pipeline_create(int dim, int nx, int ny, int npx, int npy, int 
         pi.ext1 = dim == 2 ? pi.n1 + 2 * halo : 1;
         p->patches.push_back(pi);
         p->max_n0 = std::max(p->max_n0, pi.n0);
+        p->ncells += dim == 1 ? pi.n0 : 0;
     }
     cudaError_t e;
+    if (dim == 1 && p->ncells <= 16 * LOOP_THREADS * LOOP_K && (p->loop_ctas = loop_ctas_for(p->ncells)) > 0) {
+        std::vector<int2> pairs;
+        for (auto [d, src] : exchange_pairs_1d(p->plan)) pairs.push_back(make_int2((int)d, (int)src));
+        p->ncopies = (int)pairs.size();
+        if ((e = cudaMalloc(&p->dcopies, sizeof(int2) * pairs.size())) != cudaSuccess ||
+            (e = cudaMemcpy(p->dcopies, pairs.data(), sizeof(int2) * pairs.size(), cudaMemcpyHostToDevice)) !=
+                cudaSuccess)
+            return cleanup(cuda_fail(e, "exchange pairs"));
+    }
     if ((e = cudaMalloc(&p->dpatches, sizeof(PatchInfo) * p->npatch)) != cudaSuccess) return cleanup(cuda_fail(e, "cudaMalloc"));
     if ((e = cudaMemcpy(p->dpatches, p->patches.data(), sizeof(PatchInfo) * p->npatch, cudaMemcpyHostToDevice)) !=
         cudaSuccess)
@@ -364,6 +686,7 @@ nest_status nest_pipeline_destroy(nest_pipeline* p) {
     drop_pipe_graphs(p);
     for (double* b : p->work) cudaFree(b);
     cudaFree(p->dpatches);
+    cudaFree(p->dcopies);
     cudaFree(p->ctrl);
     if (p->host_ctrl) cudaFreeHost(p->host_ctrl);
     if (p->own) cudaStreamDestroy(p->own);
@@ -400,7 +723,7 @@ nest_status nest_pipeline_execute(nest_pipeline* p, void* d_state, void* stream)
     if (r != NEST_OK) return r;
     if (!d_state) return fail(NEST_ERR_INVALID, "null state");
     cudaStream_t st = stream ? (cudaStream_t)stream : p->own;
-    cudaError_t e = launch_all(p, d_state, st);
+    cudaError_t e = use_loop(p) ? launch_loop(p, d_state, 1, 0, 0, st) : launch_all(p, d_state, st);
     if (e != cudaSuccess) return cuda_fail(e, "pipeline stage launch");
     return NEST_OK;
 }
@@ -419,9 +742,15 @@ nest_status nest_pipeline_run(nest_pipeline* p, void* d_state, double t_final, i
     // t_final into the control block (the CFL stages read it)
     CK(cudaMemcpyAsync(&p->ctrl->t_final, &t_final, sizeof(double), cudaMemcpyHostToDevice, st));
     CK(cudaStreamSynchronize(st));
+    const bool loop = use_loop(p);
+    // executions per launch of the one-launch form (without a CLOCK stage no step
+    // is counted, and the loop below gives up after two batches)
+    bool has_clock = false;
+    for (auto& s : p->stages) has_clock |= s.kind == NEST_STAGE_CLOCK;
+    const int chunk = has_clock ? 512 * PIPE_GRAPH_STEPS : PIPE_GRAPH_STEPS;
     auto key = std::make_pair(d_state, st);
     auto it = p->graphs.find(key);
-    if (it == p->graphs.end()) {
+    if (!loop && it == p->graphs.end()) {
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = cudaSuccess;
@@ -440,7 +769,12 @@ nest_status nest_pipeline_run(nest_pipeline* p, void* d_state, double t_final, i
     }
     int last = -1;
     for (;;) {
-        CK(cudaGraphLaunch(it->second, st));
+        if (loop) {
+            cudaError_t e = launch_loop(p, d_state, chunk, max_steps, start, st);
+            if (e != cudaSuccess) { r = cuda_fail(e, "pipeline launch"); break; }
+        } else {
+            CK(cudaGraphLaunch(it->second, st));
+        }
         if ((r = read_pipe_ctrl(p, st)) != NEST_OK) break;
         const PipeCtrl& c = *p->host_ctrl;
         if (!(c.time < t_final) || !c.active) break;

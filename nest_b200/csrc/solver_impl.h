@@ -7,6 +7,8 @@
 #include <map>
 #include <string>
 #include <tuple>
+#include <utility>
+#include <vector>
 
 #include "../../include/nest_b200.h"
 #include "common.cuh"
@@ -90,6 +92,7 @@ struct nest_solver {
 };
 
 namespace nestb {
+std::vector<std::pair<long long, long long>> exchange_pairs_1d(const nest_exchange* x);
 namespace rt {
 // Ghost fill + wave-speed maxima of the solver's current state.
 nest_status prepare(nest_solver* s);
