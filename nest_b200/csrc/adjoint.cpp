@@ -159,7 +159,7 @@ struct nest_adjoint {
     void* tmp = nullptr;
     double* d_dts = nullptr;       // all dts (device), for the adjoint kernels of the binomial schedule
     double* seg_dts = nullptr;     // dts of the current segment (device), uniform schedule
-    double* h_seg_dts = nullptr;   // pinned staging for seg_dts
+    void* arena = nullptr;         // one device allocation that holds all of the above
     std::map<int, cudaGraphExec_t> seg_graphs;  // uniform: one graph per segment length
     bool forward_done = false;
     double fwd_ms = 0.0, bwd_ms = 0.0;
@@ -168,13 +168,6 @@ struct nest_adjoint {
 };
 
 namespace {
-
-nest_status adj_alloc(nest_adjoint* a, void** p) {
-    CK(cudaMalloc(p, a->s->state_bytes()));
-    CK(cudaMemsetAsync(*p, 0, a->s->state_bytes(), a->s->st));
-    a->snap_bytes += (long long)a->s->state_bytes();
-    return NEST_OK;
-}
 
 nest_status copy_state_dev(nest_adjoint* a, void* dst, const void* src) {
     CK(cudaMemcpyAsync(dst, src, a->s->state_bytes(), cudaMemcpyDeviceToDevice, a->s->st));
@@ -320,49 +313,44 @@ nest_status nest_adjoint_create(nest_solver* s, int nsteps, int policy, int para
     a->policy = policy;
     a->param = policy == NEST_CKPT_UNIFORM ? std::min(param, nsteps) : std::min(param, nsteps);
     auto cleanup = [&](nest_status st) { nest_adjoint_destroy(a); return st; };
-    cudaError_t e = cudaMalloc(&a->ctrl, sizeof(StepCtrl));
-    if (e != cudaSuccess) return cleanup(cuda_fail(e, "cudaMalloc(ctrl)"));
-    if ((e = cudaMemset(a->ctrl, 0, sizeof(StepCtrl))) != cudaSuccess) return cleanup(cuda_fail(e, "memset"));
-    if (s->d.dim == 1) a->stepper.reset(new Stepper1D(s, a->ctrl));
-    else a->stepper.reset(new Stepper2D(s, a->ctrl));
-    nest_status st;
     int nslots = policy == NEST_CKPT_UNIFORM ? (nsteps + a->param - 1) / a->param : a->param;
     a->slots.assign(nslots, nullptr);
     a->slot_pos.assign(nslots + 1, -1);
-    for (auto& p : a->slots)
-        if ((st = adj_alloc(a, &p)) != NEST_OK) return cleanup(st);
     if (policy == NEST_CKPT_UNIFORM) {
         a->seg_un.assign(a->param, nullptr);
         a->seg_u1.assign(a->param, nullptr);
-        for (int i = 0; i < a->param; ++i) {
-            if ((st = adj_alloc(a, &a->seg_un[i])) != NEST_OK) return cleanup(st);
-            if ((st = adj_alloc(a, &a->seg_u1[i])) != NEST_OK) return cleanup(st);
-        }
     }
-    for (void** p : {&a->work, &a->u1, &a->lam[0], &a->lam[1], &a->tmp})
-        if ((st = adj_alloc(a, p)) != NEST_OK) return cleanup(st);
-    if ((e = cudaMalloc(&a->d_dts, sizeof(double) * nsteps)) != cudaSuccess) return cleanup(cuda_fail(e, "cudaMalloc(dts)"));
-    if ((e = cudaMalloc(&a->seg_dts, sizeof(double) * a->param)) != cudaSuccess)
-        return cleanup(cuda_fail(e, "cudaMalloc(seg dts)"));
-    if ((e = cudaMallocHost(&a->h_seg_dts, sizeof(double) * a->param)) != cudaSuccess)
-        return cleanup(cuda_fail(e, "cudaMallocHost"));
+    std::vector<void**> states;
+    for (auto& p : a->slots) states.push_back(&p);
+    for (auto& p : a->seg_un) states.push_back(&p);
+    for (auto& p : a->seg_u1) states.push_back(&p);
+    for (void** p : {&a->work, &a->u1, &a->lam[0], &a->lam[1], &a->tmp}) states.push_back(p);
+    a->snap_bytes = (long long)states.size() * (long long)s->state_bytes();
+    Arena ar;
+    std::vector<size_t> at;
+    for (size_t i = 0; i < states.size(); ++i) at.push_back(ar.add(s->state_bytes()));
+    const size_t oC = ar.add(sizeof(StepCtrl)), oD = ar.add(sizeof(double) * nsteps),
+                 oS = ar.add(sizeof(double) * a->param);
+    cudaError_t e = cudaMalloc(&a->arena, ar.bytes);
+    if (e != cudaSuccess) return cleanup(cuda_fail(e, "cudaMalloc(adjoint)"));
+    if ((e = cudaMemsetAsync(a->arena, 0, ar.bytes, s->st)) != cudaSuccess) return cleanup(cuda_fail(e, "memset"));
+    char* const base = (char*)a->arena;
+    for (size_t i = 0; i < states.size(); ++i) *states[i] = base + at[i];
+    a->ctrl = (StepCtrl*)(base + oC);
+    a->d_dts = (double*)(base + oD);
+    a->seg_dts = (double*)(base + oS);
+    if (s->d.dim == 1) a->stepper.reset(new Stepper1D(s, a->ctrl));
+    else a->stepper.reset(new Stepper2D(s, a->ctrl));
     *out = a;
     return NEST_OK;
 }
 
 nest_status nest_adjoint_destroy(nest_adjoint* a) {
     // Does not touch the solver (it may already be destroyed); cudaFree waits
-    // for outstanding work on these buffers.
+    // for outstanding work on the buffers.
     if (!a) return NEST_OK;
-    for (void* p : a->slots) cudaFree(p);
-    for (void* p : a->seg_un) cudaFree(p);
-    for (void* p : a->seg_u1) cudaFree(p);
-    for (void* p : {a->work, a->u1, a->lam[0], a->lam[1], a->tmp}) cudaFree(p);
     for (auto& kv : a->seg_graphs) cudaGraphExecDestroy(kv.second);
-    cudaFree(a->d_dts);
-    cudaFree(a->seg_dts);
-    if (a->h_seg_dts) cudaFreeHost(a->h_seg_dts);
-    cudaFree(a->ctrl);
+    cudaFree(a->arena);
     delete a;
     return NEST_OK;
 }
@@ -426,12 +414,9 @@ nest_status nest_adjoint_backward(nest_adjoint* a, const void* lam_final, void* 
             int j0 = g * K, L = std::min(a->nsteps, j0 + K) - j0;
             cudaGraphExec_t ge;
             if ((st = segment_graph(a, L, &ge)) != NEST_OK) return st;
-            for (int r = 0; r < L; ++r) a->h_seg_dts[r] = a->dts[j0 + r];
-            CK(cudaMemcpyAsync(a->seg_dts, a->h_seg_dts, sizeof(double) * L, cudaMemcpyHostToDevice, s->st));
+            CK(cudaMemcpyAsync(a->seg_dts, a->d_dts + j0, sizeof(double) * L, cudaMemcpyDeviceToDevice, s->st));
             if ((st = copy_state_dev(a, a->seg_un[0], a->slots[g])) != NEST_OK) return st;
             CK(cudaGraphLaunch(ge, s->st));
-            // the staging buffer is reused by the next segment
-            CK(cudaStreamSynchronize(s->st));
             a->advanced += L - 1;
         }
     } else {

@@ -65,6 +65,10 @@ std::string nestb::ctrl_error_text(const StepCtrl& c, int steps_now) {
 
 namespace {
 
+__global__ void k_set_clock(StepCtrl* c, double time, int steps) {
+    for (int p = 0; p < 2; ++p) { c->time[p] = time; c->step[p] = steps; }
+}
+
 nest_status drop_graphs(nest_solver* s) {
     for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
     s->graphs.clear();
@@ -158,6 +162,10 @@ nest_status enqueue_steps(nest_solver* s, int nsteps, const LoopParams& lp) {
                        lp.dts_out, lp.dts_cap, s->tx, s->warps};
             auto it = s->graphs.find(k);
             if (it == s->graphs.end()) {
+                if (s->graphs.size() >= MAX_GRAPHS) {
+                    CK(cudaStreamSynchronize(s->st));
+                    drop_graphs(s);
+                }
                 cudaGraph_t g;
                 CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
                 int p = s->parity;
@@ -359,27 +367,28 @@ nest_status nest_solver_create(const nest_solver_desc* d, nest_solver** out) {
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "cudaStreamCreate"));
         s->own_stream = true;
     }
-    size_t bytes = s->state_bytes();
-    if ((e = cudaMalloc(&s->U, bytes)) != cudaSuccess) return cleanup(cuda_fail(e, "cudaMalloc(U)"));
-    if ((e = cudaMalloc(&s->U1, bytes)) != cudaSuccess) return cleanup(cuda_fail(e, "cudaMalloc(U1)"));
-    if ((e = cudaMalloc(&s->ctrl, sizeof(StepCtrl))) != cudaSuccess) return cleanup(cuda_fail(e, "cudaMalloc(ctrl)"));
-    if ((e = cudaMallocHost(&s->host_ctrl, sizeof(StepCtrl))) != cudaSuccess) return cleanup(cuda_fail(e, "cudaMallocHost"));
-    if ((e = cudaMemsetAsync(s->U, 0, bytes, s->st)) != cudaSuccess) return cleanup(cuda_fail(e, "memset"));
-    if ((e = cudaMemsetAsync(s->U1, 0, bytes, s->st)) != cudaSuccess) return cleanup(cuda_fail(e, "memset"));
-    if ((e = cudaMemsetAsync(s->ctrl, 0, sizeof(StepCtrl), s->st)) != cudaSuccess) return cleanup(cuda_fail(e, "memset"));
-    if (d->dim == 2 && (d->flags & NEST_FLAG_TOTALS)) {
+    const bool totals = d->dim == 2 && (d->flags & NEST_FLAG_TOTALS);
+    if (totals) {
         long long nstrips = (d->ny + STRIP - 1) / STRIP;
         // sized for the default tile height and the smallest one the tiling
         // hook accepts (8 rows)
         const int rows = std::min(8, s->tx);
         s->nrec = nstrips * ((d->nx + rows - 1) / rows);
-        if ((e = cudaMalloc(&s->partials, sizeof(double) * 4 * s->nrec)) != cudaSuccess)
-            return cleanup(cuda_fail(e, "cudaMalloc(partials)"));
-        if ((e = cudaMemsetAsync(s->partials, 0, sizeof(double) * 4 * s->nrec, s->st)) != cudaSuccess)
-            return cleanup(cuda_fail(e, "memset"));
-        if ((e = cudaMalloc(&s->totals_dev, sizeof(double) * 4)) != cudaSuccess)
-            return cleanup(cuda_fail(e, "cudaMalloc(totals)"));
     }
+    Arena ar;
+    const size_t oU = ar.add(s->state_bytes()), oU1 = ar.add(s->state_bytes()), oC = ar.add(sizeof(StepCtrl)),
+                 oP = ar.add(sizeof(double) * 4 * s->nrec), oT = ar.add(sizeof(double) * 4);
+    if ((e = cudaMalloc(&s->arena, ar.bytes)) != cudaSuccess) return cleanup(cuda_fail(e, "cudaMalloc(solver)"));
+    char* const base = (char*)s->arena;
+    s->U = base + oU;
+    s->U1 = base + oU1;
+    s->ctrl = (StepCtrl*)(base + oC);
+    if (totals) {
+        s->partials = (double*)(base + oP);
+        s->totals_dev = (double*)(base + oT);
+    }
+    if ((e = cudaMallocHost(&s->host_ctrl, sizeof(StepCtrl))) != cudaSuccess) return cleanup(cuda_fail(e, "cudaMallocHost"));
+    if ((e = cudaMemsetAsync(s->arena, 0, ar.bytes, s->st)) != cudaSuccess) return cleanup(cuda_fail(e, "memset"));
     if ((e = cudaStreamSynchronize(s->st)) != cudaSuccess) return cleanup(cuda_fail(e, "sync"));
     *out = s;
     return NEST_OK;
@@ -389,8 +398,8 @@ nest_status nest_solver_destroy(nest_solver* s) {
     if (!s) return NEST_OK;
     if (s->st) cudaStreamSynchronize(s->st);
     drop_graphs(s);
-    cudaFree(s->U); cudaFree(s->U1); cudaFree(s->ctrl); cudaFree(s->partials); cudaFree(s->totals_dev);
-    cudaFree(s->dts_in); cudaFree(s->dts_out);
+    cudaFree(s->arena);
+    cudaFree(s->dts_buf);
     if (s->host_ctrl) cudaFreeHost(s->host_ctrl);
     if (s->own_stream && s->st) cudaStreamDestroy(s->st);
     delete s;
@@ -559,12 +568,8 @@ nest_status nest_solver_set_time(nest_solver* s, double time, int steps) {
     nest_status r = check(s);
     if (r != NEST_OK) return r;
     if (!(time >= 0.0) || steps < 0) return fail(NEST_ERR_INVALID, "time and step count must be non-negative");
-    CK(cudaStreamSynchronize(s->st));
-    CK(cudaMemcpyAsync(s->host_ctrl, s->ctrl, sizeof(StepCtrl), cudaMemcpyDeviceToHost, s->st));
-    CK(cudaStreamSynchronize(s->st));
-    for (int p = 0; p < 2; ++p) { s->host_ctrl->time[p] = time; s->host_ctrl->step[p] = steps; }
-    CK(cudaMemcpyAsync(s->ctrl, s->host_ctrl, sizeof(StepCtrl), cudaMemcpyHostToDevice, s->st));
-    CK(cudaStreamSynchronize(s->st));
+    k_set_clock<<<1, 1, 0, s->st>>>(s->ctrl, time, steps);
+    CK(cudaGetLastError());
     return NEST_OK;
 }
 
@@ -608,23 +613,31 @@ nest_status nest_solver_set_tiling(nest_solver* s, int rows_per_tile, int warps_
 nest_status nest_solver_set_dt_sequence(nest_solver* s, const double* dts, int n, int mode) {
     nest_status r = check(s);
     if (r != NEST_OK) return r;
-    CK(cudaStreamSynchronize(s->st));
-    drop_graphs(s);
-    cudaFree(s->dts_in); s->dts_in = nullptr;
-    cudaFree(s->dts_out); s->dts_out = nullptr;
+    slab_release(s);  // the slab driver's graphs do not tell dt sequences apart
+    s->dts_in = s->dts_out = nullptr;
     s->dts_cap = 0;
     s->dts_mode = 2;
     if (mode == 2) return NEST_OK;
     if (n <= 0) return fail(NEST_ERR_INVALID, "sequence length must be positive");
+    if (mode != 0 && mode != 1) return fail(NEST_ERR_INVALID, "mode must be 0, 1 or 2");
+    if (mode == 0 && !dts) return fail(NEST_ERR_INVALID, "null dt sequence");
+    CK(cudaStreamSynchronize(s->st));
+    if (n > s->dts_alloc) {
+        // the buffer moves: graphs that hold its address go (the others are
+        // told apart by it, its use and its length)
+        drop_graphs(s);
+        cudaFree(s->dts_buf);
+        s->dts_buf = nullptr;
+        s->dts_alloc = 0;
+        CK(cudaMalloc(&s->dts_buf, sizeof(double) * n));
+        s->dts_alloc = n;
+    }
     if (mode == 0) {
-        if (!dts) return fail(NEST_ERR_INVALID, "null dt sequence");
-        CK(cudaMalloc(&s->dts_in, sizeof(double) * n));
-        CK(cudaMemcpy(s->dts_in, dts, sizeof(double) * n, cudaMemcpyHostToDevice));
-    } else if (mode == 1) {
-        CK(cudaMalloc(&s->dts_out, sizeof(double) * n));
-        CK(cudaMemset(s->dts_out, 0, sizeof(double) * n));
+        CK(cudaMemcpy(s->dts_buf, dts, sizeof(double) * n, cudaMemcpyHostToDevice));
+        s->dts_in = s->dts_buf;
     } else {
-        return fail(NEST_ERR_INVALID, "mode must be 0, 1 or 2");
+        CK(cudaMemsetAsync(s->dts_buf, 0, sizeof(double) * n, s->st));
+        s->dts_out = s->dts_buf;
     }
     s->dts_cap = n;
     s->dts_mode = mode;

@@ -30,6 +30,18 @@ nest_status cuda_fail(cudaError_t e, const char* what);
 double bits_to_double(unsigned long long b);
 
 constexpr int GRAPH_STEPS = 16;  // steps per captured graph (even: parity-neutral)
+constexpr size_t MAX_GRAPHS = 64;  // captured graphs kept per solver
+
+// Parts of one device allocation, each on a 256-byte boundary.  (A cudaMalloc or
+// cudaFree of a few megabytes takes about 0.3 ms each, a small one 3 us.)
+struct Arena {
+    size_t bytes = 0;
+    size_t add(size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    }
+};
 
 struct GraphKey {
     int nsteps, parity;
@@ -56,6 +68,7 @@ struct nest_solver {
     long long vstride = 0;     // elements per variable plane
     int nvars = 3;
     size_t esize = 8;
+    void* arena = nullptr;     // one device allocation: U, U1, ctrl, partials, totals_dev
     void* U = nullptr;
     void* U1 = nullptr;
     nestb::StepCtrl* ctrl = nullptr;
@@ -63,6 +76,8 @@ struct nest_solver {
     double* partials = nullptr;
     long long nrec = 0;
     double* totals_dev = nullptr;
+    double* dts_buf = nullptr;   // device dt sequence (kept and grown), in use as one of:
+    int dts_alloc = 0;           // its capacity
     double* dts_in = nullptr;
     double* dts_out = nullptr;
     int dts_cap = 0;
