@@ -206,6 +206,8 @@ struct AdjX2Args {
 };
 
 __global__ void __maxnreg__(NEST_ADJX2_REGS) k2d_adjoint_x2(AdjX2Args A) {
+    pdl_wait();
+    pdl_trigger();
     const Geo2D& g = A.g;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int strip = blockIdx.x * AWARPS + warp;
@@ -475,8 +477,7 @@ cudaError_t launch_2d_adjoint_stage_f32x2(const float* U, const float* Lout, con
     if (seg_rows < 2) seg_rows = 2;
     segs = (g.nx + seg_rows - 1) / seg_rows;
     AdjX2Args a{ U, Lout, Extra, Lin, g, dtp, (float)alpha, (float)beta, seg_rows };
-    k2d_adjoint_x2<<<dim3(cx, segs), 32 * AWARPS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(k2d_adjoint_x2, dim3(cx, segs), dim3(32 * AWARPS), smem, st, a);
 }
 
 }  // namespace nestb

@@ -148,6 +148,8 @@ struct AdjD64Args {
 #define NEST_ADJ64_ATTR __launch_bounds__(32 * DWARPS)
 #endif
 __global__ void NEST_ADJ64_ATTR k2d_adjoint_rm64(AdjD64Args A) {
+    pdl_wait();
+    pdl_trigger();
     const Geo2D& g = A.g;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int strip = blockIdx.x * DWARPS + warp;
@@ -413,8 +415,7 @@ cudaError_t launch_2d_adjoint_stage_f64rm(const double* U, const double* Lout, c
     if (seg_rows < 2) seg_rows = 2;
     segs = (g.nx + seg_rows - 1) / seg_rows;
     AdjD64Args a{ U, Lout, Extra, Lin, g, dtp, alpha, beta, seg_rows };
-    k2d_adjoint_rm64<<<dim3(cx, segs), 32 * DWARPS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(k2d_adjoint_rm64, dim3(cx, segs), dim3(32 * DWARPS), smem, st, a);
 }
 
 }  // namespace nestb

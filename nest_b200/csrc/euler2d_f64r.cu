@@ -143,25 +143,6 @@ __device__ __forceinline__ void f64r_body(const Args& a, int strip, int tile_row
     const double gamma = g.gamma;
     const double gm1 = g.gamma - 1.0;
 
-    double dt;
-    if (STAGE == 1) {
-        bool done = step_is_done(a.ctrl, a.p, a.lp);
-        double pd = done ? -1.0 : prescribed_dt(a.ctrl, a.p, a.lp);
-        if (pd > 0.0) {
-            dt = pd;
-        } else {
-            dt = dt_from_speeds(bits_speed(a.ctrl->maxs[a.p][0]), bits_speed(a.ctrl->maxs[a.p][1]),
-                                g.dx, g.dy, a.lp.cfl);
-            if (a.lp.t_final > 0.0) dt = smin(dt, a.lp.t_final - a.ctrl->time[a.p]);
-        }
-        if (strip == 0 && tile_row == 0 && lane == 0) publish_step(a.ctrl, a.p, a.lp, done, dt);
-        if (done) return;
-    } else {
-        if (!a.ctrl->active[a.p]) return;
-        dt = a.ctrl->dt[a.p];
-    }
-    const double dtdx = dt / g.dx;
-    const double dtdy = dt / g.dy;
     const int lim = LIM >= 0 ? LIM : a.lp.lim;
 
     const int nx = g.nx, ny = g.ny, pitch = g.pitch;
@@ -222,14 +203,21 @@ __device__ __forceinline__ void f64r_body(const Args& a, int strip, int tile_row
     // prologue: rows i0-2 .. i0+1, the x-flux of face i0-1/2 and the upper
     // x-face state of row i0
     W4 Wq, Wq1, Pq, Fm;
+    double dtdx, dtdy;
     {
         const W4 c0 = load(i0 - 2), c1 = load(i0 - 1);
         for (int r = 0; r < LOOKD; ++r) stage_row(i0 + r);
         if (STAGE == 2)
             for (int r = 0; r < LOOKD - 2; ++r) stage_un(i0 + r);
         cpd_commit();
+        // the step's dt while the first rows are on their way
+        double dt;
+        const bool run = stage_dt<STAGE>(a, strip == 0 && tile_row == 0 && lane == 0, dt);
         cpd_wait<0>();
         __syncwarp();
+        if (!run) return;
+        dtdx = div_rn(dt, g.dx);
+        dtdy = div_rn(dt, g.dy);
         auto pro = [&](auto& m, auto& mp, const auto& ig) {
             const W4 Wa = prim_d(mp, c0, gm1), Wb = prim_d(mp, c1, gm1);
             Wq = prim_d(mp, ring_row(i0), gm1);
@@ -353,8 +341,8 @@ __device__ __forceinline__ void f64r_body(const Args& a, int strip, int tile_row
     cpd_wait<0>();
     __syncwarp();
     if (STAGE == 2) {
-        smx = warp_max(smx);
-        smy = warp_max(smy);
+        smx = warp_max_speed(smx);
+        smy = warp_max_speed(smy);
         if (lane == 0) {
             if (!(smx == smx) || !(smy == smy) || smx > 1.79e308 || smy > 1.79e308)
                 atomicOr(&a.ctrl->err, ERRW_NONFINITE);
@@ -383,12 +371,16 @@ __device__ __forceinline__ void f64r_body(const Args& a, int strip, int tile_row
 // quotients tested one by one by an exact residual and the IEEE square root the
 // step took 2.090 ms, 1000 steps of the 2048^2 periodic Kelvin-Helmholtz state
 // 576 -> 349 ms.  Tile rows now: 16 1.286, 24 1.261, 32 1.265, 48 1.283.
+// Dependent launch, and dt worked out while the first rows are on their way:
+// 4096^2 1.256 -> 1.229, 2048^2 Kelvin-Helmholtz 0.348 -> 0.339, 256 x 192 25.5 -> 22.9 us.
 #ifndef NEST_F64R_REGS
 #define NEST_F64R_REGS 168
 #endif
 
 template <int STAGE, bool TOT, int LIM>
 __global__ void __maxnreg__(NEST_F64R_REGS) k2d_f64r(StageArgs<double> a) {
+    pdl_wait();
+    pdl_trigger();
     f64r_body<STAGE, TOT, LIM>(a, blockIdx.x * blockDim.y + threadIdx.y, blockIdx.y);
 }
 
@@ -414,6 +406,8 @@ struct F64View {
 // 190 (258), 64 of 48..320 312 (508).
 template <int STAGE, bool TOT>
 __global__ void __maxnreg__(NEST_F64R_REGS) kbatch_f64(BatchArgs<double> b) {
+    pdl_wait();
+    pdl_trigger();
     const int nw = gridDim.x * blockDim.y;
     for (int it = blockIdx.x * blockDim.y + threadIdx.y; it < b.nitems; it += nw) {
         const int4 w = b.items[it];
@@ -426,13 +420,13 @@ __global__ void __maxnreg__(NEST_F64R_REGS) kbatch_f64(BatchArgs<double> b) {
 }
 
 template <int LIM>
-void launch_f64r_lim(const StageArgs<double>& a1, const StageArgs<double>& a2, dim3 gr, dim3 b, size_t sm1,
-                     size_t sm2, int which, bool tot, cudaStream_t st) {
-    if (which & 1) k2d_f64r<1, false, LIM><<<gr, b, sm1, st>>>(a1);
-    if (which & 2) {
-        if (tot) k2d_f64r<2, true, LIM><<<gr, b, sm2, st>>>(a2);
-        else k2d_f64r<2, false, LIM><<<gr, b, sm2, st>>>(a2);
-    }
+cudaError_t launch_f64r_lim(const StageArgs<double>& a1, const StageArgs<double>& a2, dim3 gr, dim3 b, size_t sm1,
+                            size_t sm2, int which, bool tot, cudaStream_t st) {
+    cudaError_t e = cudaSuccess;
+    if (which & 1) e = launch_pdl(k2d_f64r<1, false, LIM>, gr, b, sm1, st, a1);
+    if ((which & 2) && e == cudaSuccess)
+        e = launch_pdl(tot ? k2d_f64r<2, true, LIM> : k2d_f64r<2, false, LIM>, gr, b, sm2, st, a2);
+    return e;
 }
 
 size_t f64r_ring_bytes(int stage, int warps) { return (size_t)warps * ring_d_per_warp(stage) * sizeof(double); }
@@ -447,20 +441,18 @@ cudaError_t launch_2d_step_f64r(double* U, double* U1, const Geo2D& g, const Loo
     StageArgs<double> a1{U, nullptr, U1, g, lp, ctrl, nullptr, p, tx};
     StageArgs<double> a2{U1, U, Uout ? Uout : U, g, lp, ctrl, partials, p, tx};
     const size_t sm1 = f64r_ring_bytes(1, warps), sm2 = f64r_ring_bytes(2, warps);
-    if (lp.lim == LIM_MINMOD) launch_f64r_lim<LIM_MINMOD>(a1, a2, gr, b, sm1, sm2, which, partials != nullptr, st);
-    else launch_f64r_lim<-1>(a1, a2, gr, b, sm1, sm2, which, partials != nullptr, st);
-    return cudaGetLastError();
+    return lp.lim == LIM_MINMOD ? launch_f64r_lim<LIM_MINMOD>(a1, a2, gr, b, sm1, sm2, which, partials != nullptr, st)
+                                : launch_f64r_lim<-1>(a1, a2, gr, b, sm1, sm2, which, partials != nullptr, st);
 }
 
 cudaError_t launch_batch_f64(const BatchArgs<double>& b, int which, int blocks, int warps, cudaStream_t st) {
     const dim3 blk(32, warps);
     const size_t sm1 = f64r_ring_bytes(1, warps), sm2 = f64r_ring_bytes(2, warps);
-    if (which & 1) kbatch_f64<1, false><<<blocks, blk, sm1, st>>>(b);
-    if (which & 2) {
-        if (b.partials) kbatch_f64<2, true><<<blocks, blk, sm2, st>>>(b);
-        else kbatch_f64<2, false><<<blocks, blk, sm2, st>>>(b);
-    }
-    return cudaGetLastError();
+    cudaError_t e = cudaSuccess;
+    if (which & 1) e = launch_pdl(kbatch_f64<1, false>, dim3(blocks), blk, sm1, st, b);
+    if ((which & 2) && e == cudaSuccess)
+        e = launch_pdl(b.partials ? kbatch_f64<2, true> : kbatch_f64<2, false>, dim3(blocks), blk, sm2, st, b);
+    return e;
 }
 
 // Resident blocks per SM of the batched stages (6 KB of rings a warp: no

@@ -23,6 +23,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "f64div.cuh"
 
 namespace nestb {
 
@@ -175,8 +176,8 @@ __device__ __forceinline__ void cell_speeds(T U0, T U1, T U2, T U3, T gamma, T g
 // dt = cfl * min(dx / max(|u|+c), dy / max(|v|+c)), euler2d.hpp:249-270.
 __device__ __forceinline__ double dt_from_speeds(double sx, double sy, double dx, double dy, double cfl) {
     double dtx = 1e10, dty = 1e10;
-    if (sx > 0.0) dtx = smin(dtx, dx / sx);
-    if (sy > 0.0) dty = smin(dty, dy / sy);
+    if (sx > 0.0) dtx = smin(dtx, div_rn(dx, sx));
+    if (sy > 0.0) dty = smin(dty, div_rn(dy, sy));
     return cfl * smin(dtx, dty);
 }
 
@@ -235,6 +236,26 @@ struct StageArgs {
     int p;                      // step parity
     int tx;                     // rows per tile
 };
+
+// dt of the step, published by stage 1's `lead` thread; false: nothing to do.
+template <int STAGE, class A>
+__device__ __forceinline__ bool stage_dt(const A& a, bool lead, double& dt) {
+    if (STAGE == 1) {
+        const bool done = step_is_done(a.ctrl, a.p, a.lp);
+        const double pd = done ? -1.0 : prescribed_dt(a.ctrl, a.p, a.lp);
+        if (pd > 0.0) {
+            dt = pd;
+        } else {
+            dt = dt_from_speeds(bits_speed(a.ctrl->maxs[a.p][0]), bits_speed(a.ctrl->maxs[a.p][1]),
+                                a.g.dx, a.g.dy, a.lp.cfl);
+            if (a.lp.t_final > 0.0) dt = smin(dt, a.lp.t_final - a.ctrl->time[a.p]);
+        }
+        if (lead) publish_step(a.ctrl, a.p, a.lp, done, dt);
+        return !done;
+    }
+    dt = a.ctrl->dt[a.p];
+    return a.ctrl->active[a.p] != 0;
+}
 
 // One stage.  STAGE 1: U1 = U + dt L(U).  STAGE 2: U = 0.5 (U + U1 + dt L(U1)),
 // plus the max wave speeds of the new state (next dt) and optional totals.
