@@ -67,12 +67,20 @@ __device__ __forceinline__ W4 face_dn(const A& m, const W4& w, const W4& s) {
 
 // cons2prim, hlle4 and cell_speeds_p of euler2d_kernels.cuh for the FP64
 // plain form (the same expressions in the same order, so the same values),
-// with their divisions and square roots taken from a policy.
+// with their divisions and square roots taken from a policy.  The checked policy
+// also takes the halves out of the kinetic energies: ((0.5 r) u) u is 0.5 ((r u) u)
+// and so on, exactly, unless a product is subnormal, and there it is far below
+// the rounding of the energy (at least 2^-130) it is added to.
+
+// (r u) u + (r v) v, twice ke2(r, u, v).
+__device__ __forceinline__ double twice_ke(double r, double u, double v) { return r * u * u + r * v * v; }
+
 template <class A>
 __device__ __forceinline__ W4 prim_d(A& m, const W4& c, double gm1) {
     const auto ir = m.recip(c.a);
     const double u = m.quot(c.b, ir), v = m.quot(c.c, ir);
-    const double p = smax(gm1 * (c.d - ke2(c.a, u, v)), 0.0);
+    // (a p that the clamp would change fails its test)
+    const double p = A::checked ? gm1 * fma(-0.5, twice_ke(c.a, u, v), c.d) : smax(gm1 * (c.d - ke2(c.a, u, v)), 0.0);
     m.pos(c.a); m.pos(p); m.num(c.b); m.num(c.c);
     return { c.a, u, v, p };
 }
@@ -84,8 +92,9 @@ __device__ __forceinline__ void hlle4_d(A& m, double gamma, const typename A::Re
                                         double& f1, double& f2, double& f3) {
     const double cL = m.root(m.quot(gamma * pL, m.recip(rL)));
     const double cR = m.root(m.quot(gamma * pR, m.recip(rR)));
-    const double EL = m.quot(pL, ig) + ke2(rL, nL, tL);
-    const double ER = m.quot(pR, ig) + ke2(rR, nR, tR);
+    // (r n) n, r t and (r t) t below are shared with the fluxes
+    const double EL = A::checked ? fma(0.5, twice_ke(rL, nL, tL), m.quot(pL, ig)) : m.quot(pL, ig) + ke2(rL, nL, tL);
+    const double ER = A::checked ? fma(0.5, twice_ke(rR, nR, tR), m.quot(pR, ig)) : m.quot(pR, ig) + ke2(rR, nR, tR);
     const double SL = smin(nL - cL, nR - cR);
     const double SR = smax(nL + cL, nR + cR);
     const double mL = rL * nL, mR = rR * nR;
@@ -99,7 +108,8 @@ __device__ __forceinline__ void hlle4_d(A& m, double gamma, const typename A::Re
         const double a0 = SR * FL0 - SL * FR0 + SLR * (rR - rL), a1 = SR * FL1 - SL * FR1 + SLR * (mR - mL);
         const double a2 = SR * FL2 - SL * FR2 + SLR * (rR * tR - rL * tL), a3 = SR * FL3 - SL * FR3 + SLR * (ER - EL);
         m.num(a0); m.num(a2); m.num(a3);
-        const bool l = SL >= 0.0, r = SR <= 0.0;
+        // SL >= 0 and SR <= 0 from the bits (c > 0, so neither is -0)
+        const bool l = __double2hiint(SL) >= 0, r = __double_as_longlong(SR) <= 0;
         f0 = l ? FL0 : r ? FR0 : m.quot(a0, id);
         f1 = l ? FL1 : r ? FR1 : m.quot(a1, id);
         f2 = l ? FL2 : r ? FR2 : m.quot(a2, id);
@@ -124,13 +134,16 @@ __device__ __forceinline__ double speeds_d(A& m, double U0, double U1, double U2
     const double rho = smax(U0, 1e-10);
     const auto ir = m.recip(rho);
     const double u = m.quot(U1, ir), v = m.quot(U2, ir);
-    const double ke = 0.5 * rho * (u * u + v * v);
-    const double p = smax(gm1 * (U3 - ke), 1e-10);
+    const double uv = u * u + v * v;
+    const double p = smax(gm1 * (A::checked ? fma(-0.5, rho * uv, U3) : U3 - 0.5 * rho * uv), 1e-10);
     const double c = m.root(m.quot(gamma * p, ir));
-    m.pos(rho); m.pos(p); m.num(U1); m.num(U2);
     sx = fabs(u) + c;
     sy = fabs(v) + c;
-    return gm1 * (U3 - ke2(rho, u, v));
+    // p is at least 1e-10, and at most a few pc where pc > 0; the test of pc also
+    // takes cells to be flagged and states that are not finite to the IEEE forms
+    const double pc = A::checked ? gm1 * fma(-0.5, twice_ke(rho, u, v), U3) : gm1 * (U3 - ke2(rho, u, v));
+    m.pos(rho); m.pos(pc); m.num(U1); m.num(U2);
+    return pc;
 }
 
 // LIM: the slope limiter fixed at compile time (LIM_MINMOD, nest's default),
@@ -373,6 +386,9 @@ __device__ __forceinline__ void f64r_body(const Args& a, int strip, int tile_row
 // 576 -> 349 ms.  Tile rows now: 16 1.286, 24 1.261, 32 1.265, 48 1.283.
 // Dependent launch, and dt worked out while the first rows are on their way:
 // 4096^2 1.256 -> 1.229, 2048^2 Kelvin-Helmholtz 0.348 -> 0.339, 256 x 192 25.5 -> 22.9 us.
+// Halves of the kinetic energies fused, Goldschmidt's square root, regimes and
+// numerator tests from integer words: 4096^2 1.233 -> 1.164, 2048^2 Kelvin-
+// Helmholtz 0.339 -> 0.322 (then: budget 160 1.176, 176 1.166).
 #ifndef NEST_F64R_REGS
 #define NEST_F64R_REGS 168
 #endif
@@ -403,7 +419,7 @@ struct F64View {
 // grid's warp count as stride (one item each by default).
 // Us per step with TOTALS, against the register-window march with IEEE
 // divisions in 32-row items: 4 problems of 64..128 a side 24 (216), 48 of 64..256
-// 190 (258), 64 of 48..320 312 (508).
+// 182 (258), 64 of 48..320 312 (508; before the fused halves).
 template <int STAGE, bool TOT>
 __global__ void __maxnreg__(NEST_F64R_REGS) kbatch_f64(BatchArgs<double> b) {
     pdl_wait();

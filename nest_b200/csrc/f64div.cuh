@@ -33,11 +33,12 @@
 //     RN(a / b).
 //   * r = b q0 - a rather than a - b q0 keeps the sign of a zero quotient:
 //     with b > 0, a = -0 gives r = +0 and q = q0 - 0 = -0.
-// Square root (Markstein, as above): h ~ 1 / (2 sqrt(x)) from the hardware
-// approximation (measured: |1 - x y0^2| < 2^-19.0) by two Newton-Raphson steps
-// h <- h + h (1/2 - 2 x h^2), with relative error |eta| < 1.6 2^-53 in the end,
-// and g ~ s = sqrt(x) from the first of them (2^-39), then twice
-// g <- g + (x - g^2) h.  The first leaves g within half an ulp (and a few
+// Square root (Markstein, as above, and Goldschmidt's iteration: P. Markstein,
+// "Software division and square root using Goldschmidt's algorithms", RNC6,
+// 2004): from the hardware approximation y0 (measured: |1 - x y0^2| < 2^-19.0)
+// g ~ s = sqrt(x) and h ~ 1 / (2 s) together, g <- g + g r, h <- h + h r with
+// r = 1/2 - g h (2^-39), then h once more, with relative error |eta| <= 2 2^-53,
+// then twice g <- g + (x - g^2) h.  The first leaves g within half an ulp (and a few
 // 2^-26 of one) of s; the second has an exact residual and rounds
 // s - d^2 / (2 s) + d eta (d = s - g).  With s in [1, 2), a midpoint m below s has
 // s - m >= 7 ulp^2 / (8 s) (in units of ulp^2 / 4, m^2 is 1 modulo 8 and x a
@@ -69,10 +70,10 @@ __device__ __forceinline__ double quot_f64(double a, double b, double y) {
 __device__ __forceinline__ double sqrt_f64(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double x2 = x + x;
-    double h = 0.5 * y;
-    h = fma(h, fma(-(x2 * h), h, 0.5), h);
-    double g = x2 * h;
+    double h = 0.5 * y, g = x * y;
+    const double r = fma(-g, h, 0.5);
+    h = fma(h, r, h);
+    g = fma(g, r, g);
     h = fma(h, fma(-g, h, 0.5), h);
     g = fma(fma(-g, g, x), h, g);
     return fma(fma(-g, g, x), h, g);
@@ -90,7 +91,7 @@ __device__ __forceinline__ double sqrt_quot_f64(double a, double b, double& y) {
     double h;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(h) : "d"(t));
     h *= 0.5;
-    h = fma(h, fma(-(t2 * h), h, 0.5), h);
+    h = fma(h, fma(-(t2 * h), h, 0.5), h);  // 1 / (2 sqrt(q)) to 2^-39
     y = fma(y, fma(-b, y, 1.0), y);
     y = fma(y, fma(-b, y, 1.0), y);
     const double q = quot_f64(a, b, y);
@@ -127,7 +128,9 @@ struct F64Range {
         all &= (unsigned)__double2hiint(x) + ((897u << 20) ^ 0x80000000u);
     }
     __device__ __forceinline__ void num(double a) {
-        const unsigned k = 2u * (unsigned)__double2hiint(a) + (__double2loint(a) != 0 ? 1u : 0u) - 1u;
+        unsigned k;  // 2 hi + (lo != 0) - 1: the first addition carries where lo != 0
+        asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %1, 0xffffffff;\n\taddc.u32 %0, %2, 0xffffffff;\n\t}"
+            : "=r"(k) : "r"(__double2loint(a)), "r"(2u * (unsigned)__double2hiint(a)));
         low = min(low, k);
     }
     __device__ __forceinline__ bool ok() const { return all >= 0xf0000000u && low >= (223u << 21); }
