@@ -138,32 +138,6 @@ constexpr int STEP_WARPS = 4;  // warps per CTA of k1d_step
 // output cells of a warp with CPL cells per lane: all but four at each end
 __host__ __device__ constexpr int step_cells(int cpl) { return 32 * cpl - 8; }
 
-// Stage fluxes of a warp whose lanes hold the primitives w of CPL neighbouring
-// cells each: f[i] is the face to the right of the lane's cell i, in the
-// expressions of plm_flux (valid two cells inside the valid ones).
-template <typename T, int CPL>
-__device__ __forceinline__ void warp_flux(const Gas<T>& g, int lim, const T (&w)[CPL][3], F3<T> (&f)[CPL]) {
-    T P[CPL][3], M[CPL + 1][3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        T d[CPL];
-#pragma unroll
-        for (int i = 0; i < CPL; ++i)
-            d[i] = (i + 1 < CPL ? w[i + 1 < CPL ? i + 1 : 0][k] : __shfl_down_sync(0xffffffffu, w[0][k], 1)) - w[i][k];
-        const T dm = __shfl_up_sync(0xffffffffu, d[CPL - 1], 1);
-#pragma unroll
-        for (int i = 0; i < CPL; ++i) {
-            const T s = limit(i > 0 ? d[i > 0 ? i - 1 : 0] : dm, d[i], lim);
-            P[i][k] = w[i][k] + T(0.5) * s;
-            M[i][k] = w[i][k] - T(0.5) * s;
-        }
-        M[CPL][k] = __shfl_down_sync(0xffffffffu, M[0][k], 1);
-    }
-#pragma unroll
-    for (int i = 0; i < CPL; ++i)
-        f[i] = face_flux(g, P[i][0], P[i][1], P[i][2], M[i + 1][0], M[i + 1][1], M[i + 1][2]);
-}
-
 // v[i] = u[i] - dtdx (right flux - left flux) of the lane's cells.
 template <typename T, int CPL>
 __device__ __forceinline__ void warp_update(const T (&u)[CPL][3], const F3<T> (&f)[CPL], T dtdx, T (&v)[CPL][3]) {

@@ -213,10 +213,14 @@ struct Stage {
 
 constexpr int LOOP_STAGES = 32, LOOP_BUFFERS = 17;
 constexpr int LOOP_THREADS = 512, LOOP_K = 2;  // threads per CTA, cells per thread
-// Up to this many cells one CTA (cheap barriers), above a cluster of 16, whose six
-// barriers a step cost about 0.45 us each: us per step, one CTA / cluster, 400 cells
-// 10.1 / 14.2, 640 14.0 / 13.9, 1024 16.9 / 14.5.
-constexpr int LOOP_ONE_CTA = 640;
+constexpr size_t LOOP_SMEM = 160 << 10;        // most that the buffers of the one-CTA form take
+constexpr int LOOP_SLOT = 28;                  // cells of a warp that shares faces
+// One CTA (cheap barriers, buffers in shared memory) where its warps take the cells in
+// two slots each or where there are few, else a cluster of 16, whose six barriers a
+// step cost about 0.45 us each: us per step, one CTA / cluster, 100 cells in 2 patches
+// 4.6 / 11.4, 400 in 4 6.3 / 12.5, 800 in 5 (30 slots) 8.9 / 12.6, 900 in 8 (40, no slots)
+// 13.3 / 12.4.
+constexpr int LOOP_ONE_CTA = 640, LOOP_ONE_SLOTS = LOOP_K * LOOP_THREADS / 32;
 
 struct LoopArgs {
     int nstages;
@@ -229,6 +233,8 @@ struct LoopArgs {
     int ncopies;
     double dx, gamma;
     int lim;
+    int share;                    // a warp per LOOP_SLOT cells of a patch, faces shared by shuffles
+    int total, nbuf;              // elements of a buffer, buffers (SMEM)
     PipeCtrl* c;
     int steps;                    // executions of the stage list at most
     int max_steps, step0;         // > 0: stop at a multiple of 8 executions once step - step0 reaches it
@@ -243,12 +249,18 @@ struct LoopArgs {
 // the stage kernels above, with the branch-free division and square root.
 // An execution whose CFL stage finds the run finished is the last one (its halo
 // exchanges still run; further ones would change nothing).
+// share: a warp takes up to 28 neighbouring cells of a patch and a halo of two on each side,
+// and every primitive, slope and flux is computed once instead of by up to five cells.
+// SMEM (one CTA): the buffers live in shared memory for the launch.
 // Bound: the latency of the stages' chains and their barriers.  nest's sod1d step
 // (ten stages, twelve launches), us per step against a launch per stage: 100 cells
-// 7.0 (26), 400 10.1 (30), 1024 14.5 (31), 4000 14.6 (31), 16000 26 (38).
-template <bool CLUSTER>
+// 4.6 (26), 400 6.3 (30), 1024 12.7 (31), 4000 12.9 (31), 16000 25 (38); with every cell
+// computing both its faces and the buffers in global memory 100 cells 6.4, 400 9.8,
+// 1024 14.1, 4000 14.4.
+template <bool CLUSTER, bool SMEM>
 __global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
     namespace cg = cooperative_groups;
+    extern __shared__ double pipe_buf[];
     __shared__ double red[2][16 * (LOOP_THREADS / 32)];
     const int NC = CLUSTER ? (int)cg::this_cluster().num_blocks() : 1;
     const int rank = CLUSTER ? (int)cg::this_cluster().block_rank() : 0;
@@ -262,21 +274,40 @@ __global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
     const double gm1 = a.gamma - 1.0;
     PipeCtrl* const c = a.c;
 
-    // the thread's cells: element offset, plane stride, place in the patch
+    // the thread's cells: element offset, plane stride, place in the patch (patch -1:
+    // none; with shared faces a warp's lanes hold neighbouring cells, two of halo on each side, and
+    // e is the element that a lane reads as its cell)
     struct Own {
-        long long e;
-        int plane, patch, i, n0;
+        int e, plane, patch, i, n0;
     } own[LOOP_K];
 #pragma unroll
     for (int k = 0; k < LOOP_K; ++k) {
         own[k] = { 0, 0, -1, 0, 0 };
-        int f = gt + k * NT;
-        if (f < a.ncells) {
-            int p = 0;
-            while (f >= a.P[p].n0) f -= a.P[p++].n0;
-            own[k] = { a.P[p].off + a.h + f, a.P[p].ext0, p, f, a.P[p].n0 };
+        if (a.share) {
+            int f = (gt + k * NT) >> 5, p = 0;
+            while (p < a.npatch && f >= (a.P[p].n0 + LOOP_SLOT - 1) / LOOP_SLOT)
+                f -= (a.P[p++].n0 + LOOP_SLOT - 1) / LOOP_SLOT;
+            if (p < a.npatch) {
+                // one-sided at the patch edges: the cell two outside reads as the one outside
+                const int i = LOOP_SLOT * f - 2 + lane, n0 = a.P[p].n0;
+                own[k] = { (int)a.P[p].off + a.h + min(max(i, -1), n0), a.P[p].ext0,
+                           lane >= 2 && lane < 2 + LOOP_SLOT && i < n0 ? p : -1, i, n0 };
+            }
+        } else {
+            int f = gt + k * NT;
+            if (f < a.ncells) {
+                int p = 0;
+                while (f >= a.P[p].n0) f -= a.P[p++].n0;
+                own[k] = { (int)a.P[p].off + a.h + f, a.P[p].ext0, p, f, a.P[p].n0 };
+            }
         }
     }
+    if (SMEM) {
+        for (int b = 0; b < a.nbuf; ++b)
+            for (int q = threadIdx.x; q < a.total; q += T) pipe_buf[b * a.total + q] = a.buf[b][q];
+        __syncthreads();
+    }
+    auto buf = [&](int b) { return SMEM ? pipe_buf + b * a.total : a.buf[b]; };
     double time = c->time, dt = c->dt;
     int step = c->step, active = c->active;
     const double t_final = c->t_final;
@@ -290,14 +321,14 @@ __global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
         for (int s = 0; s < a.nstages; ++s) {
             const Stage& g = a.st[s];
             if ((a.sync_before >> s) & 1u) sync();
-            double* const src = a.buf[g.src];
-            double* const dst = a.buf[g.dst];
+            double* const src = buf(g.src);
+            double* const dst = buf(g.dst);
             if (g.kind == NEST_STAGE_CFL_DT) {
                 double ms = 0.0;
 #pragma unroll
                 for (int k = 0; k < LOOP_K; ++k)
                     if (own[k].patch >= 0) {
-                        const long long e = own[k].e;
+                        const int e = own[k].e;
                         const int pl = own[k].plane;
                         const Cell1<double> w = cell1d<true>(gas, src[e], src[e + pl], src[e + 2 * pl]);
                         ms = smax(ms, fabs(w.u) + w.cs);
@@ -331,16 +362,36 @@ __global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
             switch (g.kind) {
                 case NEST_STAGE_EULER_RHS: {
                     const double dtdx = div_rn(dt, a.dx);
+                    if (a.share) {
+#pragma unroll
+                        for (int k = 0; k < LOOP_K; ++k) {
+                            const int e = own[k].e, pl = own[k].plane;
+                            if (pl == 0) continue;  // the whole warp
+                            const double U[1][3] = { { src[e], src[e + pl], src[e + 2 * pl] } };
+                            const Cell1<double> q = cell1d<false>(gas, U[0][0], U[0][1], U[0][2]);
+                            const double W[1][3] = { { U[0][0], q.u, q.p } };
+                            F3<double> f[1];
+                            warp_flux(gas, a.lim, W, f);
+                            const double fa = __shfl_up_sync(0xffffffffu, f[0].a, 1);
+                            const double fb = __shfl_up_sync(0xffffffffu, f[0].b, 1);
+                            const double fc = __shfl_up_sync(0xffffffffu, f[0].c, 1);
+                            if (own[k].patch < 0) continue;
+                            dst[e] = U[0][0] - dtdx * (f[0].a - fa);
+                            dst[e + pl] = U[0][1] - dtdx * (f[0].b - fb);
+                            dst[e + 2 * pl] = U[0][2] - dtdx * (f[0].c - fc);
+                        }
+                        break;
+                    }
 #pragma unroll
                     for (int k = 0; k < LOOP_K; ++k) {
                         if (own[k].patch < 0) continue;
-                        const long long e = own[k].e;
+                        const int e = own[k].e;
                         const int pl = own[k].plane, i = own[k].i;
                         double U[3], W[5][3];  // cells i-2 .. i+2
 #pragma unroll
                         for (int q = 0; q < 5; ++q) {
                             // one-sided at the patch edges: i-2 -> i-1 on the first cell, i+2 -> i+1 on the last
-                            const long long x = e + (q == 0 && i == 0 ? -1 : q == 4 && i == own[k].n0 - 1 ? 1 : q - 2);
+                            const int x = e + (q == 0 && i == 0 ? -1 : q == 4 && i == own[k].n0 - 1 ? 1 : q - 2);
                             const double r = src[x], m = src[x + pl], E = src[x + 2 * pl];
                             const Cell1<double> w = cell1d<false>(gas, r, m, E);
                             W[q][0] = r; W[q][1] = w.u; W[q][2] = w.p;
@@ -360,12 +411,12 @@ __global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
                 }
                 case NEST_STAGE_COPY:
                 case NEST_STAGE_AVERAGE: {
-                    const double* const aux = a.buf[g.aux];
+                    const double* const aux = buf(g.aux);
 #pragma unroll
                     for (int k = 0; k < LOOP_K; ++k)
                         if (own[k].patch >= 0)
                             for (int v = 0; v < 3; ++v) {
-                                const long long e = own[k].e + (long long)v * own[k].plane;
+                                const int e = own[k].e + v * own[k].plane;
                                 dst[e] = g.kind == NEST_STAGE_COPY ? src[e] : 0.5 * src[e] + 0.5 * aux[e];
                             }
                     break;
@@ -395,6 +446,11 @@ __global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
         }
         if (finished) break;
     }
+    if (SMEM) {
+        __syncthreads();
+        for (int b = 0; b < a.nbuf; ++b)
+            for (int q = threadIdx.x; q < a.total; q += T) a.buf[b][q] = pipe_buf[b * a.total + q];
+    }
     if (CLUSTER) sync();  // no CTA leaves while another's stores to it may be in flight
     if (gt == 0) { c->time = time; c->dt = dt; c->step = step; c->active = active; }
 }
@@ -417,6 +473,8 @@ struct nest_pipeline {
     int ncells = 0;
     int2* dcopies = nullptr;          // 1D: the exchange plan's element pairs
     int ncopies = 0;
+    int slots = 0;                    // 1D: groups of up to LOOP_SLOT cells of one patch
+    size_t loop_smem = 0;             // shared memory that the one-CTA form may take for the buffers
     int loop_ctas = 0;                // CTAs of the one-launch form (0: a launch per stage)
     cudaStream_t own = nullptr;
     std::map<std::pair<void*, cudaStream_t>, cudaGraphExec_t> graphs;
@@ -533,10 +591,23 @@ cudaError_t launch_loop(nest_pipeline* p, void* state, int steps, int max_steps,
     a.c = p->ctrl;
     a.steps = steps; a.max_steps = max_steps; a.step0 = step0;
     const int NC = p->loop_ctas;
-    const int per = (p->ncells + NC - 1) / NC;  // cells per CTA
+    // shared faces where the slots take no more rounds of the warps than the cells do of the
+    // threads (8000 cells in 16 patches, two rounds for one: 19.4 us a step for 16.9) and
+    // short patches do not leave their lanes idle
+    auto rounds = [&](int units, int per_cta) { return (units + NC * per_cta - 1) / (NC * per_cta); };
+    const int cell_rounds = NC == 1 ? LOOP_K : rounds(p->ncells, LOOP_THREADS);
+    a.share = rounds(p->slots, LOOP_THREADS / 32) <= cell_rounds && LOOP_SLOT * p->slots <= 2 * p->ncells;
+    const int per = ((a.share ? 32 * p->slots : p->ncells) + NC - 1) / NC;  // lanes per CTA
     const int threads = std::min(LOOP_THREADS, (per + 31) / 32 * 32);
     if (NC == 1) {
-        k_pipe_loop<false><<<1, threads, 0, st>>>(a);
+        a.total = (int)p->total;
+        a.nbuf = p->nwork + 1;
+        const size_t smem = sizeof(double) * (size_t)a.total * a.nbuf;
+        // (a caller may pass one of the work arrays as the state)
+        bool apart = true;
+        for (double* w : p->work) apart = apart && ((double*)state + p->total <= w || w + p->total <= (double*)state);
+        if (!apart || smem > p->loop_smem) k_pipe_loop<false, false><<<1, threads, 0, st>>>(a);
+        else k_pipe_loop<false, true><<<1, threads, smem, st>>>(a);
         return cudaGetLastError();
     }
     cudaLaunchConfig_t cfg = {};
@@ -550,17 +621,17 @@ cudaError_t launch_loop(nest_pipeline* p, void* state, int steps, int max_steps,
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_pipe_loop<true>, a);
+    return cudaLaunchKernelEx(&cfg, k_pipe_loop<true, false>, a);
 }
 
 // CTAs of the one-launch form for a 1D pipeline: one for the smallest, else a
 // cluster of 16 (or the 8 every device places), 0 where the cells do not fit.
-int loop_ctas_for(int ncells) {
-    if (ncells <= LOOP_ONE_CTA) return 1;
+int loop_ctas_for(int ncells, int slots) {
+    if (ncells <= LOOP_ONE_CTA || (slots <= LOOP_ONE_SLOTS && LOOP_SLOT * slots <= 2 * ncells)) return 1;
     for (int NC : {16, 8}) {
         if (ncells > NC * LOOP_THREADS * LOOP_K) continue;
         if (NC > 8 &&
-            cudaFuncSetAttribute(k_pipe_loop<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaFuncSetAttribute(k_pipe_loop<true, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             cudaGetLastError();
             continue;
         }
@@ -575,7 +646,7 @@ int loop_ctas_for(int ncells) {
         cfg.attrs = at;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, k_pipe_loop<true>, &cfg) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&clusters, k_pipe_loop<true, false>, &cfg) != cudaSuccess) {
             cudaGetLastError();
             continue;
         }
@@ -646,9 +717,18 @@ nest_status nest_pipeline_create(int dim, int nx, int ny, int npx, int npy, int 
         p->patches.push_back(pi);
         p->max_n0 = std::max(p->max_n0, pi.n0);
         p->ncells += dim == 1 ? pi.n0 : 0;
+        p->slots += dim == 1 ? (pi.n0 + LOOP_SLOT - 1) / LOOP_SLOT : 0;
     }
     cudaError_t e;
-    if (dim == 1 && p->ncells <= 16 * LOOP_THREADS * LOOP_K && (p->loop_ctas = loop_ctas_for(p->ncells)) > 0) {
+    if (dim == 1 && p->ncells <= 16 * LOOP_THREADS * LOOP_K && (p->loop_ctas = loop_ctas_for(p->ncells, p->slots)) > 0) {
+        const size_t need = sizeof(double) * (size_t)p->total * (nwork + 1);
+        if (p->loop_ctas == 1 && need <= LOOP_SMEM) {
+            if (cudaFuncSetAttribute(k_pipe_loop<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)LOOP_SMEM) == cudaSuccess)
+                p->loop_smem = LOOP_SMEM;
+            else
+                cudaGetLastError();
+        }
         std::vector<int2> pairs;
         for (auto [d, src] : exchange_pairs_1d(p->plan)) pairs.push_back(make_int2((int)d, (int)src));
         p->ncopies = (int)pairs.size();

@@ -90,3 +90,48 @@ def test_failures_and_scales(gpu, n, patches):
         if not break_it:
             assert ends[0][0] == ends[1][0] == ""
             assert np.array_equal(ends[0][1].view(np.int64), ends[1][1].view(np.int64))
+
+
+@pytest.mark.parametrize("n,patches,nwork,alias", [
+    (28, 1, 3, False), (29, 1, 3, False), (84, 3, 3, False), (87, 3, 3, False), (300, 20, 3, False),
+    (301, 10, 3, True), (630, 2, 16, False), (1300, 13, 3, False), (1400, 100, 3, False), (15000, 2, 3, False)])
+def test_shared_faces_and_buffers(gpu, n, patches, nwork, alias):
+    """Patches around the cells of a warp that shares faces (28) and too short
+    for it; buffers too large for shared memory, and a work array passed as
+    the state: state and work arrays equal a launch per stage, bit for bit."""
+    import torch
+    from nest_b200 import _capi as A
+    from nest_b200 import pipeline as P
+    ends = []
+    for pad in (0, 30):
+        p = P.Pipeline(1, n, patches, nwork=nwork)
+        p.add(P.CFL_DT, src=P.STATE, param=0.4).add(P.EXCHANGE, src=P.STATE).add(P.COPY, src=P.STATE, dst=1)
+        p.add(P.EULER_RHS, src=P.STATE, dst=2).add(P.COPY, src=2, dst=P.STATE).add(P.EXCHANGE, src=P.STATE)
+        p.add(P.EULER_RHS, src=P.STATE, dst=2).add(P.AVERAGE, src=1, aux=2, dst=P.STATE).add(P.CLOCK)
+        for _ in range(pad):
+            p.add(P.COPY, src=1, dst=1)
+        U = torch.from_numpy(p.scatter(initial(n, n))).cuda()
+        work = []
+        for w in range(1, nwork + 1):
+            ptr = A.C.c_void_p()
+            A.check(A.lib.nest_pipeline_buffer(p._h, w, A.C.byref(ptr)), "nest_pipeline_buffer")
+            work.append(ptr.value)
+
+        def view(ptr):
+            import types
+            o = types.SimpleNamespace(__cuda_array_interface__={
+                "shape": (p.size,), "typestr": "<f8", "data": (ptr, False), "version": 3})
+            return torch.as_tensor(o, device="cuda")
+        state = view(work[2]) if alias else U
+        state.copy_(U)
+        torch.cuda.synchronize()
+        steps = p.run(state.data_ptr(), 1e9, max_steps=8)
+        p.execute(state.data_ptr())
+        clock = p.clock()
+        ends.append((steps, clock, state.cpu().numpy(), [view(w).cpu().numpy() for w in work]))
+        p.close()
+    assert ends[0][:2] == ends[1][:2] and ends[0][1][2] == 9
+    assert np.isfinite(ends[0][2]).all()
+    assert np.array_equal(ends[0][2].view(np.int64), ends[1][2].view(np.int64))
+    for a, b in zip(ends[0][3], ends[1][3]):
+        assert np.array_equal(a.view(np.int64), b.view(np.int64))
