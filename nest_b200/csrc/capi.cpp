@@ -57,6 +57,8 @@ std::string nestb::ctrl_error_text(const StepCtrl& c, int steps_now) {
         std::snprintf(buf, sizeof buf, "%s at step %d in cell (%d, %d): rho = %.17g, p = %.17g",
                       nan ? "non-finite state (NaN)" : "positivity violation (rho <= 0 or p <= 0)", c.bad_step,
                       c.bad_i, c.bad_j, c.bad_rho, c.bad_p);
+    } else if (c.err & ERRW_LOST) {
+        std::snprintf(buf, sizeof buf, "a wait between thread blocks ran into its limit after step %d", steps_now);
     } else {
         std::snprintf(buf, sizeof buf, "non-finite state: infinite or NaN wave speed after step %d", steps_now);
     }

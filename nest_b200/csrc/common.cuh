@@ -53,8 +53,9 @@ enum { BC_PERIODIC = 0, BC_OUTFLOW = 1 };
 enum : unsigned {
     ERRW_NONFINITE = 1u,   // a wave speed, density or pressure was NaN / Inf
     ERRW_NONPOSITIVE = 2u, // rho <= 0 or p <= 0 in an interior cell after a step
+    ERRW_LOST = 4u,        // a wait between the CTAs of a cluster ran into its limit
 };
-constexpr unsigned ERRW_STOP = ERRW_NONFINITE | ERRW_NONPOSITIVE;
+constexpr unsigned ERRW_STOP = ERRW_NONFINITE | ERRW_NONPOSITIVE | ERRW_LOST;
 
 // Per-solver control block in device memory.  Fields indexed [p] belong to
 // the step launched with parity p; a step with parity p reads slot p and

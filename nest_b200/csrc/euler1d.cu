@@ -217,108 +217,210 @@ k1d_resident(double* __restrict__ Ug, int n, int h, double dx, double gamma, int
     }
 }
 
+// Point-to-point messages between the CTAs of a cluster: a store into another
+// CTA's shared memory that counts its bytes on an mbarrier there (st.async), so a
+// receiver waits for its data alone and a sender for nothing.
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned peer_addr(unsigned a, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void send_f64(unsigned dst, double v, unsigned bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];"
+                 ::"r"(dst), "l"(__double_as_longlong(v)), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void bar_init(unsigned bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+// The one arrival of a phase, which then completes with its last byte.
+__device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Waits for the phase of that parity; false after 2^24 polls (a quarter of a second
+// and more), which no message takes.
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
+    for (int k = 0; k < 1 << 24; ++k) {
+        unsigned done;
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
 // Largest chunk of the resident loop: cells per CTA (9 warps of 31 cells).
 constexpr int LOOP_WARPS = 9, LOOP_CELLS = 31 * LOOP_WARPS;
 
 // The resident time loop: the NC CTAs of a thread-block cluster (one per SM), or
-// one CTA, split the cells into contiguous chunks of m and run the complete
-// loop.  One thread owns one cell: its U and U1 stay in registers, and only the
-// primitives go through shared memory, with two halo cells on each side.  Lane
-// k of a warp computes the face to the right of cell first + k - 1, and takes the
-// left face of its own cell (k >= 1) from the lane below, so a warp computes 32
-// faces for 31 cells and a stage needs no barrier between its fluxes and its
-// update.  The threads of a CTA's first two and last two cells also store
-// their primitives into the halo slots of the neighbouring CTAs (distributed
-// shared memory); the primitives are double-buffered by stage, so one barrier
-// per stage orders those stores against the reads.  Each warp sends its
-// wave-speed maximum to every CTA before the stage-2 barrier, so after it dt
-// comes from local shared memory, while the stage-1 fluxes (which do not need
-// dt) are computed.
-// What bounds it is one thread's chain of dependent FP64 operations: a step is
-// two face chains and two cell chains, and in a cluster two barriers of about
-// 0.45 us.  Sod tube, us per step (with IEEE divisions and square roots, state in
-// shared memory and a barrier between fluxes and update): 100 cells 1.50 (5.87),
-// 200 cells 1.92 (6.47), both one CTA; 1024 cells on 16 CTAs 2.51 (4.67), 4080
-// cells 3.49 (5.68).
+// one CTA, split the cells into contiguous chunks (of m at most) and run the
+// complete loop.  One thread owns one cell: its U and U1 stay in registers, and
+// only the primitives go through shared memory.  Lane k of a warp computes the
+// face to the right of its cell, and takes the left face (k >= 1) from the lane
+// below, so a warp computes 32 faces for 31 cells and a stage needs no barrier
+// between its fluxes and its update.
+// In a cluster a step has one exchange: at its end the threads of a chunk's first
+// and last four cells send their new state to the neighbouring CTAs, which
+// compute U1 of the two nearest cells themselves, and every warp sends its
+// wave-speed maximum to every CTA, so dt comes from local shared memory while
+// the stage-1 fluxes (which do not need it) are computed.
+// What bounds it is one thread's chain of dependent FP64 operations (two face
+// chains and two cell chains a step) and, in a cluster, the exchange.
+// Sod tube, us per step (with IEEE divisions and square roots, state in shared
+// memory and a barrier between fluxes and update): 100 cells 1.43 (5.87), 200 cells
+// 1.85 (6.47), both one CTA; 1024 cells on 16 CTAs 2.00 (4.67), 4080 cells 2.92 (5.68).
+// Two cluster barriers a step instead (about 0.45 us each): 2.46 and 3.40; messages
+// for both stages 2.20 and 3.04; registers for two blocks an SM (96, spills) 2.13, 2.99.
 // LIM: the slope limiter fixed at compile time (LIM_MINMOD, nest's default) or
 // -1 to read it from the loop parameters.
 template <bool CLUSTER, int LIM>
-__global__ void __launch_bounds__(32 * LOOP_WARPS)
+__global__ void __launch_bounds__(32 * LOOP_WARPS, 1)
 k1d_loop(double* __restrict__ Ug, int n, int h, int m, double dx, double gamma, int bc, LoopParams lp,
          StepCtrl* ctrl, int p) {
     namespace cg = cooperative_groups;
     extern __shared__ double sm[];
     const int NC = CLUSTER ? (int)cg::this_cluster().num_blocks() : 1;
     const int r = CLUSTER ? (int)cg::this_cluster().block_rank() : 0;
-    auto sync = [&]() {
-        if (CLUSTER) cg::this_cluster().sync();
-        else __syncthreads();
-    };
-    auto peer = [&](double* a, int rank) { return CLUSTER ? cg::this_cluster().map_shared_rank(a, rank) : a; };
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int nt = n + 2 * h;
-    const int c_lo = r * m, mloc = min(n, c_lo + m) - c_lo;  // this CTA's cells [c_lo, c_lo + mloc)
-    const int mw = m + 4;                                     // W row: 2 halo slots each side
-    double* const W = sm;             // [2][3][mw]: buffer b, variable k, local cell l at 2 + l
-    double* const red = W + 6 * mw;   // [NC * nw] wave-speed maxima of every warp
+    // this CTA's cells [c_lo, c_lo + mloc)
+    const int mloc = n / NC + (r < n % NC ? 1 : 0), c_lo = r * (n / NC) + min(r, n % NC);
+    constexpr int H = CLUSTER ? 4 : 2, X = CLUSTER ? 2 : 0;   // halo slots, recomputed cells on each side
+    const int mw = m + 2 * H;
+    double* const W = sm;             // [3][3][mw]: state of even / odd steps and U1, variable k, local cell l at H + l
+    double* const Uh = W + 9 * mw;    // [2][4][2]: momentum and energy of the recomputed cells, by step
+    double* const red = Uh + 16;      // [2][NC * nw]: wave-speed maxima of every warp, by step
     const Gas<double> gas(gamma);
     const int left = (r + NC - 1) % NC, right = (r + 1) % NC;
-    const int mloc_left = min(n, left * m + m) - left * m;
+    const int mloc_left = n / NC + (left < n % NC ? 1 : 0);
+    const bool per = bc == BC_PERIODIC;
+    const bool has_left = CLUSTER && (per || r > 0), has_right = CLUSTER && (per || r < NC - 1);
 
-    const int l = 31 * warp + lane - 1;       // this lane's face is to the right of local cell l
-    const bool own = lane >= 1 && l < mloc;   // and it owns cell l
+    const int l = 31 * warp + lane - 1 - X;           // this lane's face is to the right of local cell l
+    const bool own = lane >= 1 && l >= 0 && l < mloc; // and it owns cell l,
+    const bool ext = lane >= 1 && ((has_left && l < 0) || (has_right && l >= mloc && l < mloc + X));  // or repeats its U1
     const int c = c_lo + l;
-    const int ls = min(l, mloc - 1);          // lanes past the chunk repeat its last face
+    // lanes past the faces that a stage needs repeat the last one
+    const int ls1 = min(max(l, has_left ? -1 - X : -1), mloc - 1 + (has_right ? X : 0)), ls2 = min(max(l, -1), mloc - 1);
+    const bool edge = CLUSTER && (warp == 0 || 31 * warp + 30 - X >= mloc - 2);  // reads halo slots
 
-    // stores the primitives of the own cell into buffer b and the halo slots it feeds
+    // Message q (0 before the loop, it + 1 at the end of step it) is the halo of the state
+    // and the maxima, with buffers and barriers by q & 1.  Thread 0 announces the bytes of
+    // q + 2 when q has arrived: they cannot be sent before its own warp's maximum
+    // q + 1, which it sends later.  For the same reason nothing of q is overwritten by
+    // q + 2 before every warp here has read it.
+    __shared__ unsigned long long bars[4];
+    __shared__ volatile unsigned lost;        // a wait gave up
+    const unsigned bar0 = smem_addr(bars);
+    auto bar_halo = [&](int q) { return bar0 + 8 * (q & 1); };
+    auto bar_max = [&](int q) { return bar0 + 16 + 8 * (q & 1); };
+    const unsigned halo_bytes = 128u * ((has_left ? 1 : 0) + (has_right ? 1 : 0)), max_bytes = 8u * NC * nw;
+    auto announce = [&](int q) { bar_expect(bar_halo(q), halo_bytes); bar_expect(bar_max(q), max_bytes); };
+
+    // stores the primitives of the lane's cell into buffer b, with the ghosts they feed
     auto put = [&](int b, double v0, double v1, double v2) {
-        auto to = [&](double* base, int slot) {
-            double* w = base + b * 3 * mw + slot;
-            w[0] = v0; w[mw] = v1; w[2 * mw] = v2;
-        };
-        to(W, 2 + l);
-        const bool per = bc == BC_PERIODIC;
-        if (l < 2 && (per || r > 0)) to(peer(W, left), mloc_left + 2 + l);
-        if (l >= mloc - 2 && (per || r < NC - 1)) to(peer(W, right), l - (mloc - 2));
-        if (!per && c == 0) { to(W, 0); to(W, 1); }
-        if (!per && c == n - 1) { to(W, mloc + 2); to(W, mloc + 3); }
+        double* const w = W + b * 3 * mw + H;
+        auto to = [&](int x) { w[x] = v0; w[mw + x] = v1; w[2 * mw + x] = v2; };
+        to(l);
+        if (!per) {
+            if (c == 0) { to(-1); to(-2); }
+            if (c == n - 1) { to(mloc); to(mloc + 1); }
+        } else if (!CLUSTER) {
+            if (l < 2) to(mloc + l);
+            if (l >= mloc - 2) to(l - mloc);
+        }
     };
-    auto faces = [&](int b) {
-        const double* w = W + b * 3 * mw + ls + 1;
+    // sends the own cell, four from an end of the chunk or less, to the neighbour there
+    auto send_halo = [&](int q, double v0, double v1, double v2, double m1, double e2) {
+        auto send = [&](int rank, int x, int xu) {
+            const unsigned bar = peer_addr(bar_halo(q), rank);
+            const unsigned a = peer_addr(smem_addr(W + (q & 1) * 3 * mw + H + x), rank);
+            send_f64(a, v0, bar); send_f64(a + 8 * mw, v1, bar); send_f64(a + 16 * mw, v2, bar);
+            if (xu >= 0) {
+                const unsigned u = peer_addr(smem_addr(Uh + (q & 1) * 8 + 2 * xu), rank);
+                send_f64(u, m1, bar); send_f64(u + 8, e2, bar);
+            }
+        };
+        if (l < 4 && has_left) send(left, mloc_left + l, l < 2 ? 2 + l : -1);
+        if (l >= mloc - 4 && has_right) send(right, l - mloc, l >= mloc - 2 ? l - (mloc - 2) : -1);
+    };
+    auto faces = [&](int b, int ls) {
+        const double* w = W + b * 3 * mw + H + ls - 1;
         return plm_flux(gas, LIM >= 0 ? LIM : lp.lim, [&](int k, int s) { return w[k * mw + s]; }, 0, 1, 2, 3);
     };
-    auto send_max = [&](double s) {
+    auto send_max = [&](double s, int q) {
         s = warp_max_speed(s);
-        if (lane < NC) peer(red, lane)[r * nw + warp] = s;
+        double* const d = red + (CLUSTER ? (q & 1) * NC * nw : 0) + r * nw + warp;
+        if (CLUSTER) {
+            if (lane < NC) send_f64(peer_addr(smem_addr(d), lane), s, peer_addr(bar_max(q), lane));
+        } else if (lane == 0) {
+            *d = s;
+        }
     };
-    auto read_max = [&]() {
+    auto read_max = [&](int q) {
+        const double* const d = red + (CLUSTER ? (q & 1) * NC * nw : 0);
         double s = 0.0;
-        for (int q = lane; q < NC * nw; q += 32) s = smax(s, red[q]);
+        for (int k = lane; k < NC * nw; k += 32) s = smax(s, d[k]);
         return warp_max_speed(s);
     };
-
-    // prologue: the own cell, its primitives (buffer 0) and the first wave speeds
     double u0 = 1.0, u1 = 0.0, u2 = 1.0;
-    if (own) { u0 = Ug[h + c]; u1 = Ug[nt + h + c]; u2 = Ug[2 * nt + h + c]; }
-    if (CLUSTER) sync();  // every CTA of the cluster runs before its memory is written
-    {
-        const Cell1<double> w = cell1d<true>(gas, u0, u1, u2);
-        if (own) put(0, u0, w.u, w.p);
-        send_max(own ? smax(0.0, fabs(w.u) + w.cs) : 0.0);
-    }
-    sync();
+    // waits for message q and takes the state of a recomputed cell from it.  (Waiting for the
+    // maxima after the stage-1 fluxes took dt's division out of their shadow: 2.13 -> 2.25
+    // us a step at 1024 cells.)
+    auto receive = [&](int q) {
+        if (!CLUSTER) return;
+        const unsigned parity = (q >> 1) & 1;
+        const bool ok = (!edge || bar_wait(bar_halo(q), parity)) && bar_wait(bar_max(q), parity);
+        if (!ok) {
+            lost = 1u;
+            if (lane == 0) atomicOr(&ctrl->err, ERRW_LOST);
+        } else if (threadIdx.x == 0) {
+            announce(q + 2);
+        }
+        if (ext) {
+            const double* const u = Uh + (q & 1) * 8 + 2 * (l < 0 ? l + 2 : 2 + l - mloc);
+            u0 = W[(q & 1) * 3 * mw + H + l]; u1 = u[0]; u2 = u[1];
+        }
+    };
 
+    // prologue: the own cell, its primitives and the first wave speeds
+    if (own) { u0 = Ug[h + c]; u1 = Ug[nt + h + c]; u2 = Ug[2 * nt + h + c]; }
+    if (CLUSTER) {
+        if (threadIdx.x == 0) {
+            for (int k = 0; k < 4; ++k) bar_init(bar0 + 8 * k);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            announce(0);
+            announce(1);
+            lost = 0u;
+        }
+        cg::this_cluster().sync();  // every CTA of the cluster runs, its barriers announced
+    }
     double time = ctrl->time[p];
     int step = ctrl->step[p];
-    const bool stopped = (ctrl->err & ERRW_STOP) != 0;  // an earlier step failed: run nothing
+    // an earlier step failed: run nothing.  (Read before the first maximum is sent, which
+    // depends on it: other CTAs may flag a cell once they have that.)
+    const bool stopped = (*reinterpret_cast<volatile unsigned*>(&ctrl->err) & ERRW_STOP) != 0;
+    {
+        const Cell1<double> w = cell1d<true>(gas, u0, u1, u2);
+        if (own) {
+            put(0, u0, w.u, w.p);
+            if (CLUSTER) send_halo(0, u0, w.u, w.p, u1, u2);
+        }
+        send_max(own && !stopped ? smax(0.0, fabs(w.u) + w.cs) : 0.0, 0);
+    }
+    __syncthreads();
+    receive(0);
+
     for (int it = 0;; ++it) {
         if (stopped) break;
         if (lp.step_budget > 0 && it >= lp.step_budget) break;
         if (lp.t_final > 0.0 && !(time < lp.t_final)) break;
         if (lp.max_steps > 0 && step >= lp.max_steps) break;
         if (lp.dts_in && step >= lp.dts_cap) break;
-        const double ms = read_max();
-        const F3<double> f = faces(0);
+        const double ms = read_max(it);
+        const F3<double> f = faces(CLUSTER ? it & 1 : 0, ls1);
         double dt;
         if (lp.fixed_dt > 0.0) {
             dt = lp.fixed_dt;
@@ -328,8 +430,9 @@ k1d_loop(double* __restrict__ Ug, int n, int h, int m, double dx, double gamma, 
             dt = div_rn(lp.cfl * dx, ms);
             if (lp.t_final > 0.0) dt = smin(dt, lp.t_final - time);
         }
-        if (!(ms == ms) || ms > 1.79e308) { if (r == 0 && threadIdx.x == 0) atomicOr(&ctrl->err, ERRW_NONFINITE); break; }
-        if (r == 0 && threadIdx.x == 0 && lp.dts_out && step < lp.dts_cap) lp.dts_out[step] = dt;
+        const bool bad = !(ms == ms) || ms > 1.79e308;
+        if (!CLUSTER && bad) { if (threadIdx.x == 0) atomicOr(&ctrl->err, ERRW_NONFINITE); break; }
+        if (r == 0 && threadIdx.x == 0 && lp.dts_out && step < lp.dts_cap && !bad) lp.dts_out[step] = dt;
         const double dtdx = div_rn(dt, dx);
         // stage 1: U1 = U - dtdx (F_right - F_left)
         const double v0 = u0 - dtdx * (f.a - __shfl_up_sync(0xffffffffu, f.a, 1));
@@ -337,13 +440,19 @@ k1d_loop(double* __restrict__ Ug, int n, int h, int m, double dx, double gamma, 
         const double v2 = u2 - dtdx * (f.c - __shfl_up_sync(0xffffffffu, f.c, 1));
         {
             const Cell1<double> w = cell1d<false>(gas, v0, v1, v2);
-            if (own) put(1, v0, w.u, w.p);
+            if (own || ext) put(2, v0, w.u, w.p);
         }
-        sync();
+        __syncthreads();
+        if (CLUSTER) {
+            // (the same in all threads: lost was written before the barrier, and unless it
+            // was, all of them have the same maximum)
+            if (lost) break;
+            if (bad) { if (r == 0 && threadIdx.x == 0) atomicOr(&ctrl->err, ERRW_NONFINITE); break; }
+        }
         // stage 2: U = (U + U1 - dtdx (F_right - F_left)) / 2, its wave speed
         // and positivity (a failing cell makes the maximum infinite, which
         // ends the loop on every CTA)
-        const F3<double> e = faces(1);
+        const F3<double> e = faces(2, ls2);
         u0 = 0.5 * (u0 + (v0 - dtdx * (e.a - __shfl_up_sync(0xffffffffu, e.a, 1))));
         u1 = 0.5 * (u1 + (v1 - dtdx * (e.b - __shfl_up_sync(0xffffffffu, e.b, 1))));
         u2 = 0.5 * (u2 + (v2 - dtdx * (e.c - __shfl_up_sync(0xffffffffu, e.c, 1))));
@@ -351,16 +460,18 @@ k1d_loop(double* __restrict__ Ug, int n, int h, int m, double dx, double gamma, 
             const Cell1<double> w = cell1d<true>(gas, u0, u1, u2);
             double s = 0.0;
             if (own) {
-                put(0, u0, w.u, w.p);
+                put(CLUSTER ? (it + 1) & 1 : 0, u0, w.u, w.p);
+                if (CLUSTER) send_halo(it + 1, u0, w.u, w.p, u1, u2);
                 s = smax(0.0, fabs(w.u) + w.cs);
                 if (!(u0 > 0.0) || !(w.p > 0.0)) {
                     flag_cell(ctrl, step + 1, u0, w.p, c, 0);
                     s = __longlong_as_double(0x7ff0000000000000ll);
                 }
             }
-            send_max(s);
+            send_max(s, it + 1);
         }
-        sync();
+        __syncthreads();
+        receive(it + 1);
         time += dt;
         ++step;
     }
@@ -382,7 +493,13 @@ k1d_loop(double* __restrict__ Ug, int n, int h, int m, double dx, double gamma, 
         ctrl->time[p] = time; ctrl->step[p] = step;
         ctrl->time[p ^ 1] = time; ctrl->step[p ^ 1] = step;
     }
-    if (CLUSTER) sync();  // no CTA leaves while a neighbour's stores to it may be in flight
+    if (CLUSTER) {
+        // no CTA leaves while stores to it may be in flight (after a wait that gave up,
+        // some that nobody has waited for)
+        if (lost)
+            for (int k = 0; k < 100; ++k) __nanosleep(1000);
+        cg::this_cluster().sync();
+    }
 }
 
 size_t resident_smem_bytes(int n, int h) {
@@ -396,12 +513,13 @@ struct LoopShape {
     size_t smem;
 };
 // Chunk and block size for n cells on NC CTAs; false where they do not fit
-// (every CTA of a cluster needs two cells for the halos).
+// (every CTA of a cluster needs four cells for its neighbours' halos).
 static bool loop_shape(int n, int NC, LoopShape& s) {
     s.m = (n + NC - 1) / NC;
-    if (s.m > LOOP_CELLS || (NC > 1 && (s.m < 2 || n - (NC - 1) * s.m < 2))) return false;
-    s.threads = (s.m + 30) / 31 * 32;
-    s.smem = sizeof(double) * (size_t)(6 * (s.m + 4) + NC * (s.threads / 32));
+    const int lanes = s.m + (NC > 1 ? 4 : 0);
+    if (lanes > LOOP_CELLS || (NC > 1 && n / NC < 4)) return false;
+    s.threads = (lanes + 30) / 31 * 32;
+    s.smem = sizeof(double) * (size_t)(9 * (s.m + 8) + 16 + 2 * NC * (s.threads / 32));
     return true;
 }
 
@@ -480,10 +598,9 @@ bool cluster_1d_available(int n, int h) {
 cudaError_t launch_1d_resident(double* U, int n, int h, double dx, double gamma, int bc,
                                const LoopParams& lp, StepCtrl* ctrl, int p, cudaStream_t st) {
     const bool mm = lp.lim == LIM_MINMOD;
-    // up to 279 cells one CTA, whose barrier is cheap (256 cells: 2.39 us a step
-    // on one CTA, 2.43 on a cluster; 434: 2.96 on one CTA of 14 warps, 2.39 on a
-    // cluster)
-    if (n <= LOOP_CELLS) {
+    // fewer than 256 cells: one CTA, whose barrier is cheap (us a step on one CTA / a
+    // cluster: 200 cells 1.83 / 2.16, 248 1.84 / 2.17, 256 2.28 / 2.03)
+    if (n < 256) {
         LoopShape s;
         loop_shape(n, 1, s);
         (mm ? k1d_loop<false, LIM_MINMOD> : k1d_loop<false, -1>)<<<1, s.threads, s.smem, st>>>(U, n, h, s.m, dx, gamma,
