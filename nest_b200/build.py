@@ -1,7 +1,8 @@
 """Build recipe of the CUDA library (libnest_b200.so) for sm_100a.
 
 Each translation unit gets its own floating-point flags:
-  euler1d.cu, euler2d_f64.cu  -fmad=false  (FP64 plain form: bit-exact with
+  euler1d.cu, euler2d_f64*.cu, pipeline.cu
+                              -fmad=false  (FP64 plain form: bit-exact with
                                             nest's CPU operation order)
   euler1d_f32.cu, euler2d_f32*.cu
                               -use_fast_math (FP32 form)

@@ -296,6 +296,10 @@ int strip_width(int precision, int flags) {
 // of 64..256 a side 65 -> 32 (32), 48 of them 81 -> 60 (59), 64 of 48..320 108 -> 95
 // (95), 128 of 64..512 318 (32 rows; 12 rows 328); FP64 batches: 64 of 48..320 312 at
 // 16 rows, 307 at 12, 346 at 4, 128 of 64..512 1057 at 16, 1061 at 32.
+// The same shapes since the stages launch dependently and their FP64 arithmetic
+// shrank: FP32 64^2 8.5, 256 x 192 9.1, 512^2 16.4, 517 x 1003 26.5, 1024^2 43.0,
+// 2048^2 118.8, 4096^2 358; FP64 64^2 17.0, 256 x 192 22.6, 512^2 46.3, 517 x 1003
+// 61.9, 1024^2 100, 2048^2 323; batches of 48 57 (FP32) and 182 (FP64).
 int default_rows(int precision, long long work, int tall64, int tall32) {
     if (precision == NEST_F64) return (int)std::min<long long>(tall64, (work + 3999) / 4000);
     const long long one_wave = (work + 2367) / 2368;
