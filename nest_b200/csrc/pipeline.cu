@@ -302,17 +302,21 @@ __global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
             }
         }
     }
-    if (SMEM) {
+    if (SMEM)
         for (int b = 0; b < a.nbuf; ++b)
             for (int q = threadIdx.x; q < a.total; q += T) pipe_buf[b * a.total + q] = a.buf[b][q];
-        __syncthreads();
-    }
     auto buf = [&](int b) { return SMEM ? pipe_buf + b * a.total : a.buf[b]; };
     double time = c->time, dt = c->dt;
     int step = c->step, active = c->active;
     const double t_final = c->t_final;
     int cfl_count = 0;
-    if (CLUSTER) sync();  // every CTA of the cluster runs before its memory is written
+    // Whether a CHECK has failed, in an earlier launch (read before the barrier: no thread
+    // has run a CHECK) or in this one, where the news travels with the wave-speed
+    // maxima: a thread whose cell failed sends FAILED, above every speed, in the
+    // place of its own, so that all threads stop at the same CFL stage.
+    const double FAILED = __longlong_as_double(0x7fffffffffffffffll);
+    bool stopped = (*reinterpret_cast<volatile unsigned*>(&c->err) & ERRW_STOP) != 0, failed = false;
+    sync();  // the buffers are filled, and every CTA of a cluster runs before its memory is written
 
     for (int n = 0; n < a.steps; ++n) {
         // batches of 8, as a launch per stage runs them
@@ -333,17 +337,17 @@ __global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
                         const Cell1<double> w = cell1d<true>(gas, src[e], src[e + pl], src[e + 2 * pl]);
                         ms = smax(ms, fabs(w.u) + w.cs);
                     }
-                ms = warp_max_speed(ms);
+                ms = warp_max_speed(failed ? FAILED : ms);
                 double* const r = red[cfl_count & 1];
                 ++cfl_count;
                 if (lane < NC)
                     (CLUSTER ? cg::this_cluster().map_shared_rank(r, lane) : r)[rank * nw + warp] = ms;
                 sync();
-                double m = 0.0;
-                for (int q = lane; q < NC * nw; q += 32) m = smax(m, r[q]);
-                m = warp_max_speed(m);
-                const unsigned err = *reinterpret_cast<volatile unsigned*>(&c->err);
-                active = (!(t_final > 0.0) || time < t_final) && !(err & ERRW_STOP) ? 1 : 0;
+                unsigned long long mb = 0;
+                for (int q = lane; q < NC * nw; q += 32) mb = max(mb, speed_bits(r[q]));
+                const double m = warp_max_speed(bits_speed(mb));
+                stopped = stopped || m != m;
+                active = (!(t_final > 0.0) || time < t_final) && !stopped ? 1 : 0;
                 if (active) {
                     dt = div_rn(g.param * a.dx, m);
                     if (t_final > 0.0) dt = smin(dt, t_final - time);
@@ -429,6 +433,7 @@ __global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
                                 double r, u, p;
                                 prim1d(src, own[k].e, own[k].plane, gm1, r, u, p);
                                 if (!(r > 0.0) || !(p > 0.0)) {
+                                    failed = true;
                                     const unsigned bit = (r == r && p == p) ? ERRW_NONPOSITIVE : ERRW_NONFINITE;
                                     if (!(atomicOr(&c->err, bit) & ERRW_STOP)) {
                                         c->bad_step = step + 1; c->bad_cell = own[k].i; c->bad_patch = own[k].patch;
