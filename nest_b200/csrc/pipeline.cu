@@ -587,7 +587,12 @@ cudaError_t launch_loop(nest_pipeline* p, void* state, int steps, int max_steps,
     LoopArgs a{};
     a.nstages = (int)p->stages.size();
     for (int s = 0; s < a.nstages; ++s) a.st[s] = p->stages[s];
-    a.sync_before = loop_barriers(p->stages);
+    // A caller may pass one of the work arrays as the state, or memory that overlaps them:
+    // two indices then name the same elements, which the analysis by index cannot see, so
+    // every stage waits for the one before, as with a launch per stage.
+    bool apart = true;
+    for (double* w : p->work) apart = apart && ((double*)state + p->total <= w || w + p->total <= (double*)state);
+    a.sync_before = apart ? loop_barriers(p->stages) : ~0u;
     for (int b = 0; b <= p->nwork; ++b) a.buf[b] = buffer(p, state, b);
     a.P = p->dpatches;
     a.npatch = p->npatch; a.ncells = p->ncells; a.h = p->halo;
@@ -608,9 +613,6 @@ cudaError_t launch_loop(nest_pipeline* p, void* state, int steps, int max_steps,
         a.total = (int)p->total;
         a.nbuf = p->nwork + 1;
         const size_t smem = sizeof(double) * (size_t)a.total * a.nbuf;
-        // (a caller may pass one of the work arrays as the state)
-        bool apart = true;
-        for (double* w : p->work) apart = apart && ((double*)state + p->total <= w || w + p->total <= (double*)state);
         if (!apart || smem > p->loop_smem) k_pipe_loop<false, false><<<1, threads, 0, st>>>(a);
         else k_pipe_loop<false, true><<<1, threads, smem, st>>>(a);
         return cudaGetLastError();

@@ -77,3 +77,28 @@ def test_check_right_behind_cfl(gpu, n, patches, every):
             assert ends[0][0] == ends[1][0]
         assert np.array_equal(bits(ends[0][1]), bits(ends[1][1]))
         assert np.array_equal(bits(ends[0][2]), bits(ends[1][2]))
+
+
+@pytest.mark.parametrize("n,patches", [(60, 2), (300, 3), (640, 7), (900, 6), (8193, 24), (16000, 9)])
+def test_work_array_as_the_state(gpu, n, patches):
+    """The state is work array 1, which the list uses under both names: what one
+    index's stage reads from neighbours is what the other's stage overwrites."""
+    import torch
+
+    def stages(P):
+        return [(P.CFL_DT, dict(src=0, param=0.3)), (P.EXCHANGE, dict(src=0)), (P.EULER_RHS, dict(src=0, dst=2)),
+                (P.COPY, dict(src=2, dst=1)), (P.EXCHANGE, dict(src=1)), (P.EULER_RHS, dict(src=0, dst=3)),
+                (P.AVERAGE, dict(src=2, aux=3, dst=1)), (P.CHECK, dict(src=1, param=4)), (P.CLOCK, {})]
+    for _ in range(3):
+        ends = []
+        for p in forms(n, patches, stages, nwork=4):
+            d = work_view(p, 1)
+            d.copy_(torch.from_numpy(p.scatter(initial(n))))
+            torch.cuda.synchronize()
+            steps = p.run(d.data_ptr(), 1e9, max_steps=16)
+            p.execute(d.data_ptr())
+            ends.append((steps, p.clock(), [work_view(p, w).cpu().numpy() for w in (1, 2, 3)]))
+            p.close()
+        assert ends[0][:2] == ends[1][:2] and ends[0][0] == 16
+        for a, b in zip(ends[0][2], ends[1][2]):
+            assert np.isfinite(a).all() and np.array_equal(bits(a), bits(b))
