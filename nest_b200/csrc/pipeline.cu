@@ -238,6 +238,7 @@ struct LoopArgs {
     PipeCtrl* c;
     int steps;                    // executions of the stage list at most
     int max_steps, step0;         // > 0: stop at a multiple of 8 executions once step - step0 reaches it
+    int once_more;                // a CFL stage has compute stages before it
 };
 
 // Executes the stage list up to `steps` times in one CTA or one cluster: a
@@ -247,8 +248,11 @@ struct LoopArgs {
 // still be reading, waits for one (LoopArgs::sync_before).  Every thread keeps the
 // clock in registers; they all compute the same dt.  The formulas are those of
 // the stage kernels above, with the branch-free division and square root.
-// An execution whose CFL stage finds the run finished is the last one (its halo
-// exchanges still run; further ones would change nothing).
+// An execution whose CFL stage finds the run finished is the last one: its later halo
+// exchanges still run, and further executions of the batch of eight would run nothing
+// but exchanges.  They would change nothing either, unless compute stages come before the
+// CFL stage in the list and so have changed what exchanges before it have copied; then one
+// more execution of the batch (further ones repeat it) refreshes the halos.
 // share: a warp takes up to 28 neighbouring cells of a patch and a halo of two on each side,
 // and every primitive, slope and flux is computed once instead of by up to five cells.
 // SMEM (one CTA): the buffers live in shared memory for the launch.
@@ -318,6 +322,7 @@ __global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
     bool stopped = (*reinterpret_cast<volatile unsigned*>(&c->err) & ERRW_STOP) != 0, failed = false;
     sync();  // the buffers are filled, and every CTA of a cluster runs before its memory is written
 
+    bool ended = false;
     for (int n = 0; n < a.steps; ++n) {
         // batches of 8, as a launch per stage runs them
         if (n > 0 && (n & 7) == 0 && ((a.max_steps > 0 && step - a.step0 >= a.max_steps) || !(time < t_final))) break;
@@ -449,7 +454,10 @@ __global__ void __launch_bounds__(LOOP_THREADS) k_pipe_loop(LoopArgs a) {
                     break;
             }
         }
-        if (finished) break;
+        if (finished) {
+            if (ended || !a.once_more || (n & 7) == 7) break;
+            ended = true;
+        }
     }
     if (SMEM) {
         __syncthreads();
@@ -600,6 +608,11 @@ cudaError_t launch_loop(nest_pipeline* p, void* state, int steps, int max_steps,
     a.dx = p->dx; a.gamma = p->gamma; a.lim = p->lim;
     a.c = p->ctrl;
     a.steps = steps; a.max_steps = max_steps; a.step0 = step0;
+    bool computed = false;
+    for (const Stage& g : p->stages) {
+        if (g.kind == NEST_STAGE_CFL_DT && computed) a.once_more = 1;
+        computed |= g.kind == NEST_STAGE_EULER_RHS || g.kind == NEST_STAGE_COPY || g.kind == NEST_STAGE_AVERAGE;
+    }
     const int NC = p->loop_ctas;
     // shared faces where the slots take no more rounds of the warps than the cells do of the
     // threads (8000 cells in 16 patches, two rounds for one: 19.4 us a step for 16.9) and

@@ -102,3 +102,33 @@ def test_work_array_as_the_state(gpu, n, patches):
         assert ends[0][:2] == ends[1][:2] and ends[0][0] == 16
         for a, b in zip(ends[0][2], ends[1][2]):
             assert np.isfinite(a).all() and np.array_equal(bits(a), bits(b))
+
+
+@pytest.mark.parametrize("n,patches", [(40, 2), (640, 7), (900, 6), (16000, 9)])
+@pytest.mark.parametrize("steps", [3, 8])
+def test_cfl_stage_last(gpu, n, patches, steps):
+    """The stage that ends a run comes last: the executions that a launch per stage
+    still enqueues refresh the halos, unless the run ends with a batch of eight."""
+    import torch
+
+    def stages(P):
+        return [(P.EXCHANGE, dict(src=0)), (P.EULER_RHS, dict(src=0, dst=2)), (P.COPY, dict(src=2, dst=0)),
+                (P.EXCHANGE, dict(src=2)), (P.CLOCK, {}), (P.CFL_DT, dict(src=0, param=0.3))]
+    ends = []
+    for p in forms(n, patches, stages):
+        d = torch.from_numpy(p.scatter(initial(n))).cuda()
+        torch.cuda.synchronize()
+        p.set_clock(0.0, 0.1 / n, 0)
+        for _ in range(steps - 1):
+            p.execute(d.data_ptr())
+        t, dt, done = p.clock()
+        assert done == steps - 1
+        p.set_clock(0.0, 0.1 / n, 0)
+        d.copy_(torch.from_numpy(p.scatter(initial(n))))
+        torch.cuda.synchronize()
+        count = p.run(d.data_ptr(), t + 0.5 * dt)  # ends in step `steps`
+        ends.append((count, p.clock(), d.cpu().numpy(), work_view(p, 2).cpu().numpy()))
+        p.close()
+    assert ends[0][:2] == ends[1][:2] and ends[0][0] == steps
+    for a, b in zip(ends[0][2:], ends[1][2:]):
+        assert np.array_equal(bits(a), bits(b))
