@@ -76,6 +76,9 @@ struct StepCtrl {
     int bad_i, bad_j;               // its interior index (1D: bad_j = 0)
     int pad_;
     double bad_rho, bad_p;          // and its density and pressure
+    // 1D: a step before the one in slot p has failed.  A one-launch step reads this word:
+    // its own blocks may set `err` while others are starting.
+    unsigned stop[2];
 };
 
 // Time-loop parameters shared by all launches of a solver.
@@ -140,10 +143,11 @@ __device__ __forceinline__ void flag_cell(StepCtrl* c, int step_done, double rho
     c->bad_p = pr;
 }
 
-// Decide the step: returns false when the run is finished.  Every block of
+// Decide the step: returns true when the run is finished.  Every block of
 // stage 1 evaluates this on the same inputs, so all agree; block 0 publishes.
-__device__ __forceinline__ bool step_is_done(const StepCtrl* c, int p, const LoopParams& lp) {
-    if (c->err & ERRW_STOP) return true;
+// one_launch: the step's own blocks may set `err` (k1d_step).
+__device__ __forceinline__ bool step_is_done(const StepCtrl* c, int p, const LoopParams& lp, bool one_launch = false) {
+    if (one_launch ? c->stop[p] != 0 : (c->err & ERRW_STOP) != 0) return true;
     double t = c->time[p];
     int s = c->step[p];
     if (lp.t_final > 0.0 && !(t < lp.t_final)) return true;
@@ -200,6 +204,7 @@ __device__ __forceinline__ void publish_step_1d(StepCtrl* c, int p, const LoopPa
         c->maxs[q][w] = c->maxs[p][w];
         c->maxs[q][1 - w] = 0ull;
         c->sel[q] = w + 2 * (1 - w);
+        c->stop[q] = (c->err & ERRW_STOP) != 0;  // (no block of a finished step sets it)
         c->active[q] = 0;
         return;
     }

@@ -104,7 +104,10 @@ k1d_stage(const T* __restrict__ Uin, const T* Un, T* Uout,
         if (STAGE == 2) {
             const Cell1<T> w = cell1d<true>(gas, v[0], v[1], v[2]);
             ms = (double)(fabs(w.u) + w.cs);
-            if (!(v[0] > T(0)) || !(w.p > T(0))) flag_cell(ctrl, ctrl->step[p] + 1, (double)v[0], (double)w.p, c, 0);
+            if (!(v[0] > T(0)) || !(w.p > T(0))) {
+                flag_cell(ctrl, ctrl->step[p] + 1, (double)v[0], (double)w.p, c, 0);
+                ctrl->stop[p ^ 1] = 1u;
+            }
         }
     }
     if (STAGE == 2) {
@@ -116,7 +119,10 @@ k1d_stage(const T* __restrict__ Uin, const T* Un, T* Uout,
             double x = (l < (NT1 + 31) / 32) ? red[l] : 0.0;
             x = warp_max(x);
             if (l == 0) {
-                if (!(x == x) || x > 1.79e308) atomicOr(&ctrl->err, ERRW_NONFINITE);
+                if (!(x == x) || x > 1.79e308) {
+                    atomicOr(&ctrl->err, ERRW_NONFINITE);
+                    ctrl->stop[p ^ 1] = 1u;
+                }
                 atomic_max_speed(&ctrl->maxs[p ^ 1][0], x);
             }
         }
@@ -203,7 +209,7 @@ k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out,
     for (int i = 0; i < CPL; ++i)
 #pragma unroll
         for (int k = 0; k < 3; ++k) u[i][k] = Un[k * nt + e[i]];
-    if (step_is_done(ctrl, p, lp)) {
+    if (step_is_done(ctrl, p, lp, true)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) publish_step_1d(ctrl, p, lp, true, 0.0, true);
         for (int i = 0; i < CPL; ++i)
             if (own(i)) store(Unext, u[i], c + i);
@@ -268,7 +274,10 @@ k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out,
             if (U1out) store(U1out, v[i], c + i);
             // (a NaN is dropped here and flagged below)
             ms = smax(ms, (double)(fabs(q.u) + q.cs));
-            if (!(x[0] > T(0)) || !(q.p > T(0))) flag_cell(ctrl, ctrl->step[p] + 1, (double)x[0], (double)q.p, c + i, 0);
+            if (!(x[0] > T(0)) || !(q.p > T(0))) {
+                flag_cell(ctrl, ctrl->step[p] + 1, (double)x[0], (double)q.p, c + i, 0);
+                ctrl->stop[p ^ 1] = 1u;
+            }
         }
     }
     ms = warp_max_speed(ms);
@@ -277,7 +286,10 @@ k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out,
     if (threadIdx.x == 0) {
         double m = red[0];
         for (int i = 1; i < STEP_WARPS; ++i) m = smax(m, red[i]);
-        if (m > 1.79e308) atomicOr(&ctrl->err, ERRW_NONFINITE);
+        if (m > 1.79e308) {
+            atomicOr(&ctrl->err, ERRW_NONFINITE);
+            ctrl->stop[p ^ 1] = 1u;
+        }
         atomic_max_speed(&ctrl->maxs[p ^ 1][sel >> 1], m);
     }
 }
