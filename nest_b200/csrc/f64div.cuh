@@ -16,17 +16,22 @@
 // et al., Handbook of Floating-Point Arithmetic, 2nd ed., 2018, ch. 4):
 //   * y = recip_f64(b): from the hardware approximation y0 (measured over every
 //     high word: |1 - b y0| < 2^-19.9) three Newton-Raphson steps
-//     y <- y + y (1 - b y).  The second leaves 1/b to 2^-79 and its rounding;
-//     the last one's residual is exact (y is within 0.6 ulp), so y is the
-//     rounding of (1/b)(1 - eta) with 0 <= eta < 2^-105.  One y serves every
-//     quotient by b.
+//     y <- y + y (1 - b y).  The second leaves 1/b to 2^-79 and its rounding; it
+//     rounds up, so that y is 1/b at least (to 2^-79) and less than an ulp above.
+//     The last one's residual e is exact, |e| <= m_b 2^-53 (m_b in [1, 2) the
+//     significand of b), so y is the rounding of (1/b)(1 - e^2).  The reciprocal of
+//     b = 2 - ulp lies next to a midpoint, 2^-106 above it, the nearest of all:
+//     rounded to nearest the second step fell below it, and the last was a tie that
+//     stayed there.  From above it ends at RN(1/b), and so does b = 2 - 2 ulp.
+//     One y serves every quotient by b.
 //   * q0 = a y, r = b q0 - a, q = q0 - r y (quot_f64).  With eps the relative
 //     error of y, q is the rounding of a/b + (a/b - q0) eps.  A quotient of
 //     two doubles stays at least ulp(q) 2^-53 / m_b away from every midpoint
-//     of two doubles (m_b in [1, 2) the significand of b), and |eps| <= m_b
-//     2^-54 + 2^-105.  Next to a midpoint |a/b - q0| is half an ulp, or one and
-//     a half if q0 is not a faithful rounding.  Half an ulp: the
-//     perturbation is smaller than the distance, because m_b <= 2 - 2^-52.
+//     of two doubles, and |eps| <= m_b 2^-54 + m_b^2 2^-106.  Next to a midpoint
+//     |a/b - q0| is half an ulp, or one and a half if q0 is not a faithful
+//     rounding.  Half an ulp: the perturbation is smaller than the distance
+//     where (m_b / 2)^2 (1 + m_b 2^-52) < 1, for all but the two divisors above, whose
+//     y = RN(1/b) has an eps of 2^-53 - 2^-106 and 2^-104.
 //     One and a half: q0 = RN(a y) can only be that far off where a's
 //     significand exceeds 2 - 5 2^-52 and b's is larger still, and all
 //     those quotients lie next to a double, not next to a midpoint.  So q =
@@ -56,7 +61,7 @@ __device__ __forceinline__ double recip_f64(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
     y = fma(y, fma(-b, y, 1.0), y);
-    y = fma(y, fma(-b, y, 1.0), y);
+    y = __fma_ru(y, fma(-b, y, 1.0), y);
     return fma(y, fma(-b, y, 1.0), y);
 }
 
@@ -92,7 +97,7 @@ __device__ __forceinline__ double sqrt_quot_f64(double a, double b, double& y) {
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(h) : "d"(t));
     h *= 0.5;
     h = fma(h, fma(-(t2 * h), h, 0.5), h);  // 1 / (2 sqrt(q)) to 2^-39
-    y = fma(y, fma(-b, y, 1.0), y);
+    y = __fma_ru(y, fma(-b, y, 1.0), y);
     y = fma(y, fma(-b, y, 1.0), y);
     const double q = quot_f64(a, b, y);
     double g = (q + q) * h;
