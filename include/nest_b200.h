@@ -336,13 +336,14 @@ nest_status nest_adjoint_stats(nest_adjoint* a, double* fwd_ms, double* bwd_ms, 
 /* ------------------------------------------------------------------------ */
 /* Self-tests of the FP64 kernels' branch-free division and square root. No  */
 /* counterpart in nest.  For n arguments (device arrays), q[i] = the fast    */
-/* quotient of a[i] / b[i] (r[i] = the fast root of x[i]) and ok[i] = 1 in   */
-/* the range where it is the correctly rounded IEEE value (elsewhere the     */
-/* kernels run the IEEE operation).  Enqueued on the legacy stream;          */
-/* synchronises before returning.                                           */
+/* quotient of a[i] / b[i] (r[i] = the fast root of x[i], or of the quotient */
+/* a[i] / b[i] rounded to a double) and ok[i] = 1 where it is the correctly  */
+/* rounded IEEE value (elsewhere the kernels run the IEEE operation).        */
+/* Enqueued on the legacy stream; synchronises before returning.            */
 /* ------------------------------------------------------------------------ */
 nest_status nest_selftest_div_f64(const double* d_a, const double* d_b, double* d_q, int* d_ok, int n);
 nest_status nest_selftest_sqrt_f64(const double* d_x, double* d_r, int* d_ok, int n);
+nest_status nest_selftest_sqrt_quot_f64(const double* d_a, const double* d_b, double* d_r, int* d_ok, int n);
 
 /* ------------------------------------------------------------------------ */
 /* Allocation-free 1D run.  No counterpart in nest's ABI.                   */

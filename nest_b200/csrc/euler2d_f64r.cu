@@ -497,6 +497,16 @@ __global__ void k_sqrt_selftest(const double* a, double* r, int* ok, int n) {
         ok[t] = a[t] >= 0x1p-257 && a[t] < 0x1p268 ? 1 : 0;
     }
 }
+__global__ void k_sqrt_quot_selftest(const double* a, const double* b, double* r, int* ok, int n) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) {
+        double y, q;
+        F64Range m;
+        r[t] = sqrt_quot_f64(a[t], b[t], y, q);
+        m.root(q);
+        ok[t] = m.ok() && a[t] >= 0x1p-128 && a[t] < 0x1p138 && b[t] >= 0x1p-128 && b[t] < 0x1p128 ? 1 : 0;
+    }
+}
 }  // namespace
 
 }  // namespace nestb
@@ -523,4 +533,10 @@ extern "C" nest_status nest_selftest_div_f64(const double* d_a, const double* d_
 extern "C" nest_status nest_selftest_sqrt_f64(const double* d_x, double* d_r, int* d_ok, int n) {
     return selftest(d_x, d_r, d_ok, n, "square root self-test: ",
                     [&](int blocks) { nestb::k_sqrt_selftest<<<blocks, 256>>>(d_x, d_r, d_ok, n); });
+}
+
+extern "C" nest_status nest_selftest_sqrt_quot_f64(const double* d_a, const double* d_b, double* d_r, int* d_ok, int n) {
+    if (!d_b) return nestb::record_error(NEST_ERR_INVALID, "null array or n < 0");
+    return selftest(d_a, d_r, d_ok, n, "square root of a quotient self-test: ",
+                    [&](int blocks) { nestb::k_sqrt_quot_selftest<<<blocks, 256>>>(d_a, d_b, d_r, d_ok, n); });
 }

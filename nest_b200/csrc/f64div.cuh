@@ -84,12 +84,12 @@ __device__ __forceinline__ double sqrt_f64(double x) {
     return fma(fma(-g, g, x), h, g);
 }
 
-// RN(sqrt(q)) with q = RN(a / b), in range, and the reciprocal of b: the same
-// steps as recip_f64, quot_f64 and sqrt_f64, with the square root's first
-// approximation taken from a quotient of 2^-39 relative error, so that it runs
-// beside the exact quotient instead of after it (the second Newton-Raphson step
-// of h and everything after it use the exact q).
-__device__ __forceinline__ double sqrt_quot_f64(double a, double b, double& y) {
+// RN(sqrt(q)) with q = RN(a / b), in range and not one of the two arguments above,
+// the reciprocal of b and q: the same steps as recip_f64, quot_f64 and sqrt_f64,
+// with the square root's first approximation taken from a quotient of 2^-39 relative
+// error, so that it runs beside the exact quotient instead of after it (the second
+// Newton-Raphson step of h and everything after it use the exact q).
+__device__ __forceinline__ double sqrt_quot_f64(double a, double b, double& y, double& q) {
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
     y = fma(y, fma(-b, y, 1.0), y);
     const double t = a * y, t2 = t + t;
@@ -99,7 +99,7 @@ __device__ __forceinline__ double sqrt_quot_f64(double a, double b, double& y) {
     h = fma(h, fma(-(t2 * h), h, 0.5), h);  // 1 / (2 sqrt(q)) to 2^-39
     y = __fma_ru(y, fma(-b, y, 1.0), y);
     y = fma(y, fma(-b, y, 1.0), y);
-    const double q = quot_f64(a, b, y);
+    q = quot_f64(a, b, y);
     double g = (q + q) * h;
     h = fma(h, fma(-g, h, 0.5), h);
     g = fma(fma(-g, g, q), h, g);
@@ -138,6 +138,13 @@ struct F64Range {
             : "=r"(k) : "r"(__double2loint(a)), "r"(2u * (unsigned)__double2hiint(a)));
         low = min(low, k);
     }
+    // root(q): q is not (1 + ulp) 4^k or (4 - 2 ulp) 4^k.  (Nor twice those: the
+    // fraction field alone is tested, for 1 and for all ones.)
+    __device__ __forceinline__ void root(double q) {
+        const unsigned hi = (unsigned)__double2hiint(q), lo = (unsigned)__double2loint(q);
+        const unsigned away = ((lo + 1u) & ~2u) | ((hi + (lo >> 31)) & 0xfffffu);
+        low = away == 0u ? 0u : low;
+    }
     __device__ __forceinline__ bool ok() const { return all >= 0xf0000000u && low >= (223u << 21); }
 };
 
@@ -171,9 +178,12 @@ struct ArithFast {
     // 1 / b to within a rounding (recip_f64), for terms that no branch compares
     __device__ __forceinline__ double inverse(double b) const { return recip_f64(b); }
     // (one multiplication more than root(quot()), for a shorter chain)
-    __device__ __forceinline__ double root_quot(double a, double b, Recip& r) const {
-        r.b = b;
-        return sqrt_quot_f64(a, b, r.y);
+    __device__ __forceinline__ double root_quot(double a, double b, Recip& ib) {
+        double q;
+        ib.b = b;
+        const double s = sqrt_quot_f64(a, b, ib.y, q);
+        r.root(q);
+        return s;
     }
     // h = +-1/2: h s is exact (slopes in range are multiples of 2^-1000), so the
     // fused form rounds the same sum
