@@ -157,8 +157,8 @@ struct nest_adjoint {
     void* u1 = nullptr;
     void* lam[2] = {nullptr, nullptr};
     void* tmp = nullptr;
-    double* d_dts = nullptr;       // all dts (device), for the adjoint kernels of the binomial schedule
-    double* seg_dts = nullptr;     // dts of the current segment (device), uniform schedule
+    double* d_dts = nullptr;       // all dts (device)
+    double* seg_dts = nullptr;     // dts of the current segment (device, copied from d_dts), uniform schedule
     void* arena = nullptr;         // one device allocation that holds all of the above
     std::map<int, cudaGraphExec_t> seg_graphs;  // uniform: one graph per segment length
     bool forward_done = false;
@@ -389,7 +389,8 @@ nest_status nest_adjoint_forward(nest_adjoint* a, double cfl, const double* dts)
         if ((st = nest_solver_get_dts(s, a->dts.data(), a->nsteps)) != NEST_OK) return st;
     }
     if ((st = nest_solver_set_dt_sequence(s, nullptr, 0, 2)) != NEST_OK) return st;
-    CK(cudaMemcpy(a->d_dts, a->dts.data(), sizeof(double) * a->nsteps, cudaMemcpyHostToDevice));
+    // on the stream of the backward sweep, which reads it (a->dts outlives the copy)
+    CK(cudaMemcpyAsync(a->d_dts, a->dts.data(), sizeof(double) * a->nsteps, cudaMemcpyHostToDevice, s->st));
     a->forward_done = true;
     return NEST_OK;
 }

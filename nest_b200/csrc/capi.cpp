@@ -639,7 +639,10 @@ nest_status nest_solver_set_dt_sequence(nest_solver* s, const double* dts, int n
         s->dts_alloc = n;
     }
     if (mode == 0) {
-        CK(cudaMemcpy(s->dts_buf, dts, sizeof(double) * n, cudaMemcpyHostToDevice));
+        // on the solver's stream, which no copy on the legacy stream is ordered before;
+        // the caller's array may go once this returns
+        CK(cudaMemcpyAsync(s->dts_buf, dts, sizeof(double) * n, cudaMemcpyHostToDevice, s->st));
+        CK(cudaStreamSynchronize(s->st));
         s->dts_in = s->dts_buf;
     } else {
         CK(cudaMemsetAsync(s->dts_buf, 0, sizeof(double) * n, s->st));
