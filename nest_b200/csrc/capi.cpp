@@ -619,6 +619,7 @@ nest_status nest_solver_set_tiling(nest_solver* s, int rows_per_tile, int warps_
 nest_status nest_solver_set_dt_sequence(nest_solver* s, const double* dts, int n, int mode) {
     nest_status r = check(s);
     if (r != NEST_OK) return r;
+    CK(cudaStreamSynchronize(s->st));  // no step that uses the buffer or a graph below is left
     slab_release(s);  // the slab driver's graphs do not tell dt sequences apart
     s->dts_in = s->dts_out = nullptr;
     s->dts_cap = 0;
@@ -627,7 +628,6 @@ nest_status nest_solver_set_dt_sequence(nest_solver* s, const double* dts, int n
     if (n <= 0) return fail(NEST_ERR_INVALID, "sequence length must be positive");
     if (mode != 0 && mode != 1) return fail(NEST_ERR_INVALID, "mode must be 0, 1 or 2");
     if (mode == 0 && !dts) return fail(NEST_ERR_INVALID, "null dt sequence");
-    CK(cudaStreamSynchronize(s->st));
     if (n > s->dts_alloc) {
         // the buffer moves: graphs that hold its address go (the others are
         // told apart by it, its use and its length)
