@@ -776,6 +776,8 @@ nest_status nest_pipeline_create(int dim, int nx, int ny, int npx, int npy, int 
     PipeCtrl c{};
     c.active = 1;
     if ((e = cudaMemcpy(p->ctrl, &c, sizeof c, cudaMemcpyHostToDevice)) != cudaSuccess) return cleanup(cuda_fail(e, "cudaMemcpy"));
+    // the copies above went to the legacy stream, which the callers' streams do not wait for
+    if ((e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess) return cleanup(cuda_fail(e, "sync"));
     *out = p;
     return NEST_OK;
 }
@@ -883,11 +885,11 @@ nest_status nest_pipeline_run(nest_pipeline* p, void* d_state, double t_final, i
         last = c.step;
     }
     // later execute() calls run without a stopping time
-    cudaStreamSynchronize(st);
     const double zero = 0.0;
     const int one = 1;
-    cudaMemcpy(&p->ctrl->t_final, &zero, sizeof zero, cudaMemcpyHostToDevice);
-    cudaMemcpy(&p->ctrl->active, &one, sizeof one, cudaMemcpyHostToDevice);
+    cudaMemcpyAsync(&p->ctrl->t_final, &zero, sizeof zero, cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(&p->ctrl->active, &one, sizeof one, cudaMemcpyHostToDevice, st);
+    cudaStreamSynchronize(st);
     if (steps_out) *steps_out = p->host_ctrl->step - start;
     return r;
 }
@@ -905,10 +907,10 @@ nest_status nest_pipeline_clock(nest_pipeline* p, double* time, double* dt, int*
 nest_status nest_pipeline_set_clock(nest_pipeline* p, double time, double dt, int step) {
     nest_status r = pcheck(p);
     if (r != NEST_OK) return r;
-    CK(cudaStreamSynchronize(p->own));
     PipeCtrl c{};
     c.time = time; c.dt = dt; c.step = step; c.active = 1;
-    CK(cudaMemcpy(p->ctrl, &c, sizeof c, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(p->ctrl, &c, sizeof c, cudaMemcpyHostToDevice, p->own));
+    CK(cudaStreamSynchronize(p->own));
     return NEST_OK;
 }
 
