@@ -882,6 +882,9 @@ nest_status batch_build_items(nest_batch* b) {
     // problems of 64..512 a side 1123 -> 1057, 64 of 48..320 333 -> 307; FP32, 256 of
     // 64..1024 2043 -> 1972, 48 of 64..256 60.3 -> 60.0.
     const int all = ((int)b->items.size() + b->warps - 1) / b->warps;
+    // the copies and fills above (and the creation's) went to the legacy stream, which
+    // the batch's stream does not wait for
+    CK(cudaStreamSynchronize(cudaStreamLegacy));
     b->blocks = b->persistent_blocks > 0 ? b->persistent_blocks : all;
     return NEST_OK;
 }
