@@ -71,6 +71,13 @@ __global__ void k_set_clock(StepCtrl* c, double time, int steps) {
     for (int p = 0; p < 2; ++p) { c->time[p] = time; c->step[p] = steps; }
 }
 
+// 1D: the maximum of the step in slot p goes to the slot's first word (the other one
+// is cleared by that step).
+__global__ void k_first_word(StepCtrl* c, int p) {
+    c->maxs[p][0] = c->maxs[p][c->sel[p] & 1];
+    c->sel[p] &= ~1;
+}
+
 nest_status drop_graphs(nest_solver* s) {
     for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
     s->graphs.clear();
@@ -106,6 +113,7 @@ nest_status nestb::rt::prepare(nest_solver* s) {
     }
     if (e != cudaSuccess) return cuda_fail(e, "prepare kernel");
     s->prepared = true;
+    s->word_alternates = false;
     return NEST_OK;
 }
 
@@ -158,6 +166,7 @@ nest_status enqueue_steps(nest_solver* s, int nsteps, const LoopParams& lp) {
     }
     bool use_graphs = s->st != nullptr;
     const bool pairs = s->d.dim == 1;
+    s->word_alternates = s->word_alternates || pairs;
     while (nsteps > 0) {
         if (use_graphs && nsteps >= GRAPH_STEPS) {
             GraphKey k{GRAPH_STEPS, s->parity, lp.cfl, lp.t_final, lp.fixed_dt, lp.max_steps, lp.dts_in,
@@ -695,8 +704,12 @@ nest_status nest_solver_stage(nest_solver* s, int which, double cfl, double t_fi
 nest_status nest_solver_speed_slot(nest_solver* s, void** dev) {
     nest_status r = check(s);
     if (r != NEST_OK) return r;
-    // in 1D the word alternates from step to step: put it back to the first
-    if ((!s->prepared || s->d.dim == 1) && (r = prepare(s)) != NEST_OK) return r;
+    if (!s->prepared && (r = prepare(s)) != NEST_OK) return r;
+    if (s->word_alternates) {
+        k_first_word<<<1, 1, 0, s->st>>>(s->ctrl, s->parity);
+        CK(cudaGetLastError());
+        s->word_alternates = false;
+    }
     if (dev) *dev = &s->ctrl->maxs[s->parity][0];
     return NEST_OK;
 }
