@@ -144,8 +144,11 @@ nest_status nest_solver_totals(nest_solver* s, double out[4]);
 /* Number of cells repaired by the FP32 form so far. */
 nest_status nest_solver_repairs(nest_solver* s, unsigned* count);
 nest_status nest_solver_sync(nest_solver* s);
-/* 2D launch shape: rows per tile and warps per block (autotuner hook). */
+/* 2D launch shape: rows per tile, from 8 or the default if that is less, and warps
+ * per block (autotuner hook). */
 nest_status nest_solver_set_tiling(nest_solver* s, int rows_per_tile, int warps_per_block);
+/* The launch shape that a solver of this description starts with (runs on the host). */
+nest_status nest_solver_default_tiling(const nest_solver_desc* d, int* rows_per_tile, int* warps_per_block);
 /* dt sequence: mode 0 freezes the given n values (copied), mode 1 records the
  * next n dts (read back with nest_solver_get_dts), mode 2 clears. */
 nest_status nest_solver_set_dt_sequence(nest_solver* s, const double* dts, int n, int mode);
@@ -231,6 +234,9 @@ nest_status nest_batch_totals(nest_batch* b, double* out);
 /* Launch shape: rows per work item, warps per block, blocks per SM of a persistent
  * grid that walks the list (0: a warp per item). */
 nest_status nest_batch_set_tiling(nest_batch* b, int rows_per_tile, int warps_per_block, int blocks_per_sm);
+/* The launch shape that a batch of this description starts with, with a warp per
+ * item (runs on the host). */
+nest_status nest_batch_default_tiling(const nest_batch_desc* d, int* rows_per_tile, int* warps_per_block);
 /* Zero every problem's time, step count and error word (states are kept;
  * ghost rings and wave speeds are rebuilt before the next step). */
 nest_status nest_batch_reset(nest_batch* b);

@@ -84,6 +84,7 @@ _SIGS = {
     "nest_solver_repairs": (_i, [_vp, C.POINTER(C.c_uint)]),
     "nest_solver_sync": (_i, [_vp]),
     "nest_solver_set_tiling": (_i, [_vp, _i, _i]),
+    "nest_solver_default_tiling": (_i, [C.POINTER(SolverDesc), _ip, _ip]),
     "nest_solver_set_dt_sequence": (_i, [_vp, _dp, _i, _i]),
     "nest_solver_get_dts": (_i, [_vp, _dp, _i]),
     "nest_solver_state_ptr": (_i, [_vp, C.POINTER(_vp), C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)]),

@@ -28,6 +28,7 @@ A.bind({
     "nest_batch_times": (_i, [_vp, C.POINTER(C.c_double), C.POINTER(C.c_int)]),
     "nest_batch_totals": (_i, [_vp, C.POINTER(C.c_double)]),
     "nest_batch_set_tiling": (_i, [_vp, _i, _i, _i]),
+    "nest_batch_default_tiling": (_i, [C.POINTER(BatchDesc), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "nest_batch_info": (_i, [_vp, C.POINTER(C.c_longlong), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "nest_batch_reset": (_i, [_vp]),
 })
@@ -49,6 +50,7 @@ class Batch:
                       self._dx.ctypes.data_as(dp) if self._dx is not None else None,
                       self._dy.ctypes.data_as(dp) if self._dy is not None else None,
                       gamma, bc[0], bc[1], precision, flags, C.c_void_p(stream) if stream else None)
+        self._desc = d
         h = C.c_void_p()
         check(lib.nest_batch_create(C.byref(d), C.byref(h)), "nest_batch_create")
         self._h = h
@@ -95,6 +97,12 @@ class Batch:
     def set_tiling(self, rows_per_tile: int, warps_per_block: int, blocks_per_sm: int = 0):
         check(lib.nest_batch_set_tiling(self._h, rows_per_tile, warps_per_block, blocks_per_sm),
               "nest_batch_set_tiling")
+
+    def default_tiling(self):
+        """(rows per tile, warps per block) that the batch started with."""
+        r, w = C.c_int(), C.c_int()
+        check(lib.nest_batch_default_tiling(C.byref(self._desc), C.byref(r), C.byref(w)), "nest_batch_default_tiling")
+        return r.value, w.value
 
     def reset(self):
         check(lib.nest_batch_reset(self._h), "nest_batch_reset")

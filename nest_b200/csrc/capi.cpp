@@ -316,6 +316,20 @@ int default_rows(int precision, long long work, int tall64, int tall32) {
     return work < 100000 ? 8 : tall32;
 }
 
+constexpr int SOLVER_WARPS = 1, BATCH_WARPS = 2;  // default warps per block
+
+int solver_rows(const nest_solver_desc* d) {
+    const int sw = strip_width(d->precision, d->flags);
+    return default_rows(d->precision, (long long)((d->ny + sw - 1) / sw) * d->nx, 24, 16);
+}
+
+int batch_rows(const nest_batch_desc* d) {
+    const int sw = strip_width(d->precision, 0);
+    long long work = 0;
+    for (int p = 0; p < d->count; ++p) work += (long long)((d->ny[p] + sw - 1) / sw) * d->nx[p];
+    return default_rows(d->precision, work, 16, 32);
+}
+
 }  // namespace
 
 // ===========================================================================
@@ -356,9 +370,9 @@ nest_status nest_solver_create(const nest_solver_desc* d, nest_solver** out) {
     s->h = d->halo;
     s->esize = d->precision == NEST_F64 ? 8 : 4;
     if (d->dim == 2) {
-        const int sw = strip_width(d->precision, d->flags);
-        s->tx = default_rows(d->precision, (long long)((d->ny + sw - 1) / sw) * d->nx, 24, 16);
-        s->warps = 1;
+        s->tx = solver_rows(d);
+        s->min_rows = std::min(8, s->tx);
+        s->warps = SOLVER_WARPS;
     }
     if (d->dim == 1) {
         s->nvars = 3;
@@ -385,10 +399,8 @@ nest_status nest_solver_create(const nest_solver_desc* d, nest_solver** out) {
     const bool totals = d->dim == 2 && (d->flags & NEST_FLAG_TOTALS);
     if (totals) {
         long long nstrips = (d->ny + STRIP - 1) / STRIP;
-        // sized for the default tile height and the smallest one the tiling
-        // hook accepts (8 rows)
-        const int rows = std::min(8, s->tx);
-        s->nrec = nstrips * ((d->nx + rows - 1) / rows);
+        // sized for the smallest tile height that the tiling hook accepts
+        s->nrec = nstrips * ((d->nx + s->min_rows - 1) / s->min_rows);
     }
     Arena ar;
     const size_t oU = ar.add(s->state_bytes()), oU1 = ar.add(s->state_bytes()), oC = ar.add(sizeof(StepCtrl)),
@@ -617,11 +629,20 @@ nest_status nest_solver_sync(nest_solver* s) {
 nest_status nest_solver_set_tiling(nest_solver* s, int rows_per_tile, int warps_per_block) {
     nest_status r = check(s);
     if (r != NEST_OK) return r;
-    if (rows_per_tile < 8 || rows_per_tile > 4096) return fail(NEST_ERR_INVALID, "rows per tile must be in [8, 4096]");
+    if (rows_per_tile < s->min_rows || rows_per_tile > 4096)
+        return fail(NEST_ERR_INVALID, "rows per tile must be in [" + std::to_string(s->min_rows) + ", 4096]");
     if (warps_per_block < 1 || warps_per_block > 8) return fail(NEST_ERR_INVALID, "warps per block must be in [1, 8]");
     s->tx = rows_per_tile;
     s->warps = warps_per_block;
     if (s->partials) cudaMemsetAsync(s->partials, 0, sizeof(double) * 4 * s->nrec, s->st);
+    return NEST_OK;
+}
+
+nest_status nest_solver_default_tiling(const nest_solver_desc* d, int* rows_per_tile, int* warps_per_block) {
+    if (!d) return fail(NEST_ERR_INVALID, "null argument");
+    if (d->dim != 2 || d->nx < 4 || d->ny < 4) return fail(NEST_ERR_INVALID, "launch shapes are those of 2D domains");
+    if (rows_per_tile) *rows_per_tile = solver_rows(d);
+    if (warps_per_block) *warps_per_block = SOLVER_WARPS;
     return NEST_OK;
 }
 
@@ -854,7 +875,8 @@ struct nest_batch {
     bool own_stream = false;
     int parity = 0;
     bool prepared = false;
-    int tx = 32, warps = 2, blocks = 0;
+    int tx = 32, warps = BATCH_WARPS, blocks = 0;
+    int min_rows = 8;                     // smallest tile height that the tiling hook accepts
     int persistent_blocks = 0;            // 0: a warp per item
     std::map<GraphKey, cudaGraphExec_t> graphs;
     int strip_w() const { return strip_width(d.precision, 0); }
@@ -1003,9 +1025,8 @@ nest_status nest_batch_create(const nest_batch_desc* d, nest_batch** out) {
         return cleanup(cuda_fail(e, "cudaMallocHost"));
     if ((e = cudaMalloc(&b->totals_dev, sizeof(double) * 4 * b->count)) != cudaSuccess)
         return cleanup(cuda_fail(e, "cudaMalloc(totals)"));
-    long long work = 0;
-    for (const BatchProblem& q : b->probs) work += (long long)((q.g.ny + b->strip_w() - 1) / b->strip_w()) * q.g.nx;
-    b->tx = default_rows(d->precision, work, 16, 32);
+    b->tx = batch_rows(d);
+    b->min_rows = std::min(8, b->tx);
     nest_status r = batch_build_items(b);
     if (r != NEST_OK) return cleanup(r);
     *out = b;
@@ -1067,7 +1088,8 @@ nest_status nest_batch_download(nest_batch* b, int problem, void* host, int layo
 nest_status nest_batch_set_tiling(nest_batch* b, int rows_per_tile, int warps_per_block, int blocks_per_sm) {
     nest_status r = batch_check(b);
     if (r != NEST_OK) return r;
-    if (rows_per_tile < 8 || rows_per_tile > 4096) return fail(NEST_ERR_INVALID, "rows per tile must be in [8, 4096]");
+    if (rows_per_tile < b->min_rows || rows_per_tile > 4096)
+        return fail(NEST_ERR_INVALID, "rows per tile must be in [" + std::to_string(b->min_rows) + ", 4096]");
     if (warps_per_block < 1 || warps_per_block > 8) return fail(NEST_ERR_INVALID, "warps per block must be in [1, 8]");
     CK(cudaStreamSynchronize(b->st));
     b->tx = rows_per_tile;
@@ -1080,6 +1102,13 @@ nest_status nest_batch_set_tiling(nest_batch* b, int rows_per_tile, int warps_pe
     if (blocks_per_sm > 0 && blocks_per_sm < per_sm) per_sm = blocks_per_sm;
     b->persistent_blocks = blocks_per_sm > 0 ? sms * per_sm : 0;
     return batch_build_items(b);
+}
+
+nest_status nest_batch_default_tiling(const nest_batch_desc* d, int* rows_per_tile, int* warps_per_block) {
+    if (!d || !d->nx || !d->ny || d->count <= 0) return fail(NEST_ERR_INVALID, "need the sizes of the problems");
+    if (rows_per_tile) *rows_per_tile = batch_rows(d);
+    if (warps_per_block) *warps_per_block = BATCH_WARPS;
+    return NEST_OK;
 }
 
 nest_status nest_batch_step(nest_batch* b, int nsteps, double cfl) {
