@@ -15,6 +15,7 @@
 #include <cstddef>
 #include <chrono>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <new>
@@ -91,6 +92,7 @@ LoopParams base_params(const nest_solver* s) {
     lp.dts_in = (s->dts_mode == 0) ? s->dts_in : nullptr;
     lp.dts_out = (s->dts_mode == 1) ? s->dts_out : nullptr;
     lp.dts_cap = s->dts_cap;
+    lp.short_waits = s->short_waits;
     return lp;
 }
 
@@ -375,6 +377,9 @@ nest_status nest_solver_create(const nest_solver_desc* d, nest_solver** out) {
         s->warps = SOLVER_WARPS;
     }
     if (d->dim == 1) {
+        // NEST_1D_WAIT_POLLS in the environment when the solver is created limits the looks
+        // of the resident loop's waits (a diagnostic: the way out of them can then be tested)
+        if (const char* e = std::getenv("NEST_1D_WAIT_POLLS")) s->short_waits = std::clamp(std::atoi(e), 0, 1 << 20) + 1;
         s->nvars = 3;
         s->n_total = d->nx + 2 * d->halo;
         s->vstride = s->n_total;

@@ -92,6 +92,7 @@ struct LoopParams {
     double fixed_dt;       // > 0: every step uses this dt (nest's rk2_step(dt))
     int step_budget;       // resident 1D kernel: > 0 = at most this many steps per launch
     int lim;               // slope limiter: LIM_MINMOD, LIM_MC or LIM_NONE
+    int short_waits;       // resident 1D kernel: > 0 = a wait between CTAs gives up after one look less (a test)
 };
 
 enum { LIM_MINMOD = 0, LIM_MC = 1, LIM_NONE = 2 };

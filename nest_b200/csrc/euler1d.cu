@@ -237,10 +237,9 @@ __device__ __forceinline__ void bar_init(unsigned bar) {
 __device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Waits for the phase of that parity; false after 2^24 polls (a quarter of a second
-// and more), which no message takes.
-__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
-    for (int k = 0; k < 1 << 24; ++k) {
+// Waits for the phase of that parity; false where it has not come after `polls` looks.
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, int polls) {
+    for (int k = 0; k < polls; ++k) {
         unsigned done;
         asm volatile("{\n\t.reg .pred p;\n\t"
                      "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
@@ -274,8 +273,11 @@ constexpr int LOOP_WARPS = 9, LOOP_CELLS = 31 * LOOP_WARPS;
 // Two cluster barriers a step instead (about 0.45 us each): 2.46 and 3.40; messages
 // for both stages 2.20 and 3.04; registers for two blocks an SM (96, spills) 2.13, 2.99.
 // LIM: the slope limiter fixed at compile time (LIM_MINMOD, nest's default) or
-// -1 to read it from the loop parameters.
-template <bool CLUSTER, int LIM>
+// -1 to read it from the loop parameters.  SHORT: waits give up after lp.short_waits - 1
+// looks, to test the way out of them (a limit read from the parameters costs the loop
+// 1.5 %, so the instance that runs otherwise has its own).
+constexpr int WAIT_POLLS = 1 << 24;  // a quarter of a second and more, which no message takes
+template <bool CLUSTER, int LIM, bool SHORT = false>
 __global__ void __launch_bounds__(32 * LOOP_WARPS, 1)
 k1d_loop(double* __restrict__ Ug, int n, int h, int m, double dx, double gamma, int bc, LoopParams lp,
          StepCtrl* ctrl, int p) {
@@ -372,7 +374,8 @@ k1d_loop(double* __restrict__ Ug, int n, int h, int m, double dx, double gamma, 
     auto receive = [&](int q) {
         if (!CLUSTER) return;
         const unsigned parity = (q >> 1) & 1;
-        const bool ok = (!edge || bar_wait(bar_halo(q), parity)) && bar_wait(bar_max(q), parity);
+        const int polls = SHORT ? lp.short_waits - 1 : WAIT_POLLS;
+        const bool ok = (!edge || bar_wait(bar_halo(q), parity, polls)) && bar_wait(bar_max(q), parity, polls);
         if (!ok) {
             lost = 1u;
             if (lane == 0) atomicOr(&ctrl->err, ERRW_LOST);
@@ -494,9 +497,10 @@ k1d_loop(double* __restrict__ Ug, int n, int h, int m, double dx, double gamma, 
         ctrl->time[p ^ 1] = time; ctrl->step[p ^ 1] = step;
     }
     if (CLUSTER) {
-        // no CTA leaves while stores to it may be in flight (after a wait that gave up,
-        // some that nobody has waited for)
-        if (lost)
+        // No CTA leaves while stores to it may be in flight.  All that were sent have been
+        // waited for, unless a wait gave up.  A store then was sent before its receiver gave
+        // up, which gives it 0.1 ms, or by a CTA that finds the news here and gives its own.
+        if (threadIdx.x == 0 && (lost || (*reinterpret_cast<volatile unsigned*>(&ctrl->err) & ERRW_LOST)))
             for (int k = 0; k < 100; ++k) __nanosleep(1000);
         cg::this_cluster().sync();
     }
@@ -553,7 +557,8 @@ static cudaError_t launch_1d_cluster(double* U, int n, int h, double dx, double 
                                      StepCtrl* ctrl, int p, cudaStream_t st, int NC) {
     LoopShape s;
     if (!loop_shape(n, NC, s)) return cudaErrorNotSupported;
-    auto kern = lp.lim == LIM_MINMOD ? k1d_loop<true, LIM_MINMOD> : k1d_loop<true, -1>;
+    auto kern = lp.short_waits > 0 ? k1d_loop<true, -1, true>
+                : lp.lim == LIM_MINMOD ? k1d_loop<true, LIM_MINMOD> : k1d_loop<true, -1>;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
     int clusters;

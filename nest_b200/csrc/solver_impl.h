@@ -87,6 +87,7 @@ struct nest_solver {
     int parity = 0;
     bool prepared = false;
     bool word_alternates = false;  // 1D: one-launch steps may have left the speed in a slot's second word
+    int short_waits = 0;           // 1D: LoopParams::short_waits
     int tx = 64, warps = 4;
     int min_rows = 8;              // 2D: smallest tile height that the tiling hook accepts
     int xlo_ex = 0, xhi_ex = 0;    // sharded domain: x sides filled by a halo exchange
