@@ -1125,7 +1125,8 @@ nest_status nest_batch_step(nest_batch* b, int nsteps, double cfl) {
     lp.cfl = cfl;
     while (nsteps > 0) {
         if (nsteps >= GRAPH_STEPS) {
-            GraphKey k{GRAPH_STEPS, b->parity, cfl, 0.0, 0.0, 0, nullptr, nullptr, 0, b->tx, b->warps * 1000 + b->blocks};
+            // (a new launch shape drops the graphs)
+            GraphKey k{GRAPH_STEPS, b->parity, cfl, 0.0, 0.0, 0, nullptr, nullptr, 0, b->tx, b->warps};
             auto it = b->graphs.find(k);
             if (it == b->graphs.end()) {
                 cudaGraph_t g;

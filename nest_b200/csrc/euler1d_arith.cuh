@@ -39,11 +39,10 @@ template <> struct Gas<double> {
 // 2^128), dS = SR - SL in the same range, which bounds the velocities where the
 // average is taken, and the mass and energy flux numerators from below (the
 // momentum one holds SR p - SL p).
-template <class A>
-__device__ __forceinline__ F3<double> hlle1d_a(A& m, double gamma, const typename A::Recip& ig, double rL, double uL,
-                                               double pL, double rR, double uR, double pR) {
+__device__ __forceinline__ F3<double> hlle1d_fast(ArithFast& m, double gamma, const ArithFast::Recip& ig, double rL,
+                                                  double uL, double pL, double rR, double uR, double pR) {
     m.pos(rL); m.pos(pL); m.pos(rR); m.pos(pR);
-    typename A::Recip il, ir;
+    ArithFast::Recip il, ir;
     const double cL = m.root_quot(gamma * pL, rL, il);
     const double cR = m.root_quot(gamma * pR, rR, ir);
     const double EL = m.quot(pL, ig) + 0.5 * rL * uL * uL;
@@ -73,7 +72,7 @@ __device__ __noinline__ F3<double> hlle1d_ieee(double gamma, double gm1, double 
 __device__ __forceinline__ F3<double> face_flux(const Gas<double>& g, double rL, double uL, double pL, double rR,
                                                 double uR, double pR) {
     ArithFast m;
-    const F3<double> f = hlle1d_a(m, g.gamma, g.ig, rL, uL, pL, rR, uR, pR);
+    const F3<double> f = hlle1d_fast(m, g.gamma, g.ig, rL, uL, pL, rR, uR, pR);
     if (m.ok() && g.fast) return f;
     return hlle1d_ieee(g.gamma, g.gm1, rL, uL, pL, rR, uR, pR);
 }

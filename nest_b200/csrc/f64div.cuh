@@ -158,11 +158,6 @@ struct ArithIeee {
     __device__ __forceinline__ double quot(double a, const Recip& r) const { return a / r.b; }
     __device__ __forceinline__ double root(double x) const { return sqrt(x); }
     __device__ __forceinline__ double inverse(double b) const { return 1.0 / b; }
-    // sqrt(a / b); makes b's Recip
-    __device__ __forceinline__ double root_quot(double a, double b, Recip& r) const {
-        r.b = b;
-        return sqrt(a / b);
-    }
     __device__ __forceinline__ double half(double w, double h, double s) const { return w + h * s; }
     __device__ __forceinline__ void pos(double) {}
     __device__ __forceinline__ void num(double) {}
@@ -177,7 +172,8 @@ struct ArithFast {
     __device__ __forceinline__ double root(double x) const { return sqrt_f64(x); }
     // 1 / b to within a rounding (recip_f64), for terms that no branch compares
     __device__ __forceinline__ double inverse(double b) const { return recip_f64(b); }
-    // (one multiplication more than root(quot()), for a shorter chain)
+    // sqrt(a / b); makes b's Recip (one multiplication more than root(quot()), for a
+    // shorter chain)
     __device__ __forceinline__ double root_quot(double a, double b, Recip& ib) {
         double q;
         ib.b = b;
