@@ -56,6 +56,9 @@ enum : unsigned {
     ERRW_LOST = 4u,        // a wait between the CTAs of a cluster ran into its limit
 };
 constexpr unsigned ERRW_STOP = ERRW_NONFINITE | ERRW_NONPOSITIVE | ERRW_LOST;
+// 1D: a step before the one in slot p has failed.  A one-launch step looks at this bit
+// alone: its own blocks may set the others while some are starting.
+__device__ __forceinline__ unsigned errw_slot(int p) { return 0x100u << p; }
 
 // Per-solver control block in device memory.  Fields indexed [p] belong to
 // the step launched with parity p; a step with parity p reads slot p and
@@ -76,9 +79,6 @@ struct StepCtrl {
     int bad_i, bad_j;               // its interior index (1D: bad_j = 0)
     int pad_;
     double bad_rho, bad_p;          // and its density and pressure
-    // 1D: a step before the one in slot p has failed.  A one-launch step reads this word:
-    // its own blocks may set `err` while others are starting.
-    unsigned stop[2];
 };
 
 // Time-loop parameters shared by all launches of a solver.
@@ -133,10 +133,11 @@ __device__ __forceinline__ T warp_sum(T v) {
 // which a NaN fails too, and call this on the rare failing path: the bit is
 // ERRW_NONFINITE for a NaN, else ERRW_NONPOSITIVE, and the first failing
 // cell records the step (`step_done` = steps completed, this one included),
-// its interior index and its values.
-__device__ __forceinline__ void flag_cell(StepCtrl* c, int step_done, double rho, double pr, int i, int j) {
+// its interior index and its values.  slot (1D): errw_slot of the step to come.
+__device__ __forceinline__ void flag_cell(StepCtrl* c, int step_done, double rho, double pr, int i, int j,
+                                          unsigned slot = 0) {
     const unsigned bit = (rho == rho && pr == pr) ? ERRW_NONPOSITIVE : ERRW_NONFINITE;
-    if (atomicOr(&c->err, bit) & ERRW_STOP) return;  // an earlier cell holds the record
+    if (atomicOr(&c->err, bit | slot) & ERRW_STOP) return;  // an earlier cell holds the record
     c->bad_step = step_done;
     c->bad_i = i;
     c->bad_j = j;
@@ -148,7 +149,7 @@ __device__ __forceinline__ void flag_cell(StepCtrl* c, int step_done, double rho
 // stage 1 evaluates this on the same inputs, so all agree; block 0 publishes.
 // one_launch: the step's own blocks may set `err` (k1d_step).
 __device__ __forceinline__ bool step_is_done(const StepCtrl* c, int p, const LoopParams& lp, bool one_launch = false) {
-    if (one_launch ? c->stop[p] != 0 : (c->err & ERRW_STOP) != 0) return true;
+    if (c->err & (one_launch ? errw_slot(p) : ERRW_STOP)) return true;
     double t = c->time[p];
     int s = c->step[p];
     if (lp.t_final > 0.0 && !(t < lp.t_final)) return true;
@@ -205,7 +206,7 @@ __device__ __forceinline__ void publish_step_1d(StepCtrl* c, int p, const LoopPa
         c->maxs[q][w] = c->maxs[p][w];
         c->maxs[q][1 - w] = 0ull;
         c->sel[q] = w + 2 * (1 - w);
-        c->stop[q] = (c->err & ERRW_STOP) != 0;  // (no block of a finished step sets it)
+        if (c->err & ERRW_STOP) c->err |= errw_slot(q);  // (no other block of a finished step writes it)
         c->active[q] = 0;
         return;
     }

@@ -104,10 +104,8 @@ k1d_stage(const T* __restrict__ Uin, const T* Un, T* Uout,
         if (STAGE == 2) {
             const Cell1<T> w = cell1d<true>(gas, v[0], v[1], v[2]);
             ms = (double)(fabs(w.u) + w.cs);
-            if (!(v[0] > T(0)) || !(w.p > T(0))) {
-                flag_cell(ctrl, ctrl->step[p] + 1, (double)v[0], (double)w.p, c, 0);
-                ctrl->stop[p ^ 1] = 1u;
-            }
+            if (!(v[0] > T(0)) || !(w.p > T(0)))
+                flag_cell(ctrl, ctrl->step[p] + 1, (double)v[0], (double)w.p, c, 0, errw_slot(p ^ 1));
         }
     }
     if (STAGE == 2) {
@@ -119,10 +117,7 @@ k1d_stage(const T* __restrict__ Uin, const T* Un, T* Uout,
             double x = (l < (NT1 + 31) / 32) ? red[l] : 0.0;
             x = warp_max(x);
             if (l == 0) {
-                if (!(x == x) || x > 1.79e308) {
-                    atomicOr(&ctrl->err, ERRW_NONFINITE);
-                    ctrl->stop[p ^ 1] = 1u;
-                }
+                if (!(x == x) || x > 1.79e308) atomicOr(&ctrl->err, ERRW_NONFINITE | errw_slot(p ^ 1));
                 atomic_max_speed(&ctrl->maxs[p ^ 1][0], x);
             }
         }
@@ -274,10 +269,8 @@ k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out,
             if (U1out) store(U1out, v[i], c + i);
             // (a NaN is dropped here and flagged below)
             ms = smax(ms, (double)(fabs(q.u) + q.cs));
-            if (!(x[0] > T(0)) || !(q.p > T(0))) {
-                flag_cell(ctrl, ctrl->step[p] + 1, (double)x[0], (double)q.p, c + i, 0);
-                ctrl->stop[p ^ 1] = 1u;
-            }
+            if (!(x[0] > T(0)) || !(q.p > T(0)))
+                flag_cell(ctrl, ctrl->step[p] + 1, (double)x[0], (double)q.p, c + i, 0, errw_slot(p ^ 1));
         }
     }
     ms = warp_max_speed(ms);
@@ -286,10 +279,7 @@ k1d_step(const T* __restrict__ Un, T* __restrict__ Unext, T* __restrict__ U1out,
     if (threadIdx.x == 0) {
         double m = red[0];
         for (int i = 1; i < STEP_WARPS; ++i) m = smax(m, red[i]);
-        if (m > 1.79e308) {
-            atomicOr(&ctrl->err, ERRW_NONFINITE);
-            ctrl->stop[p ^ 1] = 1u;
-        }
+        if (m > 1.79e308) atomicOr(&ctrl->err, ERRW_NONFINITE | errw_slot(p ^ 1));
         atomic_max_speed(&ctrl->maxs[p ^ 1][sel >> 1], m);
     }
 }
