@@ -67,11 +67,10 @@ __device__ __forceinline__ FaceDiv<float> face_div(float gamma, St3<float> L, St
 }
 __device__ __forceinline__ FaceDiv<double> face_div(double gamma, St3<double> L, St3<double> R) {
     ArithFast m;
-    ArithFast::Recip r;
     FaceDiv<double> d;
     m.pos(L.r); m.pos(L.p); m.pos(R.r); m.pos(R.p);
-    d.cL = m.root_quot(gamma * L.p, L.r, r);
-    d.cR = m.root_quot(gamma * R.p, R.r, r);
+    d.cL = m.root_quot(gamma * L.p, L.r);
+    d.cR = m.root_quot(gamma * R.p, R.r);
     const double spread = face_spread(L, R, d.cL, d.cR);
     m.pos(spread); m.pos(gamma);
     d.iD = m.inverse(spread);

@@ -294,7 +294,7 @@ k1d_loop(double* __restrict__ Ug, int n, int h, int m, double dx, double gamma, 
     double* const W = sm;             // [3][3][mw]: state of even / odd steps and U1, variable k, local cell l at H + l
     double* const Uh = W + 9 * mw;    // [2][4][2]: momentum and energy of the recomputed cells, by step
     double* const red = Uh + 16;      // [2][NC * nw]: wave-speed maxima of every warp, by step
-    const Gas<double> gas(gamma);
+    const Gas<double, ArithChain> gas(gamma);
     const int left = (r + NC - 1) % NC, right = (r + 1) % NC;
     const int mloc_left = n / NC + (left < n % NC ? 1 : 0);
     const bool per = bc == BC_PERIODIC;

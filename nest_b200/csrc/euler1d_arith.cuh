@@ -7,9 +7,8 @@
 // ten divisions and square roots.  With nvcc's IEEE forms each of them is a
 // branch that the next has to wait for; here they interleave, and a value whose
 // range tests fail (rare) is computed again, out of line, with the IEEE ones.
-// The square root's approximation runs beside the quotient it is taken of
-// (root_quot: 1.563 -> 1.497 us a step at 100 cells, 2.582 -> 2.508 at 1024), and
-// the pressure takes neither clamp nor halving on its chain (Sod's tube, with the
+// In the resident loop the square root's approximation runs beside the quotient it
+// is taken of (ArithChain), and the pressure takes neither clamp nor halving on its chain (Sod's tube, with the
 // host's copies: 100 cells to t = 0.1 169 -> 163 us, 1024 cells to 0.2 2880 -> 2800).
 #pragma once
 
@@ -23,11 +22,12 @@ template <typename T> struct F3 { T a, b, c; };
 
 // Constants of a launch: gamma, gamma - 1 and, for FP64, its reciprocal (in
 // range: else `fast` is false and everything takes the IEEE forms).
-template <typename T> struct Gas {
+// A: the branch-free policy that FP64 takes.
+template <typename T, class A = ArithFast> struct Gas {
     T gamma, gm1;
     __device__ __forceinline__ explicit Gas(double g) : gamma((T)g), gm1((T)(g - 1.0)) {}
 };
-template <> struct Gas<double> {
+template <class A> struct Gas<double, A> {
     double gamma, gm1;
     ArithFast::Recip ig;
     bool fast;
@@ -39,12 +39,12 @@ template <> struct Gas<double> {
 // 2^128), dS = SR - SL in the same range, which bounds the velocities where the
 // average is taken, and the mass and energy flux numerators from below (the
 // momentum one holds SR p - SL p).
-__device__ __forceinline__ F3<double> hlle1d_fast(ArithFast& m, double gamma, const ArithFast::Recip& ig, double rL,
-                                                  double uL, double pL, double rR, double uR, double pR) {
+template <class A>
+__device__ __forceinline__ F3<double> hlle1d_fast(A& m, double gamma, const typename A::Recip& ig, double rL, double uL,
+                                                  double pL, double rR, double uR, double pR) {
     m.pos(rL); m.pos(pL); m.pos(rR); m.pos(pR);
-    ArithFast::Recip il, ir;
-    const double cL = m.root_quot(gamma * pL, rL, il);
-    const double cR = m.root_quot(gamma * pR, rR, ir);
+    const double cL = m.root_quot(gamma * pL, rL);
+    const double cR = m.root_quot(gamma * pR, rR);
     const double EL = m.quot(pL, ig) + 0.5 * rL * uL * uL;
     const double ER = m.quot(pR, ig) + 0.5 * rR * uR * uR;
     const double SL = smin(uL - cL, uR - cR);
@@ -69,9 +69,10 @@ __device__ __noinline__ F3<double> hlle1d_ieee(double gamma, double gm1, double 
     return f;
 }
 
-__device__ __forceinline__ F3<double> face_flux(const Gas<double>& g, double rL, double uL, double pL, double rR,
+template <class A>
+__device__ __forceinline__ F3<double> face_flux(const Gas<double, A>& g, double rL, double uL, double pL, double rR,
                                                 double uR, double pR) {
-    ArithFast m;
+    A m;
     const F3<double> f = hlle1d_fast(m, g.gamma, g.ig, rL, uL, pL, rR, uR, pR);
     if (m.ok() && g.fast) return f;
     return hlle1d_ieee(g.gamma, g.gm1, rL, uL, pL, rR, uR, pR);
@@ -94,16 +95,15 @@ __device__ __noinline__ Cell1<double> cell1d_ieee(double gamma, double gm1, doub
     return { u, p, CS ? sqrt(gamma * p / r) : 0.0 };
 }
 
-template <bool CS>
-__device__ __forceinline__ Cell1<double> cell1d(const Gas<double>& g, double r, double m, double e) {
-    ArithFast a;
+template <bool CS, class A>
+__device__ __forceinline__ Cell1<double> cell1d(const Gas<double, A>& g, double r, double m, double e) {
+    A a;
     const auto ir = a.recip(r);
     const double u = a.quot(m, ir);
     // (a p that the clamp would change fails its test; halving is exact, and a
     // subnormal product is far below the energy's rounding)
     const double p = g.gm1 * fma(-0.5, r * u * u, e);
-    ArithFast::Recip ic;
-    const double cs = CS ? a.root_quot(g.gamma * p, r, ic) : 0.0;
+    const double cs = CS ? a.root_quot(g.gamma * p, r) : 0.0;
     a.pos(r); a.pos(p); a.num(m);
     if (a.ok() && g.fast) return { u, p, cs };
     return cell1d_ieee<CS>(g.gamma, g.gm1, r, m, e);
@@ -116,8 +116,8 @@ __device__ __forceinline__ Cell1<float> cell1d(const Gas<float>& g, float r, flo
 
 // PLM face states and flux between cells a and b, with their outer neighbours
 // am and bp (each (rho, u, p) through w(k, cell)).
-template <typename T, class W>
-__device__ __forceinline__ F3<T> plm_flux(const Gas<T>& g, int lim, W w, int am, int a, int b, int bp) {
+template <typename T, class A, class W>
+__device__ __forceinline__ F3<T> plm_flux(const Gas<T, A>& g, int lim, W w, int am, int a, int b, int bp) {
     T L[3], R[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {

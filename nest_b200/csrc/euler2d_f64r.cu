@@ -500,9 +500,9 @@ __global__ void k_sqrt_selftest(const double* a, double* r, int* ok, int n) {
 __global__ void k_sqrt_quot_selftest(const double* a, const double* b, double* r, int* ok, int n) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) {
-        double y, q;
+        double q;
         F64Range m;
-        r[t] = sqrt_quot_f64(a[t], b[t], y, q);
+        r[t] = sqrt_quot_f64(a[t], b[t], q);
         m.root(q);
         ok[t] = m.ok() && a[t] >= 0x1p-128 && a[t] < 0x1p138 && b[t] >= 0x1p-128 && b[t] < 0x1p128 ? 1 : 0;
     }

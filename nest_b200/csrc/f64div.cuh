@@ -84,12 +84,12 @@ __device__ __forceinline__ double sqrt_f64(double x) {
     return fma(fma(-g, g, x), h, g);
 }
 
-// RN(sqrt(q)) with q = RN(a / b), in range and not one of the two arguments above,
-// the reciprocal of b and q: the same steps as recip_f64, quot_f64 and sqrt_f64,
+// RN(sqrt(q)) with q = RN(a / b), in range and not one of the two arguments above, and q: the same steps as recip_f64, quot_f64 and sqrt_f64,
 // with the square root's first approximation taken from a quotient of 2^-39 relative
 // error, so that it runs beside the exact quotient instead of after it (the second
 // Newton-Raphson step of h and everything after it use the exact q).
-__device__ __forceinline__ double sqrt_quot_f64(double a, double b, double& y, double& q) {
+__device__ __forceinline__ double sqrt_quot_f64(double a, double b, double& q) {
+    double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
     y = fma(y, fma(-b, y, 1.0), y);
     const double t = a * y, t2 = t + t;
@@ -172,21 +172,27 @@ struct ArithFast {
     __device__ __forceinline__ double root(double x) const { return sqrt_f64(x); }
     // 1 / b to within a rounding (recip_f64), for terms that no branch compares
     __device__ __forceinline__ double inverse(double b) const { return recip_f64(b); }
-    // sqrt(a / b); makes b's Recip (one multiplication more than root(quot()), for a
-    // shorter chain)
-    __device__ __forceinline__ double root_quot(double a, double b, Recip& ib) {
-        double q;
-        ib.b = b;
-        const double s = sqrt_quot_f64(a, b, ib.y, q);
-        r.root(q);
-        return s;
-    }
+    // sqrt(a / b)
+    __device__ __forceinline__ double root_quot(double a, double b) { return root(quot(a, recip(b))); }
     // h = +-1/2: h s is exact (slopes in range are multiples of 2^-1000), so the
     // fused form rounds the same sum
     __device__ __forceinline__ double half(double w, double h, double s) const { return fma(h, s, w); }
     __device__ __forceinline__ void pos(double x) { r.pos(x); }
     __device__ __forceinline__ void num(double a) { r.num(a); }
     __device__ __forceinline__ bool ok() const { return r.ok(); }
+};
+// The same with the square root's approximation beside the quotient: a shorter chain for
+// a multiplication and a range test more.  For the resident 1D loop, which the chain
+// bounds (us a step at 100 / 1024 cells 1.356 -> 1.333, 1.980 -> 1.956); the kernels of many
+// warps are faster without (1D step at 200003 cells 10.53 -> 10.26, reverse step at
+// 65536 13.35 -> 13.07, pipeline of 400 cells 6.03 -> 5.95).
+struct ArithChain : ArithFast {
+    __device__ __forceinline__ double root_quot(double a, double b) {
+        double q;
+        const double s = sqrt_quot_f64(a, b, q);
+        r.root(q);
+        return s;
+    }
 };
 
 // RN(a / b) for one quotient by a divisor that changes.
