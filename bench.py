@@ -529,7 +529,7 @@ def run_ours(args, ws, rank, local):
 def bench_batch(args, ws):
     """Batched Kelvin-Helmholtz: `count` independent periodic problems with
     sides drawn uniformly from {64, ..., 1024} (seed 0), FP32 state with FP64
-    totals and repair, one persistent launch per stage, steps replayed from
+    totals and repair, one launch per stage, steps replayed from
     captured CUDA graphs; K = batch_steps steps per problem."""
     import torch
     import nest_b200 as nb
@@ -572,7 +572,7 @@ def bench_batch(args, ws):
     return {"value": value, "unit": UNIT, "problems": args.batch_count, "problems_per_rank": int(len(nx)),
             "l1_rho_vs_f64": acc,
             "sharding": f"by problem over {ws} rank(s), no collective", "cells": int(cells), "steps": args.batch_steps,
-            "ms_total": ms, "ms_per_step": ms / args.batch_steps, "work_items": items, "persistent_blocks": blocks,
+            "ms_total": ms, "ms_per_step": ms / args.batch_steps, "work_items": items, "stage_blocks": blocks,
             "hbm_gbs_equiv_per_gpu": value / ws * 40 / 1e9, "sim_time_range": [float(times.min()), float(times.max())],
             "fp64_totals_rel_drift": {"mass": float(drift[0]), "energy": float(drift[3])},
             "tiling": {"rows_per_item": tiling[0], "warps_per_block": tiling[1], "blocks_per_sm": tiling[2]},

@@ -269,7 +269,7 @@ __device__ __forceinline__ void put_global(T* Lin, int n, int h, int i, const T 
 // bit for bit the same).  Bound: the latency of two reversed stages, and with many
 // cells the FP64 pipe.  us of backward per step of a checkpointed sweep, the
 // recomputed forward step included (FP64 65536 / 5000 cells, FP32 65536 / 5000):
-// 13.7 / 7.4, 8.6 / 5.5, against 15.6 / 10.3, 10.7 / 7.9 with CTAs of 112 cells that
+// 13.1 / 7.3, 8.6 / 5.5, against 15.6 / 10.3, 10.7 / 7.9 with CTAs of 112 cells that
 // staged ten phases through shared memory and IEEE divisions.
 template <typename T, int CPL>
 __global__ void __launch_bounds__(32 * ADJ_WARPS)

@@ -298,19 +298,15 @@ int strip_width(int precision, int flags) {
 // than that only repeat their prologue (about two rows).  Larger domains run
 // many waves anyway and amortise the prologue with tall tiles.
 // Measured, us per step with 16 (FP32) / 24 (FP64) rows -> the rule's, in
-// parentheses the best of a sweep over 1..32 rows: FP32 64^2 59.8 -> 9.7 (9.7),
-// 256 x 192 59.2 -> 10.9, 512^2 59.1 -> 18.0 (18.0), 517 x 1003 61.3 -> 29.5 (28.7),
-// 1024^2 64.9 -> 45.9 (45.9), 1500^2 82.2 -> 75.5 (74.9), 2048^2 136.0 -> 125.1
-// (124.7), 4096^2 369.1 at 16, 368.9 at 12, 393.0 at 8; FP64 64^2 89.0 -> 18.5,
-// 512^2 90.7 -> 48.8 (48.8), 517 x 1003 103.2 -> 67.4 (65.1), 1024^2 122.5 -> 108.2
-// (108.2), 2048^2 349.6 at 24, 346.3 at 20, 381.3 at 32.  FP32 batches: 12 problems
-// of 64..256 a side 65 -> 32 (32), 48 of them 81 -> 60 (59), 64 of 48..320 108 -> 95
-// (95), 128 of 64..512 318 (32 rows; 12 rows 328); FP64 batches: 64 of 48..320 312 at
-// 16 rows, 307 at 12, 346 at 4, 128 of 64..512 1057 at 16, 1061 at 32.
-// The same shapes since the stages launch dependently and their FP64 arithmetic
-// shrank: FP32 64^2 8.5, 256 x 192 9.1, 512^2 16.4, 517 x 1003 26.5, 1024^2 43.0,
-// 2048^2 118.8, 4096^2 358; FP64 64^2 17.0, 256 x 192 22.6, 512^2 46.3, 517 x 1003
-// 61.9, 1024^2 100, 2048^2 323; batches of 48 57 (FP32) and 182 (FP64).
+// parentheses the best of a sweep over 1..32 rows: FP32 64^2 59.8 -> 9.7 (9.7), 512^2
+// 59.1 -> 18.0 (18.0), 1024^2 64.9 -> 45.9 (45.9), 2048^2 136.0 -> 125.1 (124.7); FP64
+// 64^2 89.0 -> 18.5, 512^2 90.7 -> 48.8 (48.8), 517 x 1003 103.2 -> 67.4 (65.1), 1024^2
+// 122.5 -> 108.2 (108.2), 2048^2 349.6 at 24, 346.3 at 20, 381.3 at 32.  Batches: FP32, 48
+// problems of 64..256 a side 81 -> 60 (59), 128 of 64..512 318 at 32 rows, 328 at 12;
+// FP64, 64 of 48..320 312 at 16 rows, 307 at 12, 346 at 4.  With dependent launches and
+// the shorter FP64 arithmetic the same shapes are the best or within 3 % of it, at
+// FP32 64^2 8.5, 512^2 16.4, 1024^2 43.0, 2048^2 118.8; FP64 64^2 17.0, 512^2 46.3,
+// 1024^2 100, 2048^2 323.
 int default_rows(int precision, long long work, int tall64, int tall32) {
     if (precision == NEST_F64) return (int)std::min<long long>(tall64, (work + 3999) / 4000);
     const long long one_wave = (work + 2367) / 2368;
@@ -917,7 +913,7 @@ nest_status batch_build_items(nest_batch* b) {
     for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
     b->graphs.clear();
     // A warp per item by default: the hardware hands out the blocks as others
-    // end, where a persistent grid's fixed stride leaves warps idle when the
+    // end, where the fixed stride of a persistent grid leaves warps idle when the
     // items do not divide evenly.  Us per step, persistent -> this: FP64, 128
     // problems of 64..512 a side 1123 -> 1057, 64 of 48..320 333 -> 307; FP32, 256 of
     // 64..1024 2043 -> 1972, 48 of 64..256 60.3 -> 60.0.

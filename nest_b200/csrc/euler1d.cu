@@ -268,8 +268,8 @@ constexpr int LOOP_WARPS = 9, LOOP_CELLS = 31 * LOOP_WARPS;
 // What bounds it is one thread's chain of dependent FP64 operations (two face
 // chains and two cell chains a step) and, in a cluster, the exchange.
 // Sod tube, us per step (with IEEE divisions and square roots, state in shared
-// memory and a barrier between fluxes and update): 100 cells 1.43 (5.87), 200 cells
-// 1.85 (6.47), both one CTA; 1024 cells on 16 CTAs 2.00 (4.67), 4080 cells 2.92 (5.68).
+// memory and a barrier between fluxes and update): 100 cells 1.40 (5.87), 200 cells
+// 1.82 (6.47), both one CTA; 1024 cells on 16 CTAs 2.01 (4.67), 4080 cells 2.94 (5.68).
 // Two cluster barriers a step instead (about 0.45 us each): 2.46 and 3.40; messages
 // for both stages 2.20 and 3.04; registers for two blocks an SM (96, spills) 2.13, 2.99.
 // LIM: the slope limiter fixed at compile time (LIM_MINMOD, nest's default) or

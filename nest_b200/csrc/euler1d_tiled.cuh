@@ -168,7 +168,7 @@ __device__ __forceinline__ void warp_update(const T (&u)[CPL][3], const F3<T> (&
 // step count or error) copies Un to Unext so that the state ends in the buffer
 // the caller expects.
 // Bound: one chain of two stages and the launch.  us per step (FP64 5003 / 65536 /
-// 200003 cells, FP32 50021): 4.1 / 5.1 / 10.8, 3.0, against 6.0 / 7.3 / 14.3, 5.5 with
+// 200003 cells, FP32 50021): 4.2 / 5.2 / 10.3, 3.0, against 6.0 / 7.3 / 14.3, 5.5 with
 // 224-cell CTAs that staged each phase through shared memory and moved the
 // maximum with a counter of finished blocks.
 template <typename T, int LIM, int CPL>

@@ -506,8 +506,8 @@ struct X2View {
     int tx;
 };
 
-// Persistent batched stage: every warp walks the work list (problem, strip,
-// tile row) with a stride of the whole grid's warp count.  The 128-register
+// Batched stage: every warp walks the work list (problem, strip, tile row) with a
+// stride of the whole grid's warp count (one item each by default).  The 128-register
 // budget matches the single-domain kernels (16 warps per SM).  The ghost rings
 // are filled afterwards by kbatch_ghosts: with many small problems a large
 // share of the warps sit on a domain edge, and one copy pass over all rings

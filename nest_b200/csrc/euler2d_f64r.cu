@@ -414,7 +414,7 @@ struct F64View {
     int tx;
 };
 
-// Persistent batched stage (bit for bit the single-domain solver's result per
+// Batched stage (bit for bit the single-domain solver's result per
 // problem): every warp walks the work list (problem, strip, tile row) with the
 // grid's warp count as stride (one item each by default).
 // Us per step with TOTALS, against the register-window march with IEEE

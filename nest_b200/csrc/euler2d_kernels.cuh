@@ -447,7 +447,7 @@ struct BatchProblem {
     int pad;
 };
 
-// Arguments of a persistent batched stage launch.
+// Arguments of a batched stage launch.
 template <typename T>
 struct BatchArgs {
     T* U;                       // all problems' states, problem p at U + probs[p].off

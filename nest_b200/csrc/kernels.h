@@ -84,7 +84,7 @@ cudaError_t launch_2d_adjoint_stage_f32x2(const float* U, const float* Lout, con
                                           const Geo2D& g, const double* dtp, double alpha, double beta,
                                           cudaStream_t st);
 
-// Batched persistent stages (one launch per stage over the work list).
+// Batched stages (one launch per stage over the work list).
 template <typename T> struct BatchArgs;
 cudaError_t launch_batch_f64(const BatchArgs<double>& b, int which, int blocks, int warps, cudaStream_t st);
 cudaError_t launch_batch_f32x2(const BatchArgs<float>& b, bool repair, int which, int blocks, int warps,

@@ -258,7 +258,7 @@ struct LoopArgs {
 // SMEM (one CTA): the buffers live in shared memory for the launch.
 // Bound: the latency of the stages' chains and their barriers.  nest's sod1d step
 // (ten stages, twelve launches), us per step against a launch per stage: 100 cells
-// 4.6 (26), 400 6.3 (30), 1024 12.7 (31), 4000 12.9 (31), 16000 25 (38); with every cell
+// 4.6 (26), 400 6.2 (30), 1024 12.5 (31), 4000 12.6 (31), 16000 25 (38); with every cell
 // computing both its faces and the buffers in global memory 100 cells 6.4, 400 9.8,
 // 1024 14.1, 4000 14.4.
 template <bool CLUSTER, bool SMEM>
