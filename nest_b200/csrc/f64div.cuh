@@ -42,15 +42,18 @@
 // "Software division and square root using Goldschmidt's algorithms", RNC6,
 // 2004): from the hardware approximation y0 (measured: |1 - x y0^2| < 2^-19.0)
 // g ~ s = sqrt(x) and h ~ 1 / (2 s) together, g <- g + g r, h <- h + h r with
-// r = 1/2 - g h (2^-39), then h once more, with relative error |eta| <= 2 2^-53,
-// then twice g <- g + (x - g^2) h.  The first leaves g within half an ulp (and a few
-// 2^-26 of one) of s; the second has an exact residual and rounds
-// s - d^2 / (2 s) + d eta (d = s - g).  With s in [1, 2), a midpoint m below s has
-// s - m >= 7 ulp^2 / (8 s) (in units of ulp^2 / 4, m^2 is 1 modulo 8 and x a
-// multiple of 8), and one above s has m - s >= ulp^2 / (8 s), with equality only
-// for x = 1 + ulp and x = 4 - 2 ulp, the next case being 9 times as far: what is
-// added to s stays inside these but for the few arguments that come closest,
-// and tests/test_gpu_div.py runs those.
+// r = 1/2 - g h (2^-39), then h once more, with relative error eta, then twice
+// g <- g + (x - g^2) h.  The first of these leaves g within half an ulp (and a few 2^-26
+// of one) of s; the second has an exact residual and rounds s - d^2 / (2 s) + d eta
+// (d = s - g).  With s in [1, 2) and ulp = 2^-52, eta is the rounding of h and half the
+// rounding of g, at most (s + 1/s) ulp / 4, so next to a midpoint, where |d| is half an
+// ulp, at most ulp^2 s / 8 is added to s and ulp^2 (s + 2/s) / 8 taken from it.  A
+// midpoint m below s has s - m >= 7 ulp^2 / (8 s) (in units of ulp^2 / 4, m^2 is 1
+// modulo 8 and x a multiple of 8), more than is taken; one above s has m - s >= 9 ulp^2 /
+// (8 s), more than is added, but for x = 1 + ulp and x = 4 - 2 ulp, where it is ulp^2 /
+// (8 s).  sqrt_f64's steps depend on x alone, and tests/test_gpu_div.py runs it on these
+// two; sqrt_quot_f64's depend on the quotient's operands too, so the kernels do not
+// keep its root of these two (F64Range::root).
 #pragma once
 
 #include <cuda_runtime.h>
